@@ -128,12 +128,13 @@ struct PlanImpl {
   int win_half_a = 0, win_half_b = 0;
   // workspace
   int slots = 0;
-  DBuf xs, xs32, xs_tmp, comb_buf, comb_tmp, J, score, hits, comb_bits, comb_list, counters, out_idx, out_val;
+  DBuf xs, xs32, xs_tmp, pw, comb_tmp, comb_pw, J, score, hits, comb_bits, comb_list, counters, out_idx, out_val;
   DBuf man, man_tmp, g1, g2, perm, est_f, est_v, map_keys, map_vals, map_list;
   DBuf rparams, inputs, dense_ptrs, in_stage, dense_stage, trace, cnt_stash;
   std::vector<unsigned> epoch;
   int hit_cap = 0, out_cap = 0, est_cap = 0, map_cap = 0, table_cap = 0;
   int large_b = 0, large_c = 0;  // FFTs longer than one CTA's shared memory
+  int many_b = 0, many_c = 0;    // FFTs run over many CTAs (the long ones, and FP64 from 1024 points)
   int rp_stride = 0;
   std::vector<int> last_rp;  // draws of the last exec (slot 0)
   // page-locked staging for graph replays (draws and input pointers are
@@ -210,9 +211,21 @@ long xs_position(long b, long B, int lg) {
 
 // ------------------------------------------------------------- constants --
 
-bool upload_twiddles(DBuf &b, long N, int prec) {
+// Twiddles of an N-point FFT.  staged: stage by stage, entry r Ns + k holding
+// w_{4 Ns}^{r k} (r = 1 .. 3, k < Ns) for the radix-4 stages Ns = 1, 4, ... or
+// 2, 8, ... -- the table's own values w_N^{r k N / (4 Ns)}, reordered.
+bool upload_twiddles(DBuf &b, long N, int prec, bool staged) {
   const std::vector<double> &tw = sfft::fft_twiddles(N);
   std::vector<double> t(tw.begin(), tw.begin() + 2 * N);
+  if (staged) {
+    for (long Ns = ilog2(N) & 1 ? 2 : 1; Ns < N; Ns *= 4)
+      for (long r = 1; r < 4; r++)
+        for (long k = 0; k < Ns; k++) {
+          const long e = r * k * (N / (4 * Ns));
+          t[2 * (r * Ns + k)] = tw[2 * e];
+          t[2 * (r * Ns + k) + 1] = tw[2 * e + 1];
+        }
+  }
   if (prec == sfft::PREC_FP64) return b.upload(t);
   return b.upload(to_f32(t));
 }
@@ -347,13 +360,14 @@ bool ensure_slots(PlanImpl &P, int want) {
       P.out_cap = P.hit_cap;
     }
     if (P.prec == sfft::PREC_FP64 && !P.xs32.ensure(8 * p.x_samp_size * S)) return false;
-    if (P.large_b && !P.xs_tmp.ensure(cs * p.x_samp_size * S)) return false;
-    if (P.large_c && (!P.comb_buf.ensure(cs * (size_t)p.Comb_loops * p.W_Comb * S) ||
-                      !P.comb_tmp.ensure(cs * (size_t)p.Comb_loops * p.W_Comb * S)))
+    const size_t ks = cs / 2;  // a selection key
+    if (P.many_b && (!P.xs_tmp.ensure(cs * p.x_samp_size * S) || !P.pw.ensure(ks * p.x_samp_size * S))) return false;
+    if (P.many_c && (!P.comb_tmp.ensure(cs * (size_t)p.Comb_loops * p.W_Comb * S) ||
+                     !P.comb_pw.ensure(ks * (size_t)p.Comb_loops * p.W_Comb * S)))
       return false;
     if (!P.xs.ensure(cs * p.x_samp_size * S) || !P.J.ensure(sizeof(int) * L * p.B_thresh * S) ||
         !P.hits.ensure(sizeof(int) * P.hit_cap * S) ||
-        !P.comb_bits.ensure(sizeof(unsigned) * ((p.W_Comb + 31) / 32) * S) ||
+        !P.comb_bits.ensure(sizeof(unsigned) * (size_t)p.Comb_loops * ((p.W_Comb + 31) / 32) * S) ||
         !P.comb_list.ensure(sizeof(int) * p.W_Comb * S) || !P.out_idx.ensure(sizeof(int) * P.out_cap * S) ||
         !P.out_val.ensure(cs * P.out_cap * S))
       return false;
@@ -492,8 +506,9 @@ sfft::V12Dev v12_view(PlanImpl &P) {
   d.xs = P.xs.p;
   d.xs32 = P.prec == sfft::PREC_FP64 ? P.xs32.p : nullptr;
   d.xs_tmp = P.xs_tmp.p;
-  d.comb_buf = P.comb_buf.p;
+  d.pw = P.pw.p;
   d.comb_tmp = P.comb_tmp.p;
+  d.comb_pw = P.comb_pw.p;
   d.large_buckets = P.large_b;
   d.large_comb = P.large_c;
   d.win32_loc = P.win32_a.p;
@@ -593,12 +608,13 @@ void shift_view(PlanImpl &P, sfft::V12Dev &d, int base, bool own_out) {
   shift(d.xs, cs * d.xs_size, base);
   shift(d.xs32, 8 * d.xs_size, base);
   shift(d.xs_tmp, cs * d.xs_size, base);
-  shift(d.comb_buf, cs * (size_t)d.comb_loops * d.W, base);
+  shift(d.pw, cs / 2 * d.xs_size, base);
   shift(d.comb_tmp, cs * (size_t)d.comb_loops * d.W, base);
+  shift(d.comb_pw, cs / 2 * (size_t)d.comb_loops * d.W, base);
   shift(d.J, sizeof(int) * (size_t)d.L * d.num, base);
   shift(d.score, sizeof(unsigned) * (size_t)d.n, base);
   shift(d.hits, sizeof(int) * (size_t)d.hit_cap, base);
-  shift(d.comb_bits, sizeof(unsigned) * (size_t)((d.W + 31) / 32), base);
+  shift(d.comb_bits, sizeof(unsigned) * (size_t)d.comb_loops * ((d.W + 31) / 32), base);
   shift(d.comb_list, sizeof(int) * (size_t)d.W, base);
   shift(d.counters, sizeof(int) * sfft::CNT_STRIDE, base);
   if (own_out) {
@@ -1000,21 +1016,18 @@ bool plan_staged_view(sfft_plan *plan, int num, int in_type, int *out_idx, void 
 }
 
 // Per call of the persistent executor, capturable: the staged draws and
-// input pointers go to the device, the counters and comb bitmaps of `num`
+// input pointers go to the device, the counters of `num`
 // slots are cleared (what v12_run does before its first kernel).
 bool plan_persist_prepare(sfft_plan *plan, int num, cudaStream_t s) {
   PlanImpl *P = impl(plan);
   if (!P || P->version > 1 || num > P->staged_slots) return false;
   std::lock_guard<std::mutex> g(P->mu);
-  const auto &p = P->p12;
   return cuda_ok(cudaMemcpyAsync(P->rparams.p, P->h_rp, sizeof(int) * (size_t)P->rp_stride * num,
                                  cudaMemcpyHostToDevice, s),
                  "params upload") &&
          cuda_ok(cudaMemcpyAsync(P->inputs.p, P->h_in, sizeof(void *) * num, cudaMemcpyHostToDevice, s),
                  "pointer upload") &&
-         cuda_ok(cudaMemsetAsync(P->counters.p, 0, sizeof(int) * sfft::CNT_STRIDE * num, s), "memset") &&
-         cuda_ok(cudaMemsetAsync(P->comb_bits.p, 0, sizeof(unsigned) * ((p.W_Comb + 31) / 32) * (size_t)num, s),
-                 "memset");
+         cuda_ok(cudaMemsetAsync(P->counters.p, 0, sizeof(int) * sfft::CNT_STRIDE * num, s), "memset");
 }
 
 // Device side of a staged launch, capturable into a CUDA graph: copies the
@@ -1177,6 +1190,8 @@ static sfft_plan *make_plan_impl(int n, int k, enum sfft_version version, const 
     }
     P->large_b = (p.B_loc > mx || p.B_est > mx);
     P->large_c = (P->version == 1 && p.W_Comb > mx);
+    P->many_b = P->large_b || sfft::v12_many_ctas(P->prec, std::max(p.B_loc, p.B_est));
+    P->many_c = P->large_c || (P->version == 1 && sfft::v12_many_ctas(P->prec, p.W_Comb));
     if (p.B_loc > (1 << 20) || p.B_est > (1 << 20) || p.W_Comb > (1 << 22)) {
       set_err("bucket or comb FFT longer than 2^20 points");
       return nullptr;
@@ -1191,8 +1206,8 @@ static sfft_plan *make_plan_impl(int n, int k, enum sfft_version version, const 
         (P->prec == sfft::PREC_FP64 &&
          (!upload_v12_window(P->win32_a, fa.freq, n, n / p.B_loc, sfft::PREC_FP32) ||
           !upload_v12_window(P->win32_b, fb.freq, n, n / p.B_est, sfft::PREC_FP32))) ||
-        !upload_twiddles(P->tw_a, p.B_loc, P->prec) || !upload_twiddles(P->tw_b, p.B_est, P->prec) ||
-        !upload_twiddles(P->tw_c, std::max(p.W_Comb, 2), P->prec))
+        !upload_twiddles(P->tw_a, p.B_loc, P->prec, true) || !upload_twiddles(P->tw_b, p.B_est, P->prec, true) ||
+        !upload_twiddles(P->tw_c, std::max(p.W_Comb, 2), P->prec, true))
       return nullptr;
   } else {
     if (sfft::build_v3_plan((unsigned)n, (unsigned)k, P->p3, fa, fb, err, &bo)) {
@@ -1211,8 +1226,9 @@ static sfft_plan *make_plan_impl(int n, int k, enum sfft_version version, const 
     if (!P->taps_a.upload(fa.time) || !P->taps_b.upload(fb.time) ||
         !upload_v3_window(P->win_a, fa.freq, n, P->win_half_a) ||
         !upload_v3_window(P->win_b, fb.freq, n, P->win_half_b) ||
-        !upload_twiddles(P->tw_a, p.B_g1, sfft::PREC_FP64) || !upload_twiddles(P->tw_b, p.B_g2, sfft::PREC_FP64) ||
-        !upload_twiddles(P->tw_c, p.W_Man, sfft::PREC_FP64))
+        !upload_twiddles(P->tw_a, p.B_g1, sfft::PREC_FP64, false) ||
+        !upload_twiddles(P->tw_b, p.B_g2, sfft::PREC_FP64, false) ||
+        !upload_twiddles(P->tw_c, p.W_Man, sfft::PREC_FP64, false))
       return nullptr;
   }
   if (!cuda_ok(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking), "stream")) return nullptr;
@@ -1276,7 +1292,7 @@ long sfft_plan_footprint(const sfft_plan *plan) {
     return -1;
   }
   const DBuf *bufs[] = {&P->taps_a, &P->taps_b, &P->win_a, &P->win_b, &P->win32_a, &P->win32_b, &P->tw_a,
-                        &P->tw_b, &P->tw_c, &P->xs, &P->xs32, &P->xs_tmp, &P->comb_buf, &P->comb_tmp, &P->J,
+                        &P->tw_b, &P->tw_c, &P->xs, &P->xs32, &P->xs_tmp, &P->pw, &P->comb_tmp, &P->comb_pw, &P->J,
                         &P->score, &P->hits, &P->comb_bits, &P->comb_list, &P->counters, &P->out_idx,
                         &P->out_val, &P->man, &P->man_tmp, &P->g1, &P->g2, &P->perm, &P->est_f, &P->est_v, &P->map_keys,
                         &P->map_vals, &P->map_list, &P->rparams, &P->inputs, &P->dense_ptrs, &P->in_stage,

@@ -126,8 +126,11 @@ __device__ __forceinline__ int2 block_exscan2(int a, int b, int &pa, int &pb, in
 // --------------------------------------------------------- shared-mem FFT --
 
 // Forward FFT of buf[0..N) in shared memory, N = 2^logN <= PER*4*blockDim.
-// tw: the N-entry twiddle table of that length (global memory).
-template <typename R, int PER>
+// tw: the N-entry twiddle table of that length (global memory), in natural
+// order, or (STAGED) stage by stage: entry r Ns + k is w_{4 Ns}^{r k}, r = 1
+// .. 3, k < Ns, of the radix-4 stage Ns -- the same values, with those that
+// neighbouring threads use side by side.
+template <typename R, int PER, bool STAGED = false>
 __device__ void block_fft(c2_t<R> *buf, int N, int logN, const c2_t<R> *__restrict__ tw) {
   using V = c2_t<R>;
   const int T = blockDim.x;
@@ -162,8 +165,8 @@ __device__ void block_fft(c2_t<R> *buf, int N, int logN, const c2_t<R> *__restri
         for (int r = 0; r < 4; r++) v[s][r] = buf[j + r * q4];
 #pragma unroll
         for (int r = 1; r < 4; r++) {
-          int e = r * k * stride;
-          if (e) v[s][r] = cmul<R>(v[s][r], tw[e]);
+          const int e = STAGED ? r * Ns + k : r * k * stride;
+          if (k) v[s][r] = cmul<R>(v[s][r], tw[e]);
         }
         V t0 = cadd<R>(v[s][0], v[s][2]), t1 = csub<R>(v[s][0], v[s][2]);
         V t2 = cadd<R>(v[s][1], v[s][3]), t3 = csub<R>(v[s][1], v[s][3]);

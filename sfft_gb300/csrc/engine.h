@@ -24,7 +24,7 @@ enum InType { IN_C128 = 0, IN_C64 = 1 };
 
 // Per-slot counters (one block of ints per slot, zeroed before each exec).
 enum Counter { CNT_HITS = 0, CNT_COMB = 1, CNT_OUT = 2, CNT_ERR = 3, CNT_VOTED = 4, CNT_V3 = 5,
-               CNT_TRACE = 6, CNT_EST = 7, CNT_EXACT = 8, CNT_STRIDE = 16 };
+               CNT_TRACE = 6, CNT_EST = 7, CNT_EXACT = 8, CNT_TICKET = 9, CNT_STRIDE = 16 };
 
 // Error bits reported in counters[CNT_ERR].
 enum ErrBits { ERR_HIT_OVERFLOW = 1, ERR_OUT_OVERFLOW = 2, ERR_V3_NOCONVERGE = 4, ERR_V3_CAP = 8,
@@ -48,8 +48,8 @@ struct V12Dev {
   // per-slot workspace
   void *xs;                 // xs_size complex per slot
   void *xs32;               // FP64 plans: float2 copy of xs (median pre-selection)
-  void *xs_tmp;             // large bucket FFTs: ping-pong partner of xs
-  void *comb_buf, *comb_tmp;  // large comb FFTs: comb_loops * W per slot
+  void *xs_tmp, *pw;          // bucket FFTs over many CTAs (pw != null): ping-pong partner of xs, selection keys
+  void *comb_tmp, *comb_pw;   // comb FFTs over many CTAs (comb_pw != null): comb_loops * W per slot
   int large_buckets, large_comb;  // FFT longer than one CTA's shared memory
   // Bucket layout of xs (and xs32).  0: natural, bucket b of a loop at b.
   // lg > 0 (plain v2 FP32 with W a multiple of both n/B): grouped for the
@@ -60,7 +60,7 @@ struct V12Dev {
   int *J;                   // L * num per slot
   unsigned *score;          // n per slot: (epoch << 8) | votes
   int *hits;                // hit_cap per slot
-  unsigned *comb_bits;      // W/32 per slot
+  unsigned *comb_bits;      // comb_loops planes of W/32 words per slot
   int *comb_list;           // W per slot
   int *counters;            // CNT_STRIDE per slot
   int *out_idx;             // out_stride per slot
@@ -88,6 +88,14 @@ cudaError_t scatter_dense(const int *out_idx, const void *out_val, int prec, con
 
 // Maximum bucket-FFT length held in one CTA's shared memory.
 int v12_max_fft(int prec);
+// Whether FFTs of N points run over many CTAs: every one beyond a CTA's
+// shared memory, and FP64 ones from 1024 points on (see fft.cuh).  Below, a
+// one-CTA FP64 FFT already gives each sub-partition at most one warp of
+// butterflies, so more CTAs would only add launches.  Measured in FP64,
+// 4096-point buckets of 8 signals (160 FFTs) with their voting: 168 us in one
+// CTA each, 106 us over many; 16384-point combs: 174 us stage by stage
+// through global memory, 50 us.
+inline bool v12_many_ctas(int prec, int N) { return N > v12_max_fft(prec) || (prec == PREC_FP64 && N >= 1024); }
 
 // ------------------------------------------- persistent uneven executor --
 // One persistent kernel runs the whole v2 pipeline of several FP32 plans
@@ -99,7 +107,6 @@ struct PersistGroup {
   V12Dev d;          // the plan's view: staged draws and inputs, outputs in the caller's arena
   int gslot0;        // first global signal slot of this plan
   int slots;         // its signals
-  int per_comb, per_bucket;   // butterflies per thread of the comb / bucket FFTs (1, 2, 4)
   int fold_chunks;   // 1024-thread chunks of the fold per item
   int vote_cmax, vote_chunks; // comb residues at most; unused (1)
   int est_comb;      // 1: estimation by comb residue (1024 candidates per item), 0: random lookups

@@ -18,7 +18,7 @@
 // larger plans are rejected with an error.
 //
 // Sharing: every call on a device uses the same array and it keeps the last
-// call's contents.  The counters and comb bitmap are cleared on the stream
+// call's contents.  The counters are cleared on the stream
 // at the start of each call; vote counters carry a per-call tag instead of
 // being cleared, and they occupy a fixed region at the start of the array
 // that nothing else is written to, so plans of different sizes can follow
@@ -105,7 +105,7 @@ extern "C" long sfft_exec_noalloc(sfft_plan *plan, const void *d_in, int in_type
   const size_t o_hits = off;
   off += up256(sizeof(int) * (size_t)hit_cap);
   const size_t o_bits = off;
-  off += up256(sizeof(unsigned) * (size_t)((d.W + 31) / 32));
+  off += up256(sizeof(unsigned) * (size_t)d.comb_loops * ((d.W + 31) / 32));
   const size_t o_list = off;
   off += up256(sizeof(int) * (size_t)d.W);
   if (d.large_buckets || d.large_comb || d.n > SFFT_NOALLOC_MAX_N || d.xs_size > SFFT_NOALLOC_MAX_XS || L > SFFT_NOALLOC_MAX_LOOPS ||
@@ -162,6 +162,7 @@ extern "C" long sfft_exec_noalloc(sfft_plan *plan, const void *d_in, int in_type
   // count as zero votes; the region holds SFFT_NOALLOC_MAX_N >= n counters.
   d.xs = base + o_xs;
   d.xs32 = d.prec == PREC_FP64 ? base + o_xs32 : nullptr;
+  d.xs_tmp = d.pw = d.comb_tmp = d.comb_pw = nullptr;  // the plan's; here every FFT runs in one CTA
   d.J = (int *)(base + o_J);
   d.score = (unsigned *)(base + o_score);
   d.hits = (int *)(base + o_hits);

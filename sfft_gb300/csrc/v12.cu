@@ -1,8 +1,8 @@
 // v12.cu — the sFFT v1/v2 exec pipeline on GB300.
 //
 //   k_comb      (v2) strided W-point gather + shared-memory FFT + |.|^2 +
-//               top-num residues -> comb bitmap     (computefourier-1.0-2.0.cc:48-82)
-//   k_comb_list (v2) bitmap -> sorted, de-duplicated residue list   (:491-503)
+//               top-num residues (computefourier-1.0-2.0.cc:48-82) -> sorted,
+//               de-duplicated residue list of the samplings  (:491-503)
 //   k_fold      permuted-filter fold, one thread per (loop, bucket),
 //               taps summed in increasing order                      (:222-261)
 //   k_bucket    per loop: B-point FFT in shared memory, |.|^2, top-num
@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "engine.h"
+#include "fft.cuh"
 
 namespace sfft {
 
@@ -158,63 +159,84 @@ __global__ void __launch_bounds__(256) k_fold_split(V12Dev d) {
   fold_split_thread<In, S>(d, blockIdx.y, (long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// ---------------------------------------------------------- smem layout --
+// ------------------------------------------------------- one-CTA FFTs --
 
+// FFT and selection keys of N points in one CTA.  FP32: block_fft16, keys
+// recomputed from the values (two FMAs); FP64: one radix-4 butterfly per
+// thread and stage (PER of them beyond 1024 threads), keys stored beside the
+// values (a recomputed one costs three FP64 instructions).
 template <typename R>
-struct BucketSmem {
-  static size_t bytes(int B, int num) {
-    return (size_t)B * sizeof(c2_t<R>) + (size_t)B * sizeof(key_t<R>) + (264 + 64 + (size_t)num) * 4;
+struct OneCta;
+
+template <>
+struct OneCta<float> {
+  static constexpr int threads(int N) { return N / 16 < 128 ? 128 : N / 16; }
+  static size_t bytes(int N) { return sizeof(float2) * (size_t)fft16_size(N); }
+  float2 *buf;
+  __device__ __forceinline__ OneCta(unsigned char *smem, int) : buf((float2 *)smem) {}
+  template <int PER, typename Ld>
+  __device__ __forceinline__ void fft(int N, const float2 *tw, Ld ld) {
+    if (N >= 16) {
+      block_fft16<float>(buf, N, dlog2(N), tw, ld);
+    } else {
+      for (int i = threadIdx.x; i < N; i += blockDim.x) buf[i] = ld(i);
+      __syncthreads();
+      block_fft<float, 1, true>(buf, N, dlog2(N), tw);
+    }
   }
+  __device__ __forceinline__ float2 at(int i) const { return buf[fft16_at(i)]; }
+  __device__ __forceinline__ unsigned key(int i) const { return pkey(cabs2<float>(at(i))); }
 };
 
-template <typename R>
-__device__ __forceinline__ void carve(unsigned char *smem, int B, c2_t<R> *&buf, key_t<R> *&keys,
-                                      int *&hist, int *&scan, int *&Js) {
-  buf = (c2_t<R> *)smem;
-  keys = (key_t<R> *)(buf + B);
-  hist = (int *)(keys + B);
-  scan = hist + 264;
-  Js = scan + 64;
-}
+template <>
+struct OneCta<double> {
+  static constexpr int threads(int N) { return N / 4 < 128 ? 128 : N / 4 > 1024 ? 1024 : N / 4; }
+  static size_t bytes(int N) { return (sizeof(double2) + sizeof(unsigned long long)) * (size_t)N; }
+  double2 *buf;
+  unsigned long long *keys;
+  __device__ __forceinline__ OneCta(unsigned char *smem, int N)
+      : buf((double2 *)smem), keys((unsigned long long *)(buf + N)) {}
+  template <int PER, typename Ld>
+  __device__ __forceinline__ void fft(int N, const double2 *tw, Ld ld) {
+    for (int i = threadIdx.x; i < N; i += blockDim.x) buf[i] = ld(i);
+    __syncthreads();
+    block_fft<double, PER, true>(buf, N, dlog2(N), tw);
+    for (int i = threadIdx.x; i < N; i += blockDim.x) keys[i] = pkey(cabs2<double>(buf[i]));
+    __syncthreads();
+  }
+  __device__ __forceinline__ double2 at(int i) const { return buf[i]; }
+  __device__ __forceinline__ unsigned long long key(int i) const { return keys[i]; }
+};
 
 // ------------------------------------------------------------------ comb --
 
-template <typename R, int PER, typename In>
-__device__ __forceinline__ void comb_block(const V12Dev &d, int c, int slot, unsigned char *smem) {
-  const int W = d.W;
-  c2_t<R> *buf;
-  key_t<R> *keys;
-  int *hist, *scan, *Js;
-  carve<R>(smem, W, buf, keys, hist, scan, Js);
-  const int *rp = d.rparams + (long)slot * d.rp_stride;
-  const long sigma = d.n / W;
-  const long offset = rp[2 * d.L + c];
-  const In *x = (const In *)d.inputs[slot];
-  for (int i = threadIdx.x; i < W; i += blockDim.x) buf[i] = cvt_in<R>(__ldg(x + offset + i * sigma));
-  __syncthreads();
-  block_fft<R, PER>(buf, W, dlog2(W), (const c2_t<R> *)d.tw_comb);
-  for (int i = threadIdx.x; i < W; i += blockDim.x) keys[i] = pkey(cabs2<R>(buf[i]));
-  __syncthreads();
-  block_top_indices<key_t<R>>(keys, W, d.num, Js, hist, scan);
-  unsigned *bits = d.comb_bits + (long)slot * ((W + 31) >> 5);
-  for (int i = threadIdx.x; i < d.num; i += blockDim.x) atomicOr(&bits[Js[i] >> 5], 1u << (Js[i] & 31));
+// Residues of one comb sampling: one bit plane per sampling (plain stores,
+// nothing to clear); a single sampling's residues are the list itself.
+template <typename K, typename KeyAt>
+__device__ __forceinline__ void comb_select(const V12Dev &d, int c, int slot, KeyAt keyat, SelShared<K> &ss) {
+  const int W = d.W, words = (W + 31) >> 5;
+  const bool one = d.comb_loops == 1;
+  block_select<K>(keyat, W, d.num, one ? d.comb_list + (long)slot * W : nullptr,
+                  d.comb_bits + ((long)slot * d.comb_loops + c) * words, ss);
+  if (one && threadIdx.x == 0) d.counters[slot * CNT_STRIDE + CNT_COMB] = d.num;
 }
 
-template <typename R, int PER, typename In>
-__global__ void __launch_bounds__(1024) k_comb(V12Dev d) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  comb_block<R, PER, In>(d, blockIdx.x, blockIdx.y, smem);
-}
-
+// The union of the samplings' planes as a bitmap (plane 0) and as a sorted
+// list.
 __device__ __forceinline__ void comb_list_block(const V12Dev &d, int slot) {
   __shared__ int scan[64];
   const int W = d.W;
   const int words = (W + 31) >> 5;
-  const unsigned *bits = d.comb_bits + (long)slot * words;
+  unsigned *bits = d.comb_bits + (long)slot * d.comb_loops * words;
   const int C = (words + blockDim.x - 1) / blockDim.x;
   const int lo = min(words, (int)threadIdx.x * C), hi = min(words, lo + C);
   int cnt = 0;
-  for (int i = lo; i < hi; i++) cnt += __popc(bits[i]);
+  for (int i = lo; i < hi; i++) {
+    unsigned v = __ldcg(bits + i);
+    for (int c = 1; c < d.comb_loops; c++) v |= __ldcg(bits + (long)c * words + i);
+    bits[i] = v;
+    cnt += __popc(v);
+  }
   int pre, dummy;
   int2 tot = block_exscan2(cnt, 0, pre, dummy, scan);
   int *list = d.comb_list + (long)slot * W;
@@ -229,7 +251,40 @@ __device__ __forceinline__ void comb_list_block(const V12Dev &d, int slot) {
   if (threadIdx.x == 0) d.counters[slot * CNT_STRIDE + CNT_COMB] = tot.x;
 }
 
-__global__ void __launch_bounds__(1024) k_comb_list(V12Dev d) { comb_list_block(d, blockIdx.x); }
+// With several samplings the last CTA of a slot to finish builds the list.
+__device__ __forceinline__ void comb_last_list(const V12Dev &d, int slot) {
+  if (d.comb_loops == 1) return;
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0)
+    last = atomicAdd(&d.counters[slot * CNT_STRIDE + CNT_TICKET], 1) == d.comb_loops - 1;
+  __syncthreads();
+  if (last) {
+    __threadfence();
+    comb_list_block(d, slot);
+  }
+}
+
+template <typename R, int PER, typename In>
+__device__ __forceinline__ void comb_block(const V12Dev &d, int c, int slot, unsigned char *smem,
+                                           SelShared<key_t<R>> &ss) {
+  const int W = d.W;
+  OneCta<R> f(smem, W);
+  const int *rp = d.rparams + (long)slot * d.rp_stride;
+  const long sigma = d.n / W;
+  const In *x = (const In *)d.inputs[slot] + rp[2 * d.L + c];
+  f.template fft<PER>(W, (const c2_t<R> *)d.tw_comb, [=](int i) { return cvt_in<R>(__ldg(x + i * sigma)); });
+  comb_select<key_t<R>>(d, c, slot, [&](int i) { return f.key(i); }, ss);
+}
+
+template <typename R, int PER, typename In>
+__global__ void __launch_bounds__(1024) k_comb(V12Dev d) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ SelShared<key_t<R>> ss;
+  comb_block<R, PER, In>(d, blockIdx.x, blockIdx.y, smem, ss);
+  comb_last_list(d, blockIdx.y);
+}
 
 // Voting of the location loops, one thread per (loop, selected bucket,
 // position): positions p in [J*q - floor(q/2), +q) (mod n)
@@ -293,7 +348,7 @@ __global__ void __launch_bounds__(256) k_vote(V12Dev d) {
   const long n = d.n;
   const unsigned long long mask = (unsigned long long)n - 1;
   unsigned *score = d.score + (long)slot * n;
-  const unsigned *bits = d.comb_bits + (long)slot * ((d.W + 31) >> 5);
+  const unsigned *bits = d.comb_bits + (long)slot * d.comb_loops * ((d.W + 31) >> 5);
   int *cnt = d.counters + slot * CNT_STRIDE;
   {
     const int i = (int)(e >> lq), o = (int)(e & (q - 1));
@@ -398,45 +453,167 @@ __global__ void __launch_bounds__(256) k_vote_bits(V12Dev d) {
 
 // ---------------------------------------------------------------- bucket --
 
+// Place of bucket i in a loop's x_samp: (i mod T) * G + i / T in the grouped
+// layout (xs_perm = log2 G).
+__device__ __forceinline__ int xs_place(int i, int lg, int lt) {
+  return lg ? ((i & ((1 << lt) - 1)) << lg) | (i >> lt) : i;
+}
+
+struct LoopSpan {
+  int B;
+  long off;
+  bool loc;
+};
+__device__ __forceinline__ LoopSpan loop_span(const V12Dev &d, int j) {
+  LoopSpan l;
+  l.loc = j < d.L_loc;
+  l.B = l.loc ? d.B_loc : d.B_est;
+  l.off = l.loc ? (long)j * d.B_loc : (long)d.L_loc * d.B_loc + (long)(j - d.L_loc) * d.B_est;
+  return l;
+}
+
 template <typename R, int PER>
-__device__ __forceinline__ void bucket_block(const V12Dev &d, int j, int slot, unsigned char *smem) {
-  const bool loc = j < d.L_loc;
-  const int B = loc ? d.B_loc : d.B_est;
-  const long off = loc ? (long)j * d.B_loc : (long)d.L_loc * d.B_loc + (long)(j - d.L_loc) * d.B_est;
-  c2_t<R> *buf;
-  key_t<R> *keys;
-  int *hist, *scan, *Js;
-  carve<R>(smem, B, buf, keys, hist, scan, Js);
-  c2_t<R> *xs = (c2_t<R> *)d.xs + (long)slot * d.xs_size + off;
-  for (int i = threadIdx.x; i < B; i += blockDim.x) buf[i] = xs[i];
-  __syncthreads();
-  block_fft<R, PER>(buf, B, dlog2(B), (const c2_t<R> *)(loc ? d.tw_loc : d.tw_est));
-  float2 *xs32 = d.xs32 ? (float2 *)d.xs32 + (long)slot * d.xs_size + off : nullptr;
-  // grouped layout (xs_perm): bucket i goes to (i mod T) * G + i / T
-  const int lg = d.xs_perm, lt = dlog2(B) - lg;
-  const int tmask = (1 << lt) - 1;
-  for (int i = threadIdx.x; i < B; i += blockDim.x) {
-    const c2_t<R> v = buf[i];
-    const int p = lg ? ((i & tmask) << lg) | (i >> lt) : i;
+__device__ __forceinline__ void bucket_block(const V12Dev &d, int j, int slot, unsigned char *smem,
+                                             SelShared<key_t<R>> &ss) {
+  const LoopSpan l = loop_span(d, j);
+  const int B = l.B;
+  OneCta<R> f(smem, B);
+  c2_t<R> *xs = (c2_t<R> *)d.xs + (long)slot * d.xs_size + l.off;
+  f.template fft<PER>(B, (const c2_t<R> *)(l.loc ? d.tw_loc : d.tw_est), [=](int i) { return xs[i]; });
+  float2 *xs32 = d.xs32 ? (float2 *)d.xs32 + (long)slot * d.xs_size + l.off : nullptr;
+  const int lg = d.xs_perm, lt = dlog2(B) - lg, gm = (1 << lg) - 1;
+#pragma unroll 4
+  for (int p = threadIdx.x; p < B; p += blockDim.x) {  // in the order of the places: coalesced
+    const c2_t<R> v = f.at(lg ? ((p & gm) << lt) | (p >> lg) : p);
     xs[p] = v;
     if (xs32) xs32[p] = make_float2((float)v.x, (float)v.y);
-    keys[i] = pkey(cabs2<R>(v));
   }
-  __syncthreads();
-  block_top_indices<key_t<R>>(keys, B, d.num, Js, hist, scan);
-  int *Jg = d.J + ((long)slot * d.L + j) * d.num;
-  for (int i = threadIdx.x; i < d.num; i += blockDim.x) Jg[i] = Js[i];
+  block_select<key_t<R>>([&](int i) { return f.key(i); }, B, d.num, d.J + ((long)slot * d.L + j) * d.num, nullptr,
+                         ss);
 }
 
 template <typename R, int PER>
-__global__ void __launch_bounds__(1024, (sizeof(R) == 4 && PER == 1) ? 2 : 1) k_bucket(V12Dev d) {
+__global__ void __launch_bounds__(1024) k_bucket(V12Dev d) {
   extern __shared__ __align__(16) unsigned char smem[];
-  bucket_block<R, PER>(d, blockIdx.x, blockIdx.y, smem);
+  __shared__ SelShared<key_t<R>> ss;
+  bucket_block<R, PER>(d, blockIdx.x, blockIdx.y, smem, ss);
 }
 
-// ------------------------------------------------- FFTs beyond one CTA --
+// ------------------------------------------------ FFTs over many CTAs --
+//
+// Bucket and comb FFTs as two launches of fft_tile and one of the selection
+// (which reads the keys the second launch leaves).
 
-// One Stockham stage over `narr` arrays of N points per slot.
+// First launch: stages 1 .. M1 of every loop's array, xs -> xs_tmp.
+template <typename R>
+__global__ void __launch_bounds__(1024) k_bucket_a(V12Dev d, int elems, int nloc, int nest) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int x = blockIdx.x, slot = blockIdx.y;
+  const int j = x < d.L_loc * nloc ? x / nloc : d.L_loc + (x - d.L_loc * nloc) / nest;
+  const int tile = x < d.L_loc * nloc ? x % nloc : (x - d.L_loc * nloc) % nest;
+  const LoopSpan l = loop_span(d, j);
+  const int M = l.B / fft_m2(l.B), lc = fft_lc(elems, M, l.B);
+  const c2_t<R> *src = (const c2_t<R> *)d.xs + (long)slot * d.xs_size + l.off;
+  c2_t<R> *dst = (c2_t<R> *)d.xs_tmp + (long)slot * d.xs_size + l.off;
+  fft_tile<R>((c2_t<R> *)smem, M, lc, 1, l.B, tile << lc, dlog2(l.B) & 1,
+              (const c2_t<R> *)(l.loc ? d.tw_loc : d.tw_est), [=](int i) { return src[i]; },
+              [=](int i, c2_t<R> v) { dst[i] = v; });
+}
+
+// Second launch: the remaining stages, xs_tmp -> xs (in its layout), the
+// FP32 copy and the selection keys.
+template <typename R>
+__global__ void __launch_bounds__(1024) k_bucket_b(V12Dev d, int elems, int nloc, int nest) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int x = blockIdx.x, slot = blockIdx.y;
+  const int j = x < d.L_loc * nloc ? x / nloc : d.L_loc + (x - d.L_loc * nloc) / nest;
+  const int tile = x < d.L_loc * nloc ? x % nloc : (x - d.L_loc * nloc) % nest;
+  const LoopSpan l = loop_span(d, j);
+  const int M = fft_m2(l.B), lc = fft_lc(elems, M, l.B);
+  const long at = (long)slot * d.xs_size + l.off;
+  const c2_t<R> *src = (const c2_t<R> *)d.xs_tmp + at;
+  c2_t<R> *dst = (c2_t<R> *)d.xs + at;
+  float2 *dst32 = d.xs32 ? (float2 *)d.xs32 + at : nullptr;
+  key_t<R> *pw = (key_t<R> *)d.pw + at;
+  const int lg = d.xs_perm, lt = dlog2(l.B) - lg;
+  fft_tile<R>((c2_t<R> *)smem, M, lc, l.B / M, l.B, tile << lc, false,
+              (const c2_t<R> *)(l.loc ? d.tw_loc : d.tw_est), [=](int i) { return src[i]; },
+              [=](int i, c2_t<R> v) {
+                const int p = xs_place(i, lg, lt);
+                dst[p] = v;
+                if (dst32) dst32[p] = make_float2((float)v.x, (float)v.y);
+                pw[i] = pkey(cabs2<R>(v));
+              });
+}
+
+// Selection of loop j from its keys (in shared memory up to SEL_KEYS bytes).
+constexpr int SEL_KEYS = 128 * 1024;
+
+template <typename R>
+__global__ void __launch_bounds__(1024) k_bucket_select(V12Dev d) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  using K = key_t<R>;
+  __shared__ SelShared<K> ss;
+  const int j = blockIdx.x, slot = blockIdx.y;
+  const LoopSpan l = loop_span(d, j);
+  const K *pw = (const K *)d.pw + (long)slot * d.xs_size + l.off;
+  int *J = d.J + ((long)slot * d.L + j) * d.num;
+  if (l.B * sizeof(K) <= SEL_KEYS) {
+    K *keys = (K *)smem;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < l.B; i += blockDim.x) keys[i] = pw[i];
+    __syncthreads();
+    block_select<K>([=](int i) { return keys[i]; }, l.B, d.num, J, nullptr, ss);
+  } else {
+    block_select<K>([=](int i) { return pw[i]; }, l.B, d.num, J, nullptr, ss);
+  }
+}
+
+template <typename R, typename In>
+__global__ void __launch_bounds__(1024) k_comb_a(V12Dev d, int elems) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int c = blockIdx.y, slot = blockIdx.z, W = d.W;
+  const int M = W / fft_m2(W), lc = fft_lc(elems, M, W);
+  const int *rp = d.rparams + (long)slot * d.rp_stride;
+  const long sigma = d.n / W;
+  const In *x = (const In *)d.inputs[slot] + rp[2 * d.L + c];
+  c2_t<R> *dst = (c2_t<R> *)d.comb_tmp + ((long)slot * d.comb_loops + c) * W;
+  fft_tile<R>((c2_t<R> *)smem, M, lc, 1, W, (int)blockIdx.x << lc, dlog2(W) & 1, (const c2_t<R> *)d.tw_comb,
+              [=](int i) { return cvt_in<R>(__ldg(x + i * sigma)); }, [=](int i, c2_t<R> v) { dst[i] = v; });
+}
+
+template <typename R>
+__global__ void __launch_bounds__(1024) k_comb_b(V12Dev d, int elems) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int c = blockIdx.y, slot = blockIdx.z, W = d.W;
+  const int M = fft_m2(W), lc = fft_lc(elems, M, W);
+  const c2_t<R> *src = (const c2_t<R> *)d.comb_tmp + ((long)slot * d.comb_loops + c) * W;
+  key_t<R> *pw = (key_t<R> *)d.comb_pw + ((long)slot * d.comb_loops + c) * W;
+  fft_tile<R>((c2_t<R> *)smem, M, lc, W / M, W, (int)blockIdx.x << lc, false, (const c2_t<R> *)d.tw_comb,
+              [=](int i) { return src[i]; }, [=](int i, c2_t<R> v) { pw[i] = pkey(cabs2<R>(v)); });
+}
+
+template <typename R>
+__global__ void __launch_bounds__(1024) k_comb_select(V12Dev d) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  using K = key_t<R>;
+  __shared__ SelShared<K> ss;
+  const int c = blockIdx.x, slot = blockIdx.y, W = d.W;
+  const K *pw = (const K *)d.comb_pw + ((long)slot * d.comb_loops + c) * W;
+  if (W * sizeof(K) <= SEL_KEYS) {
+    K *keys = (K *)smem;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < W; i += blockDim.x) keys[i] = pw[i];
+    __syncthreads();
+    comb_select<K>(d, c, slot, [=](int i) { return keys[i]; }, ss);
+  } else {
+    comb_select<K>(d, c, slot, [=](int i) { return pw[i]; }, ss);
+  }
+  comb_last_list(d, slot);
+}
+
+// One Stockham stage over `narr` arrays of N points per slot (plan-time
+// transforms of up to 2^30 points and v3's long combs).
 template <typename R>
 __global__ void __launch_bounds__(256) k_fft_stage(const c2_t<R> *src, c2_t<R> *dst, int N, int Ns, int radix,
                                                    long arr_stride, int narr, long slot_stride,
@@ -448,47 +625,6 @@ __global__ void __launch_bounds__(256) k_fft_stage(const c2_t<R> *src, c2_t<R> *
   const int arr = (int)(g / per), j = (int)(g - (long)arr * per);
   const long base = (long)slot * slot_stride + (long)arr * arr_stride;
   stockham_stage<R>(src + base, dst + base, N, Ns, radix, j, tw);
-}
-
-// Power, top-2k selection and voting of loop j after a global-memory FFT.
-template <typename R>
-__global__ void __launch_bounds__(1024) k_select_vote(V12Dev d) {
-  __shared__ int hist[264], scan[64];
-  extern __shared__ int Js[];
-  const int j = blockIdx.x, slot = blockIdx.y;
-  const bool loc = j < d.L_loc;
-  const int B = loc ? d.B_loc : d.B_est;
-  const long off = loc ? (long)j * d.B_loc : (long)d.L_loc * d.B_loc + (long)(j - d.L_loc) * d.B_est;
-  const c2_t<R> *xs = (const c2_t<R> *)d.xs + (long)slot * d.xs_size + off;
-  if (d.xs32) {
-    float2 *xs32 = (float2 *)d.xs32 + (long)slot * d.xs_size + off;
-    for (int i = threadIdx.x; i < B; i += blockDim.x) xs32[i] = make_float2((float)xs[i].x, (float)xs[i].y);
-  }
-  block_top_indices_f<key_t<R>>([xs](int i) { return pkey(cabs2<R>(xs[i])); }, B, d.num, Js, hist, scan);
-  int *Jg = d.J + ((long)slot * d.L + j) * d.num;
-  for (int i = threadIdx.x; i < d.num; i += blockDim.x) Jg[i] = Js[i];
-}
-
-template <typename R, typename In>
-__global__ void __launch_bounds__(256) k_comb_gather(V12Dev d) {
-  const int slot = blockIdx.z, c = blockIdx.y, W = d.W;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= W) return;
-  const int *rp = d.rparams + (long)slot * d.rp_stride;
-  const long sigma = d.n / W, offset = rp[2 * d.L + c];
-  const In *x = (const In *)d.inputs[slot];
-  ((c2_t<R> *)d.comb_buf)[((long)slot * d.comb_loops + c) * W + i] = cvt_in<R>(__ldg(x + offset + i * sigma));
-}
-
-template <typename R>
-__global__ void __launch_bounds__(1024) k_comb_select(V12Dev d) {
-  __shared__ int hist[264], scan[64];
-  extern __shared__ int Js[];
-  const int c = blockIdx.x, slot = blockIdx.y, W = d.W;
-  const c2_t<R> *v = (const c2_t<R> *)d.comb_buf + ((long)slot * d.comb_loops + c) * W;
-  block_top_indices_f<key_t<R>>([v](int i) { return pkey(cabs2<R>(v[i])); }, W, d.num, Js, hist, scan);
-  unsigned *bits = d.comb_bits + (long)slot * ((W + 31) >> 5);
-  for (int i = threadIdx.x; i < d.num; i += blockDim.x) atomicOr(&bits[Js[i] >> 5], 1u << (Js[i] & 31));
 }
 
 // FFT of `narr` arrays per slot held at a (ping) with b as scratch; the
@@ -1447,33 +1583,47 @@ __global__ void k_scatter_dense(const int *out_idx, const c2_t<R> *out_val, cons
 // ---------------------------------------------------------------- launch --
 
 int v12_max_fft(int prec) { return prec == PREC_FP64 ? 8192 : 16384; }
-int v12_max_fft_any() { return 1 << 20; }
 
-static void fft_shape(int N, int &T, int &per) {
-  T = N / 4;
-  if (T > 1024) T = 1024;
-  if (T < 32) T = 32;
-  per = (N / 4 + T - 1) / T;
-}
+// Butterflies per thread and radix-4 stage of an FP64 one-CTA FFT.
+static int one_cta_per(int N) { return std::max(1, N / 4 / 1024); }
+
+// Threads of a selection over N keys: about eight per thread.
+static int select_threads(int N) { return std::min(1024, std::max(128, N / 8)); }
 
 template <typename R, typename In>
 static cudaError_t launch_comb(const V12Dev &d, int nslots, cudaStream_t s) {
-  int T, per;
-  fft_shape(d.W, T, per);
-  const size_t sm = BucketSmem<R>::bytes(d.W, d.num);
-  dim3 grid(d.comb_loops, nslots);
   cudaError_t e;
+  if (d.comb_pw) {
+    const int W = d.W, m2 = fft_m2(W);
+    const FftShape f = fft_shape2(W, W, sizeof(c2_t<R>));
+    const size_t sa = sizeof(c2_t<R>) * f.elems[0], sb = sizeof(c2_t<R>) * f.elems[1];
+    const size_t sk = (size_t)W * sizeof(key_t<R>) <= SEL_KEYS ? (size_t)W * sizeof(key_t<R>) : 0;
+    if ((e = set_smem(k_comb_a<R, In>, sa)) || (e = set_smem(k_comb_b<R>, sb)) || (e = set_smem(k_comb_select<R>, sk)))
+      return e;
+    k_comb_a<R, In><<<dim3(fft_ctas(f.elems[0], W / m2, W), d.comb_loops, nslots), f.elems[0] / 4, sa, s>>>(
+        d, f.elems[0]);
+    k_comb_b<R><<<dim3(fft_ctas(f.elems[1], m2, W), d.comb_loops, nslots), f.elems[1] / 4, sb, s>>>(d, f.elems[1]);
+    k_comb_select<R><<<dim3(d.comb_loops, nslots), select_threads(W), sk, s>>>(d);
+    note_launches(3);
+    return cudaGetLastError();
+  }
+  const int T = OneCta<R>::threads(d.W);
+  const size_t sm = OneCta<R>::bytes(d.W);
+  dim3 grid(d.comb_loops, nslots);
 #define SFFT_COMB(P)                                             \
   case P:                                                        \
     if ((e = set_smem(k_comb<R, P, In>, sm))) return e;          \
     k_comb<R, P, In><<<grid, T, sm, s>>>(d);                     \
     break;
-  switch (per) {
-    SFFT_COMB(1)
-    SFFT_COMB(2)
-    SFFT_COMB(4)
-    default:
-      return cudaErrorInvalidValue;
+  if constexpr (sizeof(R) == 4) {
+    switch (1) { SFFT_COMB(1) }
+  } else {
+    switch (one_cta_per(d.W)) {
+      SFFT_COMB(1)
+      SFFT_COMB(2)
+      default:
+        return cudaErrorInvalidValue;
+    }
   }
 #undef SFFT_COMB
   note_launches(1);
@@ -1482,29 +1632,42 @@ static cudaError_t launch_comb(const V12Dev &d, int nslots, cudaStream_t s) {
 
 template <typename R>
 static cudaError_t launch_bucket(const V12Dev &d, int nslots, cudaStream_t s) {
-  const int Bmax = d.B_loc > d.B_est ? d.B_loc : d.B_est;
-  // FP64: two butterflies per thread and stage -- half-size CTAs, two per SM,
-  // so one CTA's stage barriers overlap the other's FP64 arithmetic
-  // (measured 0.52 -> 0.455 ms per 32 signals at n = 2^22, k = 100; the FP32
-  // form is faster with one butterfly per thread)
-  int T = sizeof(R) == 8 ? Bmax / 8 : Bmax / 4, per;
-  if (T > 1024) T = 1024;
-  if (T < 32) T = 32;
-  per = (Bmax / 4 + T - 1) / T;
-  const size_t sm = BucketSmem<R>::bytes(Bmax, d.num);
-  dim3 grid(d.L, nslots);
   cudaError_t e;
+  const int Bmax = d.B_loc > d.B_est ? d.B_loc : d.B_est;
+  if (d.pw) {
+    const FftShape f = fft_shape2(d.B_loc, d.B_est, sizeof(c2_t<R>));
+    const size_t kl = (size_t)d.B_loc * sizeof(key_t<R>), ke = (size_t)d.B_est * sizeof(key_t<R>);
+    const size_t sa = sizeof(c2_t<R>) * f.elems[0], sb = sizeof(c2_t<R>) * f.elems[1];
+    const size_t sk = std::max(kl <= SEL_KEYS ? kl : 0, ke <= SEL_KEYS ? ke : 0);
+    if ((e = set_smem(k_bucket_a<R>, sa)) || (e = set_smem(k_bucket_b<R>, sb)) ||
+        (e = set_smem(k_bucket_select<R>, sk)))
+      return e;
+    const int ml = fft_m2(d.B_loc), me = fft_m2(d.B_est);
+    const int al = fft_ctas(f.elems[0], d.B_loc / ml, d.B_loc), ae = fft_ctas(f.elems[0], d.B_est / me, d.B_est);
+    const int bl = fft_ctas(f.elems[1], ml, d.B_loc), be = fft_ctas(f.elems[1], me, d.B_est);
+    k_bucket_a<R><<<dim3(d.L_loc * al + d.L_est * ae, nslots), f.elems[0] / 4, sa, s>>>(d, f.elems[0], al, ae);
+    k_bucket_b<R><<<dim3(d.L_loc * bl + d.L_est * be, nslots), f.elems[1] / 4, sb, s>>>(d, f.elems[1], bl, be);
+    k_bucket_select<R><<<dim3(d.L, nslots), select_threads(Bmax), sk, s>>>(d);
+    note_launches(2);  // the third is counted with the stage kernels
+    return cudaGetLastError();
+  }
+  const int T = OneCta<R>::threads(Bmax);
+  const size_t sm = OneCta<R>::bytes(Bmax);
+  dim3 grid(d.L, nslots);
 #define SFFT_BUCKET(P)                                        \
   case P:                                                     \
     if ((e = set_smem(k_bucket<R, P>, sm))) return e;         \
     k_bucket<R, P><<<grid, T, sm, s>>>(d);                    \
     break;
-  switch (per) {
-    SFFT_BUCKET(1)
-    SFFT_BUCKET(2)
-    SFFT_BUCKET(4)
-    default:
-      return cudaErrorInvalidValue;
+  if constexpr (sizeof(R) == 4) {
+    switch (1) { SFFT_BUCKET(1) }
+  } else {
+    switch (one_cta_per(Bmax)) {
+      SFFT_BUCKET(1)
+      SFFT_BUCKET(2)
+      default:
+        return cudaErrorInvalidValue;
+    }
   }
 #undef SFFT_BUCKET
   return cudaGetLastError();
@@ -1594,27 +1757,10 @@ static cudaError_t launch_estimate(const V12Dev &d, int nslots, cudaStream_t s) 
 template <typename R, typename In>
 static cudaError_t run_typed(const V12Dev &d, int nslots, cudaStream_t s, StageEvents *se) {
   cudaError_t e;
-  using V = c2_t<R>;
   if ((e = cudaMemsetAsync(d.counters, 0, sizeof(int) * CNT_STRIDE * nslots, s))) return e;
   mark(se, s);
   if (d.version == 1) {
-    if ((e = cudaMemsetAsync(d.comb_bits, 0, sizeof(unsigned) * ((d.W + 31) >> 5) * nslots, s))) return e;
-    if (!d.large_comb) {
-      if ((e = launch_comb<R, In>(d, nslots, s))) return e;
-    } else {
-      dim3 g((d.W + 255) / 256, d.comb_loops, nslots);
-      k_comb_gather<R, In><<<g, 256, 0, s>>>(d);
-      if ((e = cudaGetLastError())) return e;
-      if ((e = global_fft<R>((V *)d.comb_buf, (V *)d.comb_tmp, d.W, d.comb_loops, d.W, (long)d.comb_loops * d.W,
-                             nslots, (const V *)d.tw_comb, s)))
-        return e;
-      k_comb_select<R><<<dim3(d.comb_loops, nslots), 1024, sizeof(int) * d.num, s>>>(d);
-      if ((e = cudaGetLastError())) return e;
-      note_launches(2);
-    }
-    k_comb_list<<<nslots, 1024, 0, s>>>(d);
-    if ((e = cudaGetLastError())) return e;
-    note_launches(1);
+    if ((e = launch_comb<R, In>(d, nslots, s))) return e;
   }
   mark(se, s);
   if (sizeof(R) == 4) {
@@ -1627,18 +1773,7 @@ static cudaError_t run_typed(const V12Dev &d, int nslots, cudaStream_t s, StageE
   }
   if ((e = cudaGetLastError())) return e;
   mark(se, s);
-  if (!d.large_buckets) {
-    if ((e = launch_bucket<R>(d, nslots, s))) return e;
-  } else {
-    V *xs = (V *)d.xs, *tmp = (V *)d.xs_tmp;
-    const long locsz = (long)d.L_loc * d.B_loc;
-    if ((e = global_fft<R>(xs, tmp, d.B_loc, d.L_loc, d.B_loc, d.xs_size, nslots, (const V *)d.tw_loc, s))) return e;
-    if ((e = global_fft<R>(xs + locsz, tmp + locsz, d.B_est, d.L_est, d.B_est, d.xs_size, nslots,
-                           (const V *)d.tw_est, s)))
-      return e;
-    k_select_vote<R><<<dim3(d.L, nslots), 1024, sizeof(int) * d.num, s>>>(d);
-    if ((e = cudaGetLastError())) return e;
-  }
+  if ((e = launch_bucket<R>(d, nslots, s))) return e;
   {
     const long cmax = std::min<long>(d.W, (long)d.comb_loops * d.num);
     if (d.version == 1 && 4 * cmax < d.q_loc) {
@@ -1741,6 +1876,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist32(PersistProg p) {
   extern __shared__ __align__(128) unsigned char psmem[];
   __shared__ PersistGroup sg;      // the plan of the current item
   __shared__ EcShared<PT> ecsh;
+  __shared__ SelShared<unsigned> ss;
   __shared__ PersistItem sitem;
   __shared__ int s_ok;
   int *head = p.state, *abort = p.state + 1, *dep = p.state + 2;
@@ -1777,12 +1913,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist32(PersistProg p) {
     if (s_ok) {
       switch (w.kind) {
         case PK_COMB:
-          if (sg.per_comb == 1)
-            comb_block<float, 1, In>(d, w.idx, w.slot, psmem);
-          else if (sg.per_comb == 2)
-            comb_block<float, 2, In>(d, w.idx, w.slot, psmem);
-          else
-            comb_block<float, 4, In>(d, w.idx, w.slot, psmem);
+          comb_block<float, 1, In>(d, w.idx, w.slot, psmem, ss);
           break;
         case PK_FOLD:
           for (int c = 0; c < sg.fold_chunks; c++)
@@ -1792,12 +1923,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist32(PersistProg p) {
           comb_list_block(d, w.slot);
           break;
         case PK_BUCKET:
-          if (sg.per_bucket == 1)
-            bucket_block<float, 1>(d, w.idx, w.slot, psmem);
-          else if (sg.per_bucket == 2)
-            bucket_block<float, 2>(d, w.idx, w.slot, psmem);
-          else
-            bucket_block<float, 4>(d, w.idx, w.slot, psmem);
+          bucket_block<float, 1>(d, w.idx, w.slot, psmem, ss);
           break;
         case PK_VOTE: {  // loop j, buckets [i0, i0 + VB_BUCKETS)
           const int nbc = (d.num + VB_BUCKETS - 1) / VB_BUCKETS, j = w.idx / nbc;
@@ -1826,16 +1952,9 @@ bool persist_eligible(const V12Dev &d) {
          d.W >= 32 && d.W <= mx && d.B_loc <= mx && d.B_est <= mx && d.comb_loops <= 64;
 }
 
-static int per_of(int N) {
-  const int per = (N / 4 + PT - 1) / PT;
-  return per <= 1 ? 1 : per <= 2 ? 2 : 4;
-}
-
 void persist_shape(PersistGroup &g) {
   V12Dev &d = g.d;
   if (d.xs_perm && d.L > 24) d.xs_perm = 0;  // the comb-residue items hold L x PT values in shared memory
-  g.per_comb = per_of(d.W);
-  g.per_bucket = per_of(std::max(d.B_loc, d.B_est));
   g.fold_chunks = 8;
   g.nfold = (int)((d.xs_size * 4 + (long)PT * g.fold_chunks - 1) / ((long)PT * g.fold_chunks));
   g.vote_cmax = (int)std::min<long>(d.W, (long)d.comb_loops * d.num);
@@ -1851,7 +1970,7 @@ size_t persist_smem(const PersistGroup *groups, int ngroups) {
   size_t m = 0;
   for (int i = 0; i < ngroups; i++) {
     const V12Dev &d = groups[i].d;
-    m = std::max(m, BucketSmem<float>::bytes(std::max(d.W, std::max(d.B_loc, d.B_est)), d.num));
+    m = std::max(m, OneCta<float>::bytes(std::max(d.W, std::max(d.B_loc, d.B_est))));
     if (groups[i].est_comb) m = std::max(m, sizeof(float2) * (size_t)PT * d.L);
   }
   return m;
