@@ -128,7 +128,7 @@ struct PlanImpl {
   int win_half_a = 0, win_half_b = 0;
   // workspace
   int slots = 0;
-  DBuf xs, xs32, xs_tmp, pw, comb_tmp, comb_pw, J, score, hits, comb_bits, comb_list, counters, out_idx, out_val;
+  DBuf xs, xs32, xs_tmp, pw, comb_tmp, comb_pw, J, sel_bits, score, hits, comb_bits, comb_list, counters, out_idx, out_val;
   DBuf man, man_tmp, g1, g2, perm, est_f, est_v, map_keys, map_vals, map_list;
   DBuf rparams, inputs, dense_ptrs, in_stage, dense_stage, trace, cnt_stash;
   std::vector<unsigned> epoch;
@@ -366,6 +366,7 @@ bool ensure_slots(PlanImpl &P, int want) {
                      !P.comb_pw.ensure(ks * (size_t)p.Comb_loops * p.W_Comb * S)))
       return false;
     if (!P.xs.ensure(cs * p.x_samp_size * S) || !P.J.ensure(sizeof(int) * L * p.B_thresh * S) ||
+        !P.sel_bits.ensure(sizeof(unsigned) * (size_t)p.loops_loc * ((p.B_loc + 31) / 32) * S) ||
         !P.hits.ensure(sizeof(int) * P.hit_cap * S) ||
         !P.comb_bits.ensure(sizeof(unsigned) * (size_t)p.Comb_loops * ((p.W_Comb + 31) / 32) * S) ||
         !P.comb_list.ensure(sizeof(int) * p.W_Comb * S) || !P.out_idx.ensure(sizeof(int) * P.out_cap * S) ||
@@ -514,6 +515,7 @@ sfft::V12Dev v12_view(PlanImpl &P) {
   d.win32_loc = P.win32_a.p;
   d.win32_est = P.win32_b.p;
   d.J = P.J.as<int>();
+  d.sel_bits = P.sel_bits.as<unsigned>();
   d.score = P.score.as<unsigned>();
   d.hits = P.hits.as<int>();
   d.comb_bits = P.comb_bits.as<unsigned>();
@@ -612,6 +614,7 @@ void shift_view(PlanImpl &P, sfft::V12Dev &d, int base, bool own_out) {
   shift(d.comb_tmp, cs * (size_t)d.comb_loops * d.W, base);
   shift(d.comb_pw, cs / 2 * (size_t)d.comb_loops * d.W, base);
   shift(d.J, sizeof(int) * (size_t)d.L * d.num, base);
+  shift(d.sel_bits, sizeof(unsigned) * (size_t)d.L_loc * ((d.B_loc + 31) / 32), base);
   shift(d.score, sizeof(unsigned) * (size_t)d.n, base);
   shift(d.hits, sizeof(int) * (size_t)d.hit_cap, base);
   shift(d.comb_bits, sizeof(unsigned) * (size_t)d.comb_loops * ((d.W + 31) / 32), base);
@@ -1292,7 +1295,7 @@ long sfft_plan_footprint(const sfft_plan *plan) {
     return -1;
   }
   const DBuf *bufs[] = {&P->taps_a, &P->taps_b, &P->win_a, &P->win_b, &P->win32_a, &P->win32_b, &P->tw_a,
-                        &P->tw_b, &P->tw_c, &P->xs, &P->xs32, &P->xs_tmp, &P->pw, &P->comb_tmp, &P->comb_pw, &P->J,
+                        &P->tw_b, &P->tw_c, &P->xs, &P->xs32, &P->xs_tmp, &P->pw, &P->comb_tmp, &P->comb_pw, &P->J, &P->sel_bits,
                         &P->score, &P->hits, &P->comb_bits, &P->comb_list, &P->counters, &P->out_idx,
                         &P->out_val, &P->man, &P->man_tmp, &P->g1, &P->g2, &P->perm, &P->est_f, &P->est_v, &P->map_keys,
                         &P->map_vals, &P->map_list, &P->rparams, &P->inputs, &P->dense_ptrs, &P->in_stage,

@@ -58,6 +58,7 @@ struct V12Dev {
   // candidates of one residue reads in a loop are G consecutive entries.
   int xs_perm;
   int *J;                   // L * num per slot
+  unsigned *sel_bits;       // one bit per bucket of the location loops: L_loc * ceil(B_loc / 32) words per slot
   unsigned *score;          // n per slot: (epoch << 8) | votes
   int *hits;                // hit_cap per slot
   unsigned *comb_bits;      // comb_loops planes of W/32 words per slot
@@ -108,7 +109,6 @@ struct PersistGroup {
   int gslot0;        // first global signal slot of this plan
   int slots;         // its signals
   int fold_chunks;   // 1024-thread chunks of the fold per item
-  int vote_cmax, vote_chunks; // comb residues at most; unused (1)
   int est_comb;      // 1: estimation by comb residue (1024 candidates per item), 0: random lookups
   int est_chunks;    // random lookups: 1024-candidate chunks per item
   int nfold, nvote, nest;     // items per signal of those stages

@@ -102,6 +102,8 @@ extern "C" long sfft_exec_noalloc(sfft_plan *plan, const void *d_in, int in_type
   if (d.prec == PREC_FP64) off += up256(8 * (size_t)d.xs_size);
   const size_t o_J = off;
   off += up256(sizeof(int) * (size_t)L * d.num);
+  const size_t o_sel = off;
+  off += up256(sizeof(unsigned) * (size_t)d.L_loc * ((d.B_loc + 31) / 32));
   const size_t o_hits = off;
   off += up256(sizeof(int) * (size_t)hit_cap);
   const size_t o_bits = off;
@@ -164,6 +166,7 @@ extern "C" long sfft_exec_noalloc(sfft_plan *plan, const void *d_in, int in_type
   d.xs32 = d.prec == PREC_FP64 ? base + o_xs32 : nullptr;
   d.xs_tmp = d.pw = d.comb_tmp = d.comb_pw = nullptr;  // the plan's; here every FFT runs in one CTA
   d.J = (int *)(base + o_J);
+  d.sel_bits = (unsigned *)(base + o_sel);
   d.score = (unsigned *)(base + o_score);
   d.hits = (int *)(base + o_hits);
   d.comb_bits = (unsigned *)(base + o_bits);

@@ -286,169 +286,237 @@ __global__ void __launch_bounds__(1024) k_comb(V12Dev d) {
   comb_last_list(d, blockIdx.y);
 }
 
-// Voting of the location loops, one thread per (loop, selected bucket,
-// position): positions p in [J*q - floor(q/2), +q) (mod n)
-// map to frequencies f = p * a (mod n); each gets one vote (v2: only if
-// f mod W is a comb residue); reaching the threshold appends f to the
-// hits (computefourier-1.0-2.0.cc:91-116, :125-184).  Counters carry the
-// exec's epoch in their upper 24 bits, so they never need clearing.
-// One vote for frequency f: the counter is (epoch << 8) | votes, so a
-// counter from an earlier execution restarts at 1.  The vote that reaches
-// the threshold records the frequency (v1, and v2 in the voted mode).
-// Tags only grow between clears of the counters, so an atomic max with
-// (epoch << 8) resets a counter of an earlier execution to zero votes and
-// leaves one of this execution alone; the atomic add that follows (same
-// address, same thread: ordered after it) returns this vote's count.  One
-// round trip, no compare-and-swap loop.  Plain v2 builds no hit list from
-// its votes -- every frequency they reach is a comb candidate, all of
-// which are estimated (computefourier-1.0-2.0.cc:505-512) -- so its votes
-// only count: both atomics are reductions without a returned value, and
-// the voting threads do not wait for them.
-// v2's counters are stored residue-major, frequency f = rep W + r at
-// r (n / W) + rep: the votes of a round fall on the few comb residues'
-// blocks of n / W consecutive counters instead of all over the n of them,
-// which keeps the touched counters dense in L2 and DRAM.
-__device__ __forceinline__ void vote_one(const V12Dev &d, int slot, unsigned f, unsigned ep, unsigned *score,
-                                         int *cnt) {
-  unsigned *c = &score[f];
-  if (d.version == 1) {
-    const int lw = dlog2((unsigned)d.W), lr = dlog2((unsigned)d.n) - lw;
-    c = &score[((f & ((unsigned)d.W - 1u)) << lr) | (f >> lw)];
+// ---------------------------------------------------------------- voting --
+//
+// In location loop j, frequency f gets a vote iff its position p = f ai_j (mod
+// n) lies in the range [J q - q / 2, + q) (mod n) of a selected bucket J
+// (v2: and f mod W is a comb residue; computefourier-1.0-2.0.cc:91-116,
+// :125-184), that is iff bucket ((p + q / 2) mod n) / q is selected.  No count
+// is added to in global memory; one thread or block owns each frequency:
+//
+//   k_vote_residue  (v2) a block counts the n / W frequencies of one comb
+//                   residue in shared memory, one step per (loop, selected
+//                   bucket): the range of J holds the positions congruent to
+//                   r ai (mod W), at most q / W + 1 of them.
+//   k_vote_cands    (v2) one thread per comb candidate, one bit test per loop
+//                   in the bitmap of selected buckets the selection leaves.
+//   k_vote_ranges   (v1) one thread per position of the selected ranges, the
+//                   same bit tests; the first loop that selected a frequency
+//                   owns it.
+//
+// v2 takes the first form when its steps, 2 k (q / W + 1) per residue and
+// loop, are fewer than the n / W bit tests of the second.  Frequencies that
+// reach the threshold are collected per block: one returning atomic a warp
+// on a signal's hit counter, about 2 ns each at one address, takes 200 us for
+// four voted signals of n = 2^22, k = 500.  Kernel times: those signals, two
+// atomics per vote 283 -> 48 us (bit tests with the block's hits: 225 us with
+// warp atomics); 32 plain signals of n = 2^22, k = 100: 45 -> 27 us (bit
+// tests: 46); 64 v1 signals of n = 2^16: 28 -> 18 us.
+//
+// The counts stay in score for diagnostics: (epoch << 8) | votes, so that
+// counts of earlier executions need no clearing; v2 keeps them
+// residue-major, frequency f = rep W + r at r (n / W) + rep, where a
+// residue's counts are consecutive.
+
+// The bitmaps of the location loops: in shared memory unless they are large.
+constexpr int VOTE_SMEM = 32 * 1024;
+__host__ __device__ __forceinline__ int vote_words(int B) { return (B + 31) >> 5; }
+static size_t vote_smem(const V12Dev &d) {
+  const size_t b = sizeof(unsigned) * (size_t)d.L_loc * vote_words(d.B_loc);
+  return b <= VOTE_SMEM ? b : 0;
+}
+__device__ __forceinline__ const unsigned *vote_bits(const V12Dev &d, int slot, unsigned *smem) {
+  const int words = d.L_loc * vote_words(d.B_loc);
+  const unsigned *src = d.sel_bits + (long)slot * words;
+  if (words * (int)sizeof(unsigned) > VOTE_SMEM) return src;
+  for (int i = threadIdx.x; i < words; i += blockDim.x) smem[i] = src[i];
+  __syncthreads();
+  return smem;
+}
+
+// Hits of a block (v1, and v2 in the voted mode): places are taken within
+// the block first, then one place range for all of them in the signal's list.
+struct VoteHits {
+  int n, base;
+};
+__device__ __forceinline__ void hits_begin(VoteHits &h) {  // a barrier follows before the first place
+  if (threadIdx.x == 0) h.n = 0;
+}
+__device__ __forceinline__ void hits_place(const V12Dev &d, int slot, VoteHits &h) {
+  __syncthreads();
+  if (threadIdx.x == 0 && h.n) {
+    int *cnt = d.counters + slot * CNT_STRIDE;
+    h.base = atomicAdd(&cnt[CNT_HITS], h.n);
+    atomicAdd(&cnt[CNT_VOTED], h.n);
+    if (h.base + h.n > d.hit_cap) atomicOr(&cnt[CNT_ERR], ERR_HIT_OVERFLOW);
   }
-  atomicMax(c, ep << 8);
-  if (d.version == 1 && !d.voted) {
-    atomicAdd(c, 1u);
-    return;
+  __syncthreads();
+}
+__device__ __forceinline__ void hits_store(const V12Dev &d, int slot, const VoteHits &h, int place, unsigned f) {
+  if (h.base + place < d.hit_cap) d.hits[(long)slot * d.hit_cap + h.base + place] = (int)f;
+}
+
+__device__ __forceinline__ unsigned vote_in(const V12Dev &d, const unsigned *sb, int j, unsigned ai, unsigned f) {
+  const unsigned mask = (unsigned)d.n - 1u, q = (unsigned)d.q_loc;
+  const unsigned b = ((f * ai + (q >> 1)) & mask) >> dlog2(q);
+  return (sb[j * vote_words(d.B_loc) + (int)(b >> 5)] >> (b & 31u)) & 1u;
+}
+
+// v2: the votes of comb candidates h0 + u blockDim + thread, u < U
+// (candidates as in cand_freq: residue-major).
+template <int U>
+__device__ __forceinline__ void vote_cands(const V12Dev &d, int slot, long h0, const unsigned *sb, VoteHits &hits) {
+  const int *rp = d.rparams + (long)slot * d.rp_stride;
+  const unsigned ep = (unsigned)rp[2 * d.L + d.comb_loops];
+  const int lw = dlog2((unsigned)d.W), lr = dlog2((unsigned)d.n) - lw;
+  const long total = (long)d.counters[slot * CNT_STRIDE + CNT_COMB] << lr;
+  const int *list = d.comb_list + (long)slot * d.W;
+  unsigned *score = d.score + (long)slot * d.n;
+  unsigned f[U], votes[U];
+  if (d.voted) {
+    hits_begin(hits);
+    __syncthreads();
   }
-  const unsigned nv = atomicAdd(c, 1u) + 1u;
-  if ((int)(nv & 255u) == d.thresh) {
-    atomicAdd(&cnt[CNT_VOTED], 1);
-    if (d.version == 0 || d.voted) {
-      const int pos = atomicAdd(&cnt[CNT_HITS], 1);
-      if (pos < d.hit_cap)
-        d.hits[(long)slot * d.hit_cap + pos] = (int)f;
-      else
-        atomicOr(&cnt[CNT_ERR], ERR_HIT_OVERFLOW);
-    }
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const long h = h0 + (long)u * blockDim.x + threadIdx.x;
+    f[u] = h < total ? (((unsigned)h & ((1u << lr) - 1u)) << lw) | (unsigned)list[h >> lr] : 0u;
+    votes[u] = 0;
+  }
+  for (int j = 0; j < d.L_loc; j++) {
+    const unsigned ai = (unsigned)rp[d.L + j];
+#pragma unroll
+    for (int u = 0; u < U; u++) votes[u] += vote_in(d, sb, j, ai, f[u]);
+  }
+  int place[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    if (h0 + (long)u * blockDim.x + threadIdx.x >= total) votes[u] = 0;
+    // residue f mod W, repetition f / W
+    if (votes[u]) score[((f[u] & ((1u << lw) - 1u)) << lr) | (f[u] >> lw)] = (ep << 8) | votes[u];
+    place[u] = d.voted && (int)votes[u] >= d.thresh ? atomicAdd(&hits.n, 1) : -1;
+  }
+  if (d.voted) {
+    hits_place(d, slot, hits);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (place[u] >= 0) hits_store(d, slot, hits, place[u], f[u]);
   }
 }
 
-__global__ void __launch_bounds__(256) k_vote(V12Dev d) {
+template <int U>
+__global__ void __launch_bounds__(256) k_vote_cands(V12Dev d) {
+  extern __shared__ unsigned vb[];
+  __shared__ VoteHits hits;
+  const unsigned *sb = vote_bits(d, blockIdx.y, vb);
+  vote_cands<U>(d, blockIdx.y, (long)blockIdx.x * 256 * U, sb, hits);
+}
+
+// v2, one comb residue per block; n / W byte counters in shared memory (a
+// frequency gets at most one vote per loop, of at most 32).
+__device__ __forceinline__ void vote_residue(const V12Dev &d, int slot, int ridx, unsigned *cw, VoteHits &hits) {
+  const int *rp = d.rparams + (long)slot * d.rp_stride;
+  const unsigned mask = (unsigned)d.n - 1u, wm = (unsigned)d.W - 1u, q = (unsigned)d.q_loc;
+  const int lw = dlog2((unsigned)d.W), lr = dlog2((unsigned)d.n) - lw, words = (1 << lr) >> 2;
+  const unsigned r = (unsigned)d.comb_list[(long)slot * d.W + ridx], ep = (unsigned)rp[2 * d.L + d.comb_loops];
+  for (int i = threadIdx.x; i < words; i += blockDim.x) cw[i] = 0u;
+  hits_begin(hits);
+  __syncthreads();
+  for (int j = 0; j < d.L_loc; j++) {
+    const int *Js = d.J + ((long)slot * d.L + j) * d.num;
+    const unsigned a = (unsigned)rp[j], c = (r * (unsigned)rp[d.L + j]) & wm;
+    for (int t = threadIdx.x; t < d.num; t += blockDim.x) {
+      const unsigned low = ((unsigned)Js[t] * q - (q >> 1)) & mask;
+      for (unsigned k = (c - low) & wm; k < q; k += (unsigned)d.W) {
+        const unsigned rep = (((low + k) * a) & mask) >> lw;
+        atomicAdd(&cw[rep >> 2], 1u << (8 * (rep & 3u)));
+      }
+    }
+  }
+  __syncthreads();
+  uint4 *score = (uint4 *)(d.score + (long)slot * d.n + ((long)r << lr));
+  const unsigned tag = ep << 8;
+  for (int i = threadIdx.x; i < words; i += blockDim.x) {
+    const unsigned v = cw[i];
+    if (!v) continue;
+    score[i] = make_uint4(tag | (v & 255u), tag | ((v >> 8) & 255u), tag | ((v >> 16) & 255u), tag | (v >> 24));
+    if (d.voted) {
+      int c = 0;
+#pragma unroll
+      for (int b = 0; b < 4; b++) c += (int)((v >> (8 * b)) & 255u) >= d.thresh;
+      if (c) atomicAdd(&hits.n, c);
+    }
+  }
+  if (!d.voted) return;
+  hits_place(d, slot, hits);
+  if (!hits.n) return;
+  __syncthreads();  // every thread has read n
+  if (threadIdx.x == 0) hits.n = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < words; i += blockDim.x) {
+    const unsigned v = cw[i];
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+      if (v && (int)((v >> (8 * b)) & 255u) >= d.thresh)
+        hits_store(d, slot, hits, atomicAdd(&hits.n, 1), ((unsigned)(4 * i + b) << lw) | r);
+  }
+}
+
+__global__ void __launch_bounds__(256) k_vote_residue(V12Dev d) {
+  extern __shared__ unsigned cw[];
+  __shared__ VoteHits hits;
   const int slot = blockIdx.y;
+  if ((int)blockIdx.x >= d.counters[slot * CNT_STRIDE + CNT_COMB]) return;
+  vote_residue(d, slot, blockIdx.x, cw, hits);
+}
+
+// Whether v2's votes go by residue (see above): fewer steps than bit tests,
+// and the counters fit (n / W of 4 .. 32768).
+__host__ __device__ __forceinline__ bool vote_by_residue(const V12Dev &d) {
+  const long R = d.n / d.W;
+  return R >= 4 && R <= 32768 && (long)d.num * (d.q_loc / d.W + 1) < R;
+}
+
+// v1: VOTE_V positions of one loop's selected ranges per thread.
+constexpr int VOTE_V = 4;
+
+__global__ void __launch_bounds__(256) k_vote_ranges(V12Dev d, int per_loop_blocks) {
+  extern __shared__ unsigned vb[];
+  __shared__ VoteHits hits;
+  hits_begin(hits);
+  const int slot = blockIdx.y;
+  const unsigned *sb = vote_bits(d, slot, vb);
+  __syncthreads();
   const int q = d.q_loc, lq = dlog2(q);
-  const long per_loop = (long)d.num << lq;
-  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= per_loop * d.L_loc) return;
-  const int j = (int)(g / per_loop);
-  const long e = g - (long)j * per_loop;
+  const int j = blockIdx.x / per_loop_blocks, tile = blockIdx.x - j * per_loop_blocks;
+  const long per_loop = (long)d.num << lq, g0 = (long)tile * (256 * VOTE_V) + threadIdx.x;
   const int *Js = d.J + ((long)slot * d.L + j) * d.num;
   const int *rp = d.rparams + (long)slot * d.rp_stride;
-  const unsigned long long a = (unsigned)rp[j];
-  const unsigned ep = (unsigned)rp[2 * d.L + d.comb_loops];
-  const long n = d.n;
-  const unsigned long long mask = (unsigned long long)n - 1;
-  unsigned *score = d.score + (long)slot * n;
-  const unsigned *bits = d.comb_bits + (long)slot * d.comb_loops * ((d.W + 31) >> 5);
-  int *cnt = d.counters + slot * CNT_STRIDE;
-  {
-    const int i = (int)(e >> lq), o = (int)(e & (q - 1));
-    const long low = ((long)Js[i] * q - (q >> 1) + n) & (long)mask;
-    const unsigned long long p = ((unsigned long long)(low + o)) & mask;
-    const unsigned f = (unsigned)((p * a) & mask);
-    if (d.version == 1) {
-      const unsigned r = f & (unsigned)(d.W - 1);
-      if (!((bits[r >> 5] >> (r & 31)) & 1u)) return;
-    }
-    vote_one(d, slot, f, ep, score, cnt);
-  }
-}
-
-// v2 voting by residue enumeration: for selected bucket J and comb residue
-// r, the positions p of J's range whose frequency p a mod n lies in residue
-// class r mod W are p = c (mod W) with c = r a^-1 mod W -- one thread per
-// (loop, bucket, residue) visits exactly those.  Cheaper than the bitmap
-// walk below when the residues are few against the bucket width (many
-// light threads instead of a few threads with several votes each).
-__global__ void __launch_bounds__(256) k_vote_comb(V12Dev d, int cmax) {
-  const int slot = blockIdx.y;
-  const long per_loop = (long)d.num * cmax;
-  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= per_loop * d.L_loc) return;
-  const int j = (int)(g / per_loop);
-  const long e = g - (long)j * per_loop;
-  const int i = (int)(e / cmax), ri = (int)(e - (long)i * cmax);
-  int *cnt = d.counters + slot * CNT_STRIDE;
-  if (ri >= cnt[CNT_COMB]) return;
-  const unsigned r = (unsigned)d.comb_list[(long)slot * d.W + ri];
-  const int *rp = d.rparams + (long)slot * d.rp_stride;
-  const unsigned a = (unsigned)rp[j], ai = (unsigned)rp[d.L + j];
-  const unsigned ep = (unsigned)rp[2 * d.L + d.comb_loops];
-  const unsigned mask = (unsigned)d.n - 1u, wm = (unsigned)d.W - 1u;
-  const int q = d.q_loc;
-  const int J = d.J[((long)slot * d.L + j) * d.num + i];
-  const unsigned low = ((unsigned)J * (unsigned)q - (unsigned)(q >> 1) + (unsigned)d.n) & mask;
-  const unsigned c = (r * ai) & wm;
-  unsigned *score = d.score + (long)slot * d.n;
-  for (unsigned k = (c - low) & wm; k < (unsigned)q; k += (unsigned)d.W) {
-    const unsigned p = (low + k) & mask;
-    vote_one(d, slot, (p * a) & mask, ep, score, cnt);
-  }
-}
-
-// v2 voting by comb-key bitmap.  In location loop j a position p votes iff
-// its frequency p a mod n lies in an approved comb residue class, i.e. iff
-// p mod W is in K_j = {r ai mod W : r approved} (a ai = 1 mod W, W | n).  A
-// block builds K_j as a W-bit bitmap in shared memory; then each thread
-// takes 32 consecutive positions of one selected bucket's range at a time:
-// the 32 bits starting at (low + o) mod W (two words, funnel shift) name
-// exactly the positions that vote.  The reference walks the approved
-// residues in the same way through sorted (residue, key) pairs
-// (computefourier-1.0-2.0.cc:125-184); the votes are the same, in any order.
-constexpr int VB_BUCKETS = 64;   // selected buckets per block
-
-__device__ __forceinline__ void vote_bits_block(const V12Dev &d, int j, int i0, int slot, unsigned *kb) {
-  const int W = d.W, nw = W >> 5, L = d.L;
-  const int *rp = d.rparams + (long)slot * d.rp_stride;
-  const unsigned a = (unsigned)rp[j], ai = (unsigned)rp[L + j];
-  const unsigned ep = (unsigned)rp[2 * L + d.comb_loops];
-  const unsigned mask = (unsigned)d.n - 1u, wm = (unsigned)W - 1u;
-  int *cnt = d.counters + slot * CNT_STRIDE;
-  for (int w = threadIdx.x; w < nw; w += blockDim.x) kb[w] = 0u;
-  __syncthreads();
-  const int ncomb = cnt[CNT_COMB];
-  const int *list = d.comb_list + (long)slot * W;
-  for (int t = threadIdx.x; t < ncomb; t += blockDim.x) {
-    const unsigned c = ((unsigned)list[t] * ai) & wm;
-    atomicOr(&kb[c >> 5], 1u << (c & 31));
-  }
-  __syncthreads();
-  const int q = d.q_loc, nch = (q + 31) >> 5;
-  const int i1 = min(d.num, i0 + VB_BUCKETS);
-  const int tasks = (i1 - i0) * nch;
-  const int *Js = d.J + ((long)slot * L + j) * d.num;
-  unsigned *score = d.score + (long)slot * d.n;
-  for (int t = threadIdx.x; t < tasks; t += blockDim.x) {
-    const int i = i0 + t / nch, o0 = (t - (t / nch) * nch) << 5;
-    const unsigned low = ((unsigned)Js[i] * (unsigned)q - (unsigned)(q >> 1) + (unsigned)d.n) & mask;
-    const unsigned b0 = (low + (unsigned)o0) & wm;
-    const unsigned w0 = b0 >> 5;
-    unsigned word = __funnelshift_r(kb[w0], kb[(w0 + 1) & (unsigned)(nw - 1)], b0 & 31u);
-    const int rem = q - o0;
-    if (rem < 32) word &= (1u << rem) - 1u;
-    while (word) {
-      const int k = __ffs(word) - 1;
-      word &= word - 1u;
-      const unsigned p = (low + (unsigned)(o0 + k)) & mask;
-      vote_one(d, slot, (p * a) & mask, ep, score, cnt);
+  const unsigned mask = (unsigned)d.n - 1u, tag = (unsigned)rp[2 * d.L + d.comb_loops] << 8;
+  unsigned f[VOTE_V];
+  int place[VOTE_V];
+#pragma unroll
+  for (int v = 0; v < VOTE_V; v++) {
+    const long g = g0 + 256 * v;
+    place[v] = -1;
+    f[v] = 0;
+    if (g < per_loop) {
+      const unsigned e = (unsigned)g, J = (unsigned)Js[e >> lq];
+      const unsigned p = (J * (unsigned)q - (unsigned)(q >> 1) + (e & (unsigned)(q - 1))) & mask;
+      f[v] = (p * (unsigned)rp[j]) & mask;
+      unsigned before = 0, votes = 1;
+      for (int t = 0; t < j; t++) before |= vote_in(d, sb, t, (unsigned)rp[d.L + t], f[v]);
+      for (int t = j + 1; t < d.L_loc; t++) votes += vote_in(d, sb, t, (unsigned)rp[d.L + t], f[v]);
+      if (!before) {
+        d.score[(long)slot * d.n + f[v]] = tag | votes;
+        if ((int)votes >= d.thresh) place[v] = atomicAdd(&hits.n, 1);
+      }
     }
   }
-}
-
-__global__ void __launch_bounds__(256) k_vote_bits(V12Dev d) {
-  extern __shared__ unsigned vb_keys[];
-  const int nbc = (d.num + VB_BUCKETS - 1) / VB_BUCKETS;
-  const int j = blockIdx.x / nbc;
-  vote_bits_block(d, j, (blockIdx.x - j * nbc) * VB_BUCKETS, blockIdx.y, vb_keys);
+  hits_place(d, slot, hits);
+#pragma unroll
+  for (int v = 0; v < VOTE_V; v++)
+    if (place[v] >= 0) hits_store(d, slot, hits, place[v], f[v]);
 }
 
 // ---------------------------------------------------------------- bucket --
@@ -472,6 +540,11 @@ __device__ __forceinline__ LoopSpan loop_span(const V12Dev &d, int j) {
   return l;
 }
 
+// The bitmap of loop j's selected buckets (location loops only).
+__device__ __forceinline__ unsigned *sel_plane(const V12Dev &d, int slot, int j) {
+  return j < d.L_loc ? d.sel_bits + ((long)slot * d.L_loc + j) * vote_words(d.B_loc) : nullptr;
+}
+
 template <typename R, int PER>
 __device__ __forceinline__ void bucket_block(const V12Dev &d, int j, int slot, unsigned char *smem,
                                              SelShared<key_t<R>> &ss) {
@@ -488,8 +561,8 @@ __device__ __forceinline__ void bucket_block(const V12Dev &d, int j, int slot, u
     xs[p] = v;
     if (xs32) xs32[p] = make_float2((float)v.x, (float)v.y);
   }
-  block_select<key_t<R>>([&](int i) { return f.key(i); }, B, d.num, d.J + ((long)slot * d.L + j) * d.num, nullptr,
-                         ss);
+  block_select<key_t<R>>([&](int i) { return f.key(i); }, B, d.num, d.J + ((long)slot * d.L + j) * d.num,
+                         sel_plane(d, slot, j), ss);
 }
 
 template <typename R, int PER>
@@ -563,9 +636,9 @@ __global__ void __launch_bounds__(1024) k_bucket_select(V12Dev d) {
 #pragma unroll 4
     for (int i = threadIdx.x; i < l.B; i += blockDim.x) keys[i] = pw[i];
     __syncthreads();
-    block_select<K>([=](int i) { return keys[i]; }, l.B, d.num, J, nullptr, ss);
+    block_select<K>([=](int i) { return keys[i]; }, l.B, d.num, J, sel_plane(d, slot, j), ss);
   } else {
-    block_select<K>([=](int i) { return pw[i]; }, l.B, d.num, J, nullptr, ss);
+    block_select<K>([=](int i) { return pw[i]; }, l.B, d.num, J, sel_plane(d, slot, j), ss);
   }
 }
 
@@ -1775,18 +1848,19 @@ static cudaError_t run_typed(const V12Dev &d, int nslots, cudaStream_t s, StageE
   mark(se, s);
   if ((e = launch_bucket<R>(d, nslots, s))) return e;
   {
-    const long cmax = std::min<long>(d.W, (long)d.comb_loops * d.num);
-    if (d.version == 1 && 4 * cmax < d.q_loc) {
-      const long threads = (long)d.num * cmax * d.L_loc;
-      k_vote_comb<<<dim3((unsigned)((threads + 255) / 256), nslots), 256, 0, s>>>(d, (int)cmax);
-    } else if (d.version == 1 && d.W >= 32) {
-      const int nbc = (d.num + VB_BUCKETS - 1) / VB_BUCKETS;
-      const size_t sm = sizeof(unsigned) * (size_t)(d.W >> 5);
-      if ((e = set_smem(k_vote_bits, sm))) return e;
-      k_vote_bits<<<dim3((unsigned)(d.L_loc * nbc), nslots), 256, sm, s>>>(d);
+    const size_t sm = vote_smem(d);
+    const long residues = d.version ? std::min<long>(d.W, (long)d.comb_loops * d.num) : 0;
+    const long cands = d.version ? residues * (d.n / d.W) : 0;
+    if (d.version == 0) {
+      const int blocks = (int)(((long)d.num * d.q_loc + 256 * VOTE_V - 1) / (256 * VOTE_V));
+      k_vote_ranges<<<dim3((unsigned)(blocks * d.L_loc), nslots), 256, sm, s>>>(d, blocks);
+    } else if (vote_by_residue(d)) {
+      k_vote_residue<<<dim3((unsigned)residues, nslots), 256, d.n / d.W, s>>>(d);
+    } else if (cands * nslots >= (long)sm_count() * 4 * 8 * 256) {
+      // eight candidates per thread where that still gives every SM four blocks
+      k_vote_cands<8><<<dim3((unsigned)((cands + 2047) / 2048), nslots), 256, sm, s>>>(d);
     } else {
-      const long votes = ((long)d.num * d.q_loc) * d.L_loc;
-      k_vote<<<dim3((unsigned)((votes + 255) / 256), nslots), 256, 0, s>>>(d);
+      k_vote_cands<1><<<dim3((unsigned)((cands + 255) / 256), nslots), 256, sm, s>>>(d);
     }
     if ((e = cudaGetLastError())) return e;
     note_launches(1);
@@ -1815,6 +1889,7 @@ static cudaError_t run_typed(const V12Dev &d, int nslots, cudaStream_t s, StageE
 // item is skipped, so the kernel always ends.
 
 constexpr int PT = 1024;                 // threads of the executor's CTA
+constexpr int PERSIST_VOTES = 8;         // candidates per thread of a voting item
 constexpr long PERSIST_POLLS = 1L << 24;  // polls of a dependency (with back-off)
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
@@ -1877,6 +1952,7 @@ __global__ void __launch_bounds__(PT, 1) k_persist32(PersistProg p) {
   __shared__ PersistGroup sg;      // the plan of the current item
   __shared__ EcShared<PT> ecsh;
   __shared__ SelShared<unsigned> ss;
+  __shared__ VoteHits hits;
   __shared__ PersistItem sitem;
   __shared__ int s_ok;
   int *head = p.state, *abort = p.state + 1, *dep = p.state + 2;
@@ -1925,11 +2001,10 @@ __global__ void __launch_bounds__(PT, 1) k_persist32(PersistProg p) {
         case PK_BUCKET:
           bucket_block<float, 1>(d, w.idx, w.slot, psmem, ss);
           break;
-        case PK_VOTE: {  // loop j, buckets [i0, i0 + VB_BUCKETS)
-          const int nbc = (d.num + VB_BUCKETS - 1) / VB_BUCKETS, j = w.idx / nbc;
-          vote_bits_block(d, j, (w.idx - j * nbc) * VB_BUCKETS, w.slot, (unsigned *)psmem);
+        case PK_VOTE:
+          vote_cands<PERSIST_VOTES>(d, w.slot, (long)w.idx * PT * PERSIST_VOTES, vote_bits(d, w.slot, (unsigned *)psmem),
+                                    hits);
           break;
-        }
         default:  // PK_EST
           if (w.idx == 0 && threadIdx.x == 0) publish_count(d, w.slot, cand_total(d, w.slot));
           persist_est_any(d, sg, w.slot, w.idx, (float2 *)psmem, ecsh);
@@ -1957,10 +2032,8 @@ void persist_shape(PersistGroup &g) {
   if (d.xs_perm && d.L > 24) d.xs_perm = 0;  // the comb-residue items hold L x PT values in shared memory
   g.fold_chunks = 8;
   g.nfold = (int)((d.xs_size * 4 + (long)PT * g.fold_chunks - 1) / ((long)PT * g.fold_chunks));
-  g.vote_cmax = (int)std::min<long>(d.W, (long)d.comb_loops * d.num);
-  g.vote_chunks = 1;
-  g.nvote = d.L_loc * ((d.num + VB_BUCKETS - 1) / VB_BUCKETS);
-  const long cands = std::min<long>((long)g.vote_cmax * (d.n / d.W), (long)d.out_cap);
+  const long cands = std::min<long>(std::min<long>(d.W, (long)d.comb_loops * d.num) * (d.n / d.W), (long)d.out_cap);
+  g.nvote = (int)((cands + (long)PT * PERSIST_VOTES - 1) / ((long)PT * PERSIST_VOTES));
   g.est_comb = d.xs_perm != 0;
   g.est_chunks = g.est_comb ? 1 : 4;
   g.nest = (int)((cands + (long)PT * g.est_chunks - 1) / ((long)PT * g.est_chunks));
@@ -1971,6 +2044,7 @@ size_t persist_smem(const PersistGroup *groups, int ngroups) {
   for (int i = 0; i < ngroups; i++) {
     const V12Dev &d = groups[i].d;
     m = std::max(m, OneCta<float>::bytes(std::max(d.W, std::max(d.B_loc, d.B_est))));
+    m = std::max(m, vote_smem(d));
     if (groups[i].est_comb) m = std::max(m, sizeof(float2) * (size_t)PT * d.L);
   }
   return m;
@@ -2005,7 +2079,7 @@ void persist_items(const PersistGroup *groups, int ngroups, std::vector<PersistI
       }
       case PK_LIST: return 1.0;
       case PK_BUCKET: return 2.0 + std::max(d.B_loc, d.B_est) / 2048.0;
-      case PK_VOTE: return 1.0 + (double)VB_BUCKETS * ((d.q_loc + 31) / 32) / 512.0;
+      case PK_VOTE: return 1.0 + (double)PERSIST_VOTES * d.L_loc / 8.0;
       default: return 1.0 + (double)PT * G.est_chunks * d.L / 4000.0;
     }
   };
