@@ -1031,30 +1031,30 @@ __device__ __forceinline__ double2 value64(const V12Dev &d, const double2 *xs, i
                       A::div(A::sub(A::mul(v.x, h.y), A::mul(v.y, h.x)), den));
 }
 
-// Exact lower medians of all L FP64 values (used when the FP32 pre-selection
-// cannot prove which element is the median, e.g. ties).
-__device__ __noinline__ double2 median64_exact(const V12Dev &d, const double2 *xs, const int *rp, unsigned f) {
-  double vre[32], vim[32];
-  const int L = d.L;
+// Lower medians of the real and imaginary parts of the L values v of lanes 0
+// .. L - 1 (the element of rank (L - 1) / 2, ties in lane order); every lane
+// of the warp calls and receives them.
+__device__ __forceinline__ double2 warp_median64(double2 v, int L) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, m = (L - 1) >> 1;
+  const long long kx = okey(v.x), ky = okey(v.y);
+  int rx = 0, ry = 0;
   for (int j = 0; j < L; j++) {
-    const double2 v = value64(d, xs, j, f, (unsigned)rp[L + j]);
-    vre[j] = v.x;
-    vim[j] = v.y;
+    const long long a = __shfl_sync(FULL, kx, j), b = __shfl_sync(FULL, ky, j);
+    rx += a < kx || (a == kx && j < lane);
+    ry += b < ky || (b == ky && j < lane);
   }
-  const int m = (L - 1) >> 1;
-  double mre = 0, mim = 0;
-  for (int i = 0; i < L; i++) {
-    const long long ki = okey(vre[i]), kj = okey(vim[i]);
-    int rr = 0, ri = 0;
-    for (int jj = 0; jj < L; jj++) {
-      const long long a = okey(vre[jj]), b = okey(vim[jj]);
-      rr += (a < ki) || (jj < i && a == ki);
-      ri += (b < kj) || (jj < i && b == kj);
-    }
-    if (rr == m) mre = vre[i];
-    if (ri == m) mim = vim[i];
-  }
-  return make_double2(mre, mim);
+  const int sx = __ffs(__ballot_sync(FULL, lane < L && rx == m)) - 1;
+  const int sy = __ffs(__ballot_sync(FULL, lane < L && ry == m)) - 1;
+  return make_double2(__shfl_sync(FULL, v.x, sx), __shfl_sync(FULL, v.y, sy));
+}
+
+// The exact estimate of frequency f by one warp, one loop per lane.
+__device__ __forceinline__ double2 warp_estimate64(const V12Dev &d, const double2 *xs, const int *rp, unsigned f) {
+  const int lane = threadIdx.x & 31;
+  double2 v = make_double2(0.0, 0.0);
+  if (lane < d.L) v = value64(d, xs, lane, f, (unsigned)rp[d.L + lane]);
+  return warp_median64(v, d.L);
 }
 
 // Number of candidates of a slot: v1 hits, v2 every comb candidate (or,
@@ -1129,52 +1129,6 @@ __device__ __forceinline__ int proven_median(const float (&v)[LN], const float (
   return (below == m && above == Lr - 1 - m) ? idx : -1;
 }
 
-// Estimation work is dealt in chunks of one candidate per thread from a
-// per-slot queue (counters[CNT_EST]).  A block starts on the slot its SM is
-// assigned (%smid modulo the slot count) and moves on only when that slot
-// is exhausted, so the blocks resident on one SM read one slot's bucket
-// array and its random lookups hit in L1 far more often than when an SM
-// serves several slots at once.
-__device__ __forceinline__ unsigned sm_id() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%smid;" : "=r"(r));
-  return r;
-}
-
-struct EstChunk {
-  int slot;
-  long base, end;
-};
-
-__device__ __forceinline__ bool next_chunk(const V12Dev &d, int nslots, int chunk, int &slot, int &visited,
-                                           EstChunk &out) {
-  __shared__ EstChunk sc;
-  __syncthreads();  // the previous chunk is read by every thread
-  if (threadIdx.x == 0) {
-    sc.base = -1;
-    while (visited < nslots) {
-      const long total = min(cand_total(d, slot), (long)d.out_cap);
-      const long c = (long)atomicAdd(&d.counters[slot * CNT_STRIDE + CNT_EST], 1) * chunk;
-      if (c < total) {
-        sc.slot = slot;
-        sc.base = c;
-        sc.end = min(c + chunk, total);
-        break;
-      }
-      slot = slot + 1 == nslots ? 0 : slot + 1;
-      visited++;
-    }
-  }
-  __syncthreads();
-  out = sc;
-  return out.base >= 0;
-}
-
-__device__ __forceinline__ void publish_all(const V12Dev &d, int nslots) {
-  if (blockIdx.x == 0)
-    for (int sl = threadIdx.x; sl < nslots; sl += blockDim.x) publish_count(d, sl, cand_total(d, sl));
-}
-
 // Resident 128-thread blocks per SM the estimation kernels are compiled
 // for (registers per thread = 65536 / (128 * blocks), without spills).
 constexpr int est32_blocks(int LN) { return LN <= 18 ? 8 : LN <= 24 ? 6 : 5; }
@@ -1205,87 +1159,97 @@ __device__ __forceinline__ void est32_candidate(const V12Dev &d, int slot, long 
   ((float2 *)d.out_val)[o] = make_float2(mre, mim);
 }
 
-// FP32 form: values and medians in FP32.
+// FP32 form of the same plans: values and medians in FP32, one candidate per
+// thread.  Blocks belong to one signal each and step through its candidates;
+// a queue per signal that blocks moved between cost each of them an atomic
+// round trip per signal once the candidates were gone (four voted signals of
+// n = 2^22, k = 500: 18.6 -> 12 us).
 template <int LN, bool EXACT>
-__global__ void __launch_bounds__(128, est32_blocks(LN)) k_estimate32(V12Dev d, int nslots) {
-  publish_all(d, nslots);
-  const float2 *wl = (const float2 *)d.win_loc, *we = (const float2 *)d.win_est;
-  const int Lr = EXACT ? LN : d.L;
-  int slot = (int)(sm_id() % (unsigned)nslots), visited = 0;
-  EstChunk ck;
-  while (next_chunk(d, nslots, blockDim.x, slot, visited, ck)) {
-    const int *rp = d.rparams + (long)ck.slot * d.rp_stride;
-    const float2 *xs = (const float2 *)d.xs + (long)ck.slot * d.xs_size;
-    const long h = ck.base + threadIdx.x;  // one candidate per thread and chunk
-    if (h < ck.end) {
-      const unsigned f = cand_freq(d, ck.slot, h);
-      float re[LN], im[LN];
-#pragma unroll
-      for (int j = 0; j < LN; j++) {
-        if (EXACT || j < Lr) {
-          float sc;
-          value32(d, xs, wl, we, j, f, (unsigned)rp[d.L + j], re[j], im[j], sc);
-        } else {
-          re[j] = INFINITY;
-          im[j] = INFINITY;
-        }
-      }
-      const float mre = lower_median<LN, EXACT>(re, Lr), mim = lower_median<LN, EXACT>(im, Lr);
-      const long o = (long)ck.slot * d.out_stride + h;
-      d.out_idx[o] = (int)f;
-      ((float2 *)d.out_val)[o] = make_float2(mre, mim);
-    }
-  }
+__global__ void __launch_bounds__(128, est32_blocks(LN)) k_estimate32(V12Dev d) {
+  const int slot = blockIdx.y;
+  const long all = cand_total(d, slot), total = min(all, (long)d.out_cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) publish_count(d, slot, all);
+  for (long h = (long)blockIdx.x * 128 + threadIdx.x; h < total; h += (long)gridDim.x * 128)
+    est32_candidate<LN, EXACT>(d, slot, h);
 }
 
-// FP64 form, bit-exact: the median element is chosen on FP32 copies with a
-// rigorous error bound, then only that element is divided in FP64 (the
-// reference's exact operation sequence); anything not provable (ties,
-// near-ties) takes the all-exact path.
+// FP64 form, bit-exact, of v1, voted v2 and the v2 plans without the grouped
+// layout.  Few candidates (a v1 signal has about as many as tones): one warp
+// each, one loop per lane -- a candidate's L divisions then cost one lane's
+// chain instead of L of them, and no FP32 selection is needed.  Many: one
+// thread each; the median element is chosen on FP32 copies with a rigorous
+// error bound, then only that element is divided in FP64 (the reference's
+// exact operation sequence); what is not provable (ties, near-ties) is done
+// by the warp.  A warp's candidate holds an FP64 pipe for about 24
+// instructions of 64 to 76 cycles, 0.8 us; EST64_WARP of them per
+// sub-partition take as long as the other form's start-to-end latency (34 to
+// 60 us).  Kernel times, one thread per candidate taken from a queue per signal
+// -> now: one v1 signal of 2^13 points 60 -> 5.4 us, of 2^24 points 37 -> 8
+// us; 64 signals of 2^16 points 61 -> 14 us.
+constexpr int EST64_WARP = 24;
+
 template <int LN, bool EXACT>
-__global__ void __launch_bounds__(128, est64_blocks(LN)) k_estimate64(V12Dev d, int nslots) {
-  publish_all(d, nslots);
+__global__ void __launch_bounds__(128, est64_blocks(LN)) k_estimate64(V12Dev d, int warp_max) {
+  const int slot = blockIdx.y, lane = threadIdx.x & 31;
+  const long all = cand_total(d, slot), total = min(all, (long)d.out_cap);
+  if (blockIdx.x == 0 && threadIdx.x == 0) publish_count(d, slot, all);
+  const int *rp = d.rparams + (long)slot * d.rp_stride;
+  const double2 *xs = (const double2 *)d.xs + (long)slot * d.xs_size;
+  const long o = (long)slot * d.out_stride;
+  if (total <= warp_max) {
+    for (long h = (long)blockIdx.x * 4 + (threadIdx.x >> 5); h < total; h += (long)gridDim.x * 4) {
+      const unsigned f = cand_freq(d, slot, h);
+      const double2 v = warp_estimate64(d, xs, rp, f);
+      if (lane == 0) {
+        d.out_idx[o + h] = (int)f;
+        ((double2 *)d.out_val)[o + h] = v;
+      }
+    }
+    return;
+  }
   const float2 *wl = (const float2 *)d.win32_loc, *we = (const float2 *)d.win32_est;
+  const float2 *xs32 = (const float2 *)d.xs32 + (long)slot * d.xs_size;
   const int Lr = EXACT ? LN : d.L;
-  int slot = (int)(sm_id() % (unsigned)nslots), visited = 0;
-  EstChunk ck;
-  while (next_chunk(d, nslots, blockDim.x, slot, visited, ck)) {
-    const int *rp = d.rparams + (long)ck.slot * d.rp_stride;
-    const float2 *xs32 = (const float2 *)d.xs32 + (long)ck.slot * d.xs_size;
-    const double2 *xs = (const double2 *)d.xs + (long)ck.slot * d.xs_size;
-    const long h = ck.base + threadIdx.x;  // one candidate per thread and chunk
-    if (h < ck.end) {
-      const unsigned f = cand_freq(d, ck.slot, h);
-      float re[LN], im[LN], eb[LN];
+  for (long h0 = (long)blockIdx.x * 128; h0 < total; h0 += (long)gridDim.x * 128) {
+    const long h = h0 + threadIdx.x;
+    const bool live = h < total;
+    const unsigned f = live ? cand_freq(d, slot, h) : 0u;
+    float re[LN], im[LN], eb[LN];
 #pragma unroll
-      for (int j = 0; j < LN; j++) {
-        if (EXACT || j < Lr) {
-          float sc;
-          value32(d, xs32, wl, we, j, f, (unsigned)rp[d.L + j], re[j], im[j], sc);
-          // |exact - approx| <= 2^-22 * scale: each FP32 operand carries one
-          // rounding (2^-24 relative), plus two products and a sum; the
-          // bound below has a 4x margin, which also covers the rounding of
-          // the comparisons in proven_median.
-          eb[j] = sc * 0x1p-20f + 1e-30f;
-        } else {
-          re[j] = INFINITY;
-          im[j] = INFINITY;
-          eb[j] = 0.f;
-        }
-      }
-      const int ir = proven_median<LN, EXACT>(re, eb, Lr);
-      const int ii = proven_median<LN, EXACT>(im, eb, Lr);
-      double2 res;
-      if (ir >= 0 && ii >= 0) {
-        res.x = value64(d, xs, ir, f, (unsigned)rp[d.L + ir]).x;
-        res.y = value64(d, xs, ii, f, (unsigned)rp[d.L + ii]).y;
+    for (int j = 0; j < LN; j++) {
+      if (EXACT || j < Lr) {
+        float sc;
+        value32(d, xs32, wl, we, j, f, (unsigned)rp[d.L + j], re[j], im[j], sc);
+        // |exact - approx| <= 2^-22 * scale: each FP32 operand carries one
+        // rounding (2^-24 relative), plus two products and a sum; the
+        // bound below has a 4x margin, which also covers the rounding of
+        // the comparisons in proven_median.
+        eb[j] = sc * 0x1p-20f + 1e-30f;
       } else {
-        res = median64_exact(d, xs, rp, f);
-        atomicAdd(&d.counters[ck.slot * CNT_STRIDE + CNT_EXACT], 1);
+        re[j] = INFINITY;
+        im[j] = INFINITY;
+        eb[j] = 0.f;
       }
-      const long o = (long)ck.slot * d.out_stride + h;
-      d.out_idx[o] = (int)f;
-      ((double2 *)d.out_val)[o] = res;
+    }
+    const int ir = proven_median<LN, EXACT>(re, eb, Lr);
+    const int ii = proven_median<LN, EXACT>(im, eb, Lr);
+    double2 res = make_double2(0.0, 0.0);
+    const bool proven = ir >= 0 && ii >= 0;
+    if (live && proven) {
+      res.x = value64(d, xs, ir, f, (unsigned)rp[d.L + ir]).x;
+      res.y = value64(d, xs, ii, f, (unsigned)rp[d.L + ii]).y;
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, live && !proven); m; m &= m - 1u) {
+      const int src = __ffs(m) - 1;
+      const double2 v = warp_estimate64(d, xs, rp, __shfl_sync(0xffffffffu, f, src));
+      if (lane == src) {
+        res = v;
+        atomicAdd(&d.counters[slot * CNT_STRIDE + CNT_EXACT], 1);
+      }
+    }
+    if (live) {
+      d.out_idx[o + h] = (int)f;
+      ((double2 *)d.out_val)[o + h] = res;
     }
   }
 }
@@ -1525,35 +1489,12 @@ __device__ __forceinline__ double2 ec_exact64(const V12Dev &d, const EcVal &t, i
                       A::div(A::sub(A::mul(x.x, hw.y), A::mul(x.y, hw.x)), den));
 }
 
-__device__ __noinline__ double2 ec_median64_all(const V12Dev &d, const EcVal *tv, const int2 *sm, const double2 *xs,
-                                                int i, int G) {
-  double vre[EC_MAXL], vim[EC_MAXL];
-  const int L = d.L;
-  for (int j = 0; j < L; j++) {
-    const double2 v = ec_exact64(d, tv[j], sm[j], xs, i, G, j);
-    vre[j] = v.x;
-    vim[j] = v.y;
-  }
-  const int m = (L - 1) >> 1;
-  double mre = 0, mim = 0;
-  for (int a = 0; a < L; a++) {
-    const long long ka = okey(vre[a]), kb = okey(vim[a]);
-    int rr = 0, ri = 0;
-    for (int b = 0; b < L; b++) {
-      const long long x = okey(vre[b]), y = okey(vim[b]);
-      rr += (x < ka) || (b < a && x == ka);
-      ri += (y < kb) || (b < a && y == kb);
-    }
-    if (rr == m) mre = vre[a];
-    if (ri == m) mim = vim[a];
-  }
-  return make_double2(mre, mim);
-}
-
 // FP64 estimates of the staged candidates, bit-exact: the lower-median
 // element of each component is chosen on the staged FP32 copy and proven
 // with the bound of k_estimate64 (proven_median), then divided exactly in
-// FP64; anything not provable takes the all-exact path.
+// FP64; what is not provable is done by the warp, one loop per lane (by one
+// thread it took 20 us, which a single signal waited for: 31 -> 10 us at one
+// signal of 2^20 points, 310 -> 265 us at 8 of 2^22).
 template <int LN, bool EXACT, int NTH>
 __device__ __forceinline__ void ec64_block(const V12Dev &d, int slot, long h0, long total, float2 *seg,
                                            EcShared<NTH> &sh, int2 *srcmw) {
@@ -1598,13 +1539,19 @@ __device__ __forceinline__ void ec64_block(const V12Dev &d, int slot, long h0, l
     }
   }
   const int ii = proven_median<LN, EXACT>(v, eb, Lr);
-  double2 res;
-  if (ir >= 0 && ii >= 0) {
-    res.x = xre;
-    res.y = ec_exact64(d, tv[ii], sm[ii], xs, i, G, ii).y;
-  } else {
-    res = ec_median64_all(d, tv, sm, xs, i, G);
-    atomicAdd(&d.counters[slot * CNT_STRIDE + CNT_EXACT], 1);
+  double2 res = make_double2(xre, 0.0);
+  const bool proven = ir >= 0 && ii >= 0;
+  if (proven) res.y = ec_exact64(d, tv[ii], sm[ii], xs, i, G, ii).y;
+  // a warp's candidates belong to one group (G >= 32): u, tv and sm are its
+  for (unsigned m = __ballot_sync(0xffffffffu, !proven); m; m &= m - 1u) {
+    const int src = __ffs(m) - 1, lane = threadIdx.x & 31, is = __shfl_sync(0xffffffffu, i, src);
+    double2 v = make_double2(0.0, 0.0);
+    if (lane < L) v = ec_exact64(d, tv[lane], sm[lane], xs, is, G, lane);
+    v = warp_median64(v, L);
+    if (lane == src) {
+      res = v;
+      atomicAdd(&d.counters[slot * CNT_STRIDE + CNT_EXACT], 1);
+    }
   }
   const unsigned S = (unsigned)(d.n / d.W) >> lg;
   const long o = (long)slot * d.out_stride + h0 + threadIdx.x;
@@ -1746,17 +1693,26 @@ static cudaError_t launch_bucket(const V12Dev &d, int nslots, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-#define SFFT_EST_KERNEL(NAME, BLOCKS)                                           \
-  template <int LN, bool EX>                                                    \
-  struct NAME##_k {                                                             \
-    static cudaError_t go(int nslots, cudaStream_t s, const V12Dev &d, int nsm) { \
-      NAME<LN, EX><<<nsm * BLOCKS(LN), 128, 0, s>>>(d, nslots);                 \
-      return cudaSuccess;                                                       \
-    }                                                                           \
-  };
-SFFT_EST_KERNEL(k_estimate32, est32_blocks)
-SFFT_EST_KERNEL(k_estimate64, est64_blocks)
-#undef SFFT_EST_KERNEL
+template <int LN, bool EX>
+struct k_estimate32_k {
+  static cudaError_t go(int nslots, cudaStream_t s, const V12Dev &d, int nsm) {
+    const int most = std::max(1, nsm * est32_blocks(LN) / nslots);
+    const int blocks = (int)std::min<long>(most, ((long)d.out_cap + 127) / 128);
+    k_estimate32<LN, EX><<<dim3(std::max(1, blocks), nslots), 128, 0, s>>>(d);
+    return cudaSuccess;
+  }
+};
+template <int LN, bool EX>
+struct k_estimate64_k {
+  static cudaError_t go(int nslots, cudaStream_t s, const V12Dev &d, int nsm) {
+    // blocks of four warps: the resident ones shared out over the slots, at
+    // most one warp per candidate
+    const int most = std::max(1, nsm * est64_blocks(LN) / nslots);
+    const int blocks = (int)std::min<long>(most, ((long)d.out_cap + 3) / 4);
+    k_estimate64<LN, EX><<<dim3(std::max(1, blocks), nslots), 128, 0, s>>>(d, EST64_WARP * 4 * nsm / nslots);
+    return cudaSuccess;
+  }
+};
 
 template <template <int, bool> class KS>
 static cudaError_t dispatch_estimate(const V12Dev &d, int nslots, int nsm, cudaStream_t s) {
