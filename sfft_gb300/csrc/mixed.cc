@@ -194,6 +194,7 @@ sfft_mixed *sfft_mixed_create(int num, const int *n, const int *k, const int *ve
   good = good && ok(cudaMalloc((void **)&m->d_idx, sizeof(int) * std::max(1L, idx_total)), "arena") &&
          ok(cudaMalloc((void **)&m->d_val, std::max<size_t>(16, val_total)), "arena") &&
          ok(cudaMalloc((void **)&m->d_cnt, sizeof(int) * num), "arena") &&
+         ok(cudaMemset(m->d_cnt, 0, sizeof(int) * num), "arena") &&
          ok(cudaStreamCreateWithFlags(&m->master, cudaStreamNonBlocking), "stream") &&
          ok(cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming), "event");
   if (!good) {
