@@ -129,7 +129,7 @@ struct PlanImpl {
   // workspace
   int slots = 0;
   DBuf xs, xs32, xs_tmp, pw, comb_tmp, comb_pw, J, sel_bits, score, hits, comb_bits, comb_list, counters, out_idx, out_val;
-  DBuf man, man_tmp, g1, g2, perm, est_f, est_v, map_keys, map_vals, map_list;
+  DBuf man, man_tmp, g1, g2, trig, est_f, est_v, map_keys, map_vals, map_list;
   DBuf rparams, inputs, dense_ptrs, in_stage, dense_stage, trace, cnt_stash;
   std::vector<unsigned> epoch;
   int hit_cap = 0, out_cap = 0, est_cap = 0, map_cap = 0, table_cap = 0;
@@ -211,23 +211,37 @@ long xs_position(long b, long B, int lg) {
 
 // ------------------------------------------------------------- constants --
 
-// Twiddles of an N-point FFT.  staged: stage by stage, entry r Ns + k holding
-// w_{4 Ns}^{r k} (r = 1 .. 3, k < Ns) for the radix-4 stages Ns = 1, 4, ... or
-// 2, 8, ... -- the table's own values w_N^{r k N / (4 Ns)}, reordered.
-bool upload_twiddles(DBuf &b, long N, int prec, bool staged) {
+// Twiddles of an N-point FFT, stage by stage: entry r Ns + k holds w_{4
+// Ns}^{r k} (r = 1 .. 3, k < Ns) for the radix-4 stages Ns = 1, 4, ... or 2, 8,
+// ... -- the FFT table's own values w_N^{r k N / (4 Ns)}, reordered.
+bool upload_twiddles(DBuf &b, long N, int prec) {
   const std::vector<double> &tw = sfft::fft_twiddles(N);
-  std::vector<double> t(tw.begin(), tw.begin() + 2 * N);
-  if (staged) {
-    for (long Ns = ilog2(N) & 1 ? 2 : 1; Ns < N; Ns *= 4)
-      for (long r = 1; r < 4; r++)
-        for (long k = 0; k < Ns; k++) {
-          const long e = r * k * (N / (4 * Ns));
-          t[2 * (r * Ns + k)] = tw[2 * e];
-          t[2 * (r * Ns + k) + 1] = tw[2 * e + 1];
-        }
-  }
+  std::vector<double> t(2 * (size_t)N, 0.0);
+  for (long Ns = ilog2(N) & 1 ? 2 : 1; Ns < N; Ns *= 4)
+    for (long r = 1; r < 4; r++)
+      for (long k = 0; k < Ns; k++) {
+        const long e = r * k * (N / (4 * Ns));
+        t[2 * (r * Ns + k)] = tw[2 * e];
+        t[2 * (r * Ns + k) + 1] = tw[2 * e + 1];
+      }
   if (prec == sfft::PREC_FP64) return b.upload(t);
   return b.upload(to_f32(t));
+}
+
+// v3's phase table: (cos, sin)(2 pi i / 1024), each within half a unit in the
+// last place.
+bool upload_trig(DBuf &b) {
+  std::vector<double> t(2 * 1024);
+  for (int i = 0; i < 1024; i++) {
+    // the angle within an octant, so that no argument needs reduction
+    const int o = i >> 7, k = i & 127, j = o & 1 ? 128 - k : k;
+    const long double a = 3.14159265358979323846264338327950288L * j / 512;
+    const double c = (double)cosl(a), s = (double)sinl(a);
+    const double x = o == 0 || o == 7 || o == 3 || o == 4 ? c : s, y = o == 0 || o == 7 || o == 3 || o == 4 ? s : c;
+    t[2 * i] = o >= 2 && o < 6 ? -x : x;
+    t[2 * i + 1] = o >= 4 ? -y : y;
+  }
+  return b.upload(t);
 }
 
 // Plan-time FFTs of power-of-two length n >= 2^15 on the plan's device.
@@ -382,15 +396,12 @@ bool ensure_slots(PlanImpl &P, int want) {
   } else {
     const auto &p = P.p3;
     P.rp_stride = 5;
-    P.est_cap = std::max(p.W_Man, std::max(p.B_g1, p.B_g2));
+    P.est_cap = std::max(p.W_Man, std::max(p.B_g1, p.B_g2)) + 16 * 1024;  // the peel kernel's CTAs share it out
     P.map_cap = 4 * (p.W_Man + p.B_g1 + p.B_g2) + 8 * P.k;
     P.table_cap = 1;
     while (P.table_cap < 2 * P.map_cap) P.table_cap <<= 1;
     P.out_cap = P.map_cap;
-    if (!P.perm.ensure(16 * 2 * (size_t)(p.w_g2 + 2) * S)) return false;
-    if ((p.W_Man > sfft::v3_max_smem_fft() || sfft::v3_man_split(p.W_Man)) &&
-        !P.man_tmp.ensure(64 * (size_t)p.W_Man * S))
-      return false;
+    if (!P.man_tmp.ensure(32 * (size_t)p.W_Man * S)) return false;
     if (!P.man.ensure(32 * (size_t)p.W_Man * S) || !P.g1.ensure(32 * (size_t)p.B_g1 * S) ||
         !P.g2.ensure(32 * (size_t)p.B_g2 * S) || !P.est_f.ensure(sizeof(int) * P.est_cap * S) ||
         !P.est_v.ensure(16 * (size_t)P.est_cap * S) || !P.map_keys.ensure(sizeof(int) * P.table_cap * S) ||
@@ -561,10 +572,18 @@ sfft::V3Dev v3_view(PlanImpl &P) {
   d.tw_g2 = P.tw_b.p;
   d.man = P.man.p;
   d.man_tmp = P.man_tmp.p;
-  d.large_man = p.W_Man > sfft::v3_max_smem_fft();
+  d.trig = P.trig.p;
+  // the reference's constants, formed by its operations on the host
+  const double PI2 = 2 * 3.14159265358979323846;
+  d.inv_n = 1. / P.n;
+  d.n_over_pi2 = P.n / PI2;
+  d.pi2_over_n = PI2 / P.n;
+  d.w_dbl = p.W_Man;
+  d.inv_w2 = (1. / p.W_Man) * (1. / p.W_Man);
+  d.tol_man = P.n * 1e-10;
+  d.tol_gauss = P.n * 1e-12;  // (c1 / c0 - 1)^2 / n < 1e-12
   d.g1 = P.g1.p;
   d.g2 = P.g2.p;
-  d.perm = P.perm.p;
   d.est_f = P.est_f.as<int>();
   d.est_v = P.est_v.p;
   d.map_keys = P.map_keys.as<int>();
@@ -631,10 +650,9 @@ void shift_view(PlanImpl &P, sfft::V12Dev &d, int base, bool own_out) {
 void shift_view(PlanImpl &P, sfft::V3Dev &d, int base, bool own_out) {
   if (!base) return;
   shift(d.man, 32 * (size_t)d.W, base);
-  if (d.large_man || sfft::v3_man_split(d.W)) shift(d.man_tmp, 64 * (size_t)d.W, base);
+  shift(d.man_tmp, 32 * (size_t)d.W, base);
   shift(d.g1, 32 * (size_t)d.B1, base);
   shift(d.g2, 32 * (size_t)d.B2, base);
-  shift(d.perm, 16 * 2 * (size_t)(d.w2 + 2), base);
   shift(d.est_f, sizeof(int) * (size_t)d.est_cap, base);
   shift(d.est_v, 16 * (size_t)d.est_cap, base);
   shift(d.map_keys, sizeof(int) * (size_t)d.table_cap, base);
@@ -1209,8 +1227,8 @@ static sfft_plan *make_plan_impl(int n, int k, enum sfft_version version, const 
         (P->prec == sfft::PREC_FP64 &&
          (!upload_v12_window(P->win32_a, fa.freq, n, n / p.B_loc, sfft::PREC_FP32) ||
           !upload_v12_window(P->win32_b, fb.freq, n, n / p.B_est, sfft::PREC_FP32))) ||
-        !upload_twiddles(P->tw_a, p.B_loc, P->prec, true) || !upload_twiddles(P->tw_b, p.B_est, P->prec, true) ||
-        !upload_twiddles(P->tw_c, std::max(p.W_Comb, 2), P->prec, true))
+        !upload_twiddles(P->tw_a, p.B_loc, P->prec) || !upload_twiddles(P->tw_b, p.B_est, P->prec) ||
+        !upload_twiddles(P->tw_c, std::max(p.W_Comb, 2), P->prec))
       return nullptr;
   } else {
     if (sfft::build_v3_plan((unsigned)n, (unsigned)k, P->p3, fa, fb, err, &bo)) {
@@ -1229,9 +1247,8 @@ static sfft_plan *make_plan_impl(int n, int k, enum sfft_version version, const 
     if (!P->taps_a.upload(fa.time) || !P->taps_b.upload(fb.time) ||
         !upload_v3_window(P->win_a, fa.freq, n, P->win_half_a) ||
         !upload_v3_window(P->win_b, fb.freq, n, P->win_half_b) ||
-        !upload_twiddles(P->tw_a, p.B_g1, sfft::PREC_FP64, false) ||
-        !upload_twiddles(P->tw_b, p.B_g2, sfft::PREC_FP64, false) ||
-        !upload_twiddles(P->tw_c, p.W_Man, sfft::PREC_FP64, false))
+        !upload_twiddles(P->tw_a, p.B_g1, sfft::PREC_FP64) || !upload_twiddles(P->tw_b, p.B_g2, sfft::PREC_FP64) ||
+        !upload_twiddles(P->tw_c, p.W_Man, sfft::PREC_FP64) || !upload_trig(P->trig))
       return nullptr;
   }
   if (!cuda_ok(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking), "stream")) return nullptr;
@@ -1297,7 +1314,7 @@ long sfft_plan_footprint(const sfft_plan *plan) {
   const DBuf *bufs[] = {&P->taps_a, &P->taps_b, &P->win_a, &P->win_b, &P->win32_a, &P->win32_b, &P->tw_a,
                         &P->tw_b, &P->tw_c, &P->xs, &P->xs32, &P->xs_tmp, &P->pw, &P->comb_tmp, &P->comb_pw, &P->J, &P->sel_bits,
                         &P->score, &P->hits, &P->comb_bits, &P->comb_list, &P->counters, &P->out_idx,
-                        &P->out_val, &P->man, &P->man_tmp, &P->g1, &P->g2, &P->perm, &P->est_f, &P->est_v, &P->map_keys,
+                        &P->out_val, &P->man, &P->man_tmp, &P->g1, &P->g2, &P->trig, &P->est_f, &P->est_v, &P->map_keys,
                         &P->map_vals, &P->map_list, &P->rparams, &P->inputs, &P->dense_ptrs, &P->in_stage,
                         &P->dense_stage, &P->trace, &P->cnt_stash};
   long total = 0;

@@ -7,7 +7,7 @@
 // FP32 instantiations use ordinary float arithmetic (FMA allowed).
 //
 // FFT.  block_fft() is the radix-4/2 Stockham FFT defined for this project
-// (twiddle table tw[t] = (cos, -sin)(2 pi t / N) by quarter-wave symmetry,
+// (twiddle values (cos, -sin)(2 pi t / N) by quarter-wave symmetry,
 // radix-2 stage first when log2 N is odd, twiddle applied only when its
 // exponent is non-zero, out[(j - j%Ns)*R + j%Ns + r*Ns]).  It runs in place
 // in shared memory: each stage loads all of its butterfly inputs to
@@ -126,11 +126,10 @@ __device__ __forceinline__ int2 block_exscan2(int a, int b, int &pa, int &pb, in
 // --------------------------------------------------------- shared-mem FFT --
 
 // Forward FFT of buf[0..N) in shared memory, N = 2^logN <= PER*4*blockDim.
-// tw: the N-entry twiddle table of that length (global memory), in natural
-// order, or (STAGED) stage by stage: entry r Ns + k is w_{4 Ns}^{r k}, r = 1
-// .. 3, k < Ns, of the radix-4 stage Ns -- the same values, with those that
-// neighbouring threads use side by side.
-template <typename R, int PER, bool STAGED = false>
+// tw: the N-entry twiddle table of that length (global memory), stage by
+// stage: entry r Ns + k is w_{4 Ns}^{r k}, r = 1 .. 3, k < Ns, of the radix-4
+// stage Ns, so that neighbouring threads read neighbouring entries.
+template <typename R, int PER>
 __device__ void block_fft(c2_t<R> *buf, int N, int logN, const c2_t<R> *__restrict__ tw) {
   using V = c2_t<R>;
   const int T = blockDim.x;
@@ -154,7 +153,6 @@ __device__ void block_fft(c2_t<R> *buf, int N, int logN, const c2_t<R> *__restri
   }
   const int q4 = N >> 2;
   while (Ns < N) {
-    const int stride = N / (Ns * 4);
     V v[PER][4];
 #pragma unroll
     for (int s = 0; s < PER; s++) {
@@ -165,8 +163,7 @@ __device__ void block_fft(c2_t<R> *buf, int N, int logN, const c2_t<R> *__restri
         for (int r = 0; r < 4; r++) v[s][r] = buf[j + r * q4];
 #pragma unroll
         for (int r = 1; r < 4; r++) {
-          const int e = STAGED ? r * Ns + k : r * k * stride;
-          if (k) v[s][r] = cmul<R>(v[s][r], tw[e]);
+          if (k) v[s][r] = cmul<R>(v[s][r], tw[r * Ns + k]);
         }
         V t0 = cadd<R>(v[s][0], v[s][2]), t1 = csub<R>(v[s][0], v[s][2]);
         V t2 = cadd<R>(v[s][1], v[s][3]), t3 = csub<R>(v[s][1], v[s][3]);
@@ -193,128 +190,6 @@ __device__ void block_fft(c2_t<R> *buf, int N, int logN, const c2_t<R> *__restri
     __syncthreads();
     Ns *= 4;
   }
-}
-
-// ---------------------------------------------------- top-num selection --
-
-// Indices of the `num` largest of p[0..N) with the tie rule of the
-// reference's find_largest_indices (src/utils.cc:130-158): the cutoff is the
-// (N-num-1)-th smallest value, every index above it is taken, then indices
-// equal to it in increasing order until num; the output is ascending.
-// keys: order-preserving keys of p in shared memory.  hist: 256 + 2 ints of
-// shared memory; scan: 64 ints.  Writes out[0..num).  Block-wide.
-template <typename K, typename KeyAt>
-__device__ void block_top_indices_f(KeyAt keyat, int N, int num, int *__restrict__ out, int *hist,
-                                    int *scan) {
-  constexpr int BITS = sizeof(K) * 8;
-  const int rank = N - num - 1;  // ascending rank of the cutoff
-  K prefix = 0, mask = 0;
-  int remaining = rank;
-  for (int shift = BITS - 8; shift >= 0; shift -= 8) {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-    // warp-aggregated: lanes with the same digit add once (keys of similar
-    // magnitude share their top digits, which would serialise the atomics)
-    for (int i0 = 0; i0 < N; i0 += blockDim.x) {
-      const int i = i0 + threadIdx.x;
-      int bin = -1;
-      if (i < N) {
-        const K k = keyat(i);
-        if ((k & mask) == prefix) bin = (int)((k >> shift) & 0xFF);
-      }
-      const unsigned peers = __match_any_sync(0xffffffffu, bin);
-      if (bin >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&hist[bin], __popc(peers));
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      // find digit d: cum(d) <= remaining < cum(d) + hist[d]
-      const int lane = threadIdx.x;
-      int c[8], tot = 0;
-#pragma unroll
-      for (int q = 0; q < 8; q++) { c[q] = hist[lane * 8 + q]; tot += c[q]; }
-      int inc = tot;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
-      }
-      int before = inc - tot;
-      if (remaining >= before && remaining < inc) {
-        int acc = before;
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-          if (remaining >= acc && remaining < acc + c[q]) {
-            hist[256] = lane * 8 + q;
-            hist[257] = remaining - acc;
-            hist[258] = c[q];
-          }
-          acc += c[q];
-        }
-      }
-    }
-    __syncthreads();
-    const int d = hist[256];
-    remaining = hist[257];
-    const int in_bin = hist[258];
-    prefix |= ((K)d) << shift;
-    mask |= ((K)0xFF) << shift;
-    __syncthreads();
-    if (in_bin == 1 && shift > 0) {
-      // the cutoff's bin holds a single key: that key is the cutoff, so its
-      // remaining digits need no further histogram passes
-      for (int i0 = 0; i0 < N; i0 += blockDim.x) {
-        const int i = i0 + threadIdx.x;
-        if (i < N) {
-          const K k = keyat(i);
-          if ((k & mask) == prefix) {
-            hist[260] = (int)(unsigned)(k & 0xffffffffu);
-            if constexpr (sizeof(K) == 8) hist[261] = (int)(unsigned)(k >> 32);
-          }
-        }
-      }
-      __syncthreads();
-      K kk = (K)(unsigned)hist[260];
-      if constexpr (sizeof(K) == 8) kk |= ((K)(unsigned)hist[261]) << 32;
-      prefix = kk;
-      __syncthreads();
-      break;
-    }
-  }
-  const K cutoff = prefix;
-  // contiguous chunk per thread, in index order
-  const int C = (N + blockDim.x - 1) / blockDim.x;
-  const int lo = min(N, (int)threadIdx.x * C), hi = min(N, lo + C);
-  int ngt = 0, neq = 0;
-  for (int i = lo; i < hi; i++) {
-    K k = keyat(i);
-    ngt += (k > cutoff);
-    neq += (k == cutoff);
-  }
-  int pgt, peq;
-  int2 tot = block_exscan2(ngt, neq, pgt, peq, scan);
-  const int need = num - tot.x;  // equal-to-cutoff entries to take
-  int pos = pgt + min(peq, max(need, 0));
-  int eqr = peq;
-  for (int i = lo; i < hi; i++) {
-    K k = keyat(i);
-    if (k > cutoff) {
-      if (pos < num) out[pos] = i;
-      pos++;
-    } else if (k == cutoff) {
-      if (eqr < need) {
-        if (pos < num) out[pos] = i;
-        pos++;
-      }
-      eqr++;
-    }
-  }
-  __syncthreads();
-}
-
-template <typename K>
-__device__ void block_top_indices(const K *keys, int N, int num, int *__restrict__ out, int *hist,
-                                  int *scan) {
-  block_top_indices_f<K>([keys](int i) { return keys[i]; }, N, num, out, hist, scan);
 }
 
 // One radix-R stage (R = 2 with Ns = 1, or R = 4) of block_fft's Stockham

@@ -146,14 +146,14 @@ struct V3Dev {
   int win1_half, win2_half;
   const void *taps1, *taps2;    // double2
   const void *win1, *win2;      // double2, 2*half+1 entries centred on freq index 0
-  const void *tw_man, *tw_g1, *tw_g2;
+  const void *tw_man, *tw_g1, *tw_g2;  // stage by stage (block_fft)
+  const void *trig;             // double2 (cos, sin)(2 pi i / 1024)
+  double inv_n, n_over_pi2, pi2_over_n, w_dbl, inv_w2, tol_man, tol_gauss;  // 1/n, n/(2 pi), 2 pi/n, W, 1/W^2, test bounds
   // per-slot workspace
   void *man;     // 2W complex (interleaved loops)
-  void *man_tmp; // large_man: 4W complex (two W-point arrays and their FFT scratch)
-  int large_man; // W above the shared-memory FFT: Mansour comb FFTs in global memory
+  void *man_tmp; // 2W complex: the comb FFTs between their two launches
   void *g1;      // 2*B1 complex
   void *g2;      // 2*B2 complex
-  void *perm;    // (w2 + 1) complex
   int *est_f;    // cap per slot
   void *est_v;   // cap complex per slot
   int *map_keys; // map_cap per slot
@@ -176,12 +176,8 @@ struct V3Dev {
 };
 
 cudaError_t v3_run(const V3Dev &d, int nslots, cudaStream_t stream, StageEvents *se = nullptr);
-// Largest FP64 FFT the v3 filter kernel runs in shared memory.
+// Largest Gaussian bucket FFT of the v3 filter kernels (one CTA).
 int v3_max_smem_fft();
-// Whether a v3 plan's Mansour comb FFT of W points runs as eight W/8-point
-// FFTs over eight CTAs and a radix-8 combination (W from 4096 up to the
-// shared-memory limit) instead of in one CTA of the filter kernel.
-inline bool v3_man_split(int W) { return W >= 4096 && W <= v3_max_smem_fft(); }
 // Batched complex128 FFTs of length N in global memory (the same stages as
 // the shared-memory FFT): narr arrays per slot, arr_stride apart, slots
 // slot_stride apart; b is scratch of the same shape; result in a.

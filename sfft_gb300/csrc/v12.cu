@@ -181,7 +181,7 @@ struct OneCta<float> {
     } else {
       for (int i = threadIdx.x; i < N; i += blockDim.x) buf[i] = ld(i);
       __syncthreads();
-      block_fft<float, 1, true>(buf, N, dlog2(N), tw);
+      block_fft<float, 1>(buf, N, dlog2(N), tw);
     }
   }
   __device__ __forceinline__ float2 at(int i) const { return buf[fft16_at(i)]; }
@@ -200,7 +200,7 @@ struct OneCta<double> {
   __device__ __forceinline__ void fft(int N, const double2 *tw, Ld ld) {
     for (int i = threadIdx.x; i < N; i += blockDim.x) buf[i] = ld(i);
     __syncthreads();
-    block_fft<double, PER, true>(buf, N, dlog2(N), tw);
+    block_fft<double, PER>(buf, N, dlog2(N), tw);
     for (int i = threadIdx.x; i < N; i += blockDim.x) keys[i] = pkey(cabs2<double>(buf[i]));
     __syncthreads();
   }

@@ -1,25 +1,28 @@
 // v3.cu — the sFFT v3 ("exactly sparse") exec path on GB300.
 //
-//   k_v3_filters  six CTAs per signal: the two Mansour comb samplings
-//                 (computefourier-3.0.cc:96-127), the two shifts of the
-//                 contiguous Gaussian fold (:130-212) and of the permuted
-//                 Gaussian fold (:215-297), each followed by its
-//                 shared-memory FFT.  The permuted samples of the second
-//                 fold take the phases of the reference's running product
-//                 (:66-87), formed from tables of its factor's powers, one
-//                 sample per thread.
-//   k_v3_peel     one thread-block cluster (8 CTAs) per signal runs
-//                 alternate_fft's estimate / peel rounds (:784-1088):
-//                 bucket estimation spread over the cluster, subtraction of
-//                 recovered tones with FP64 atomics, and the bucket-count
-//                 fixpoint test, with a bounded number of rounds.
+//   k_v3_first   the first half of the Mansour comb FFTs on the gathered
+//                samples (computefourier-3.0.cc:96-127), and the folds of the
+//                contiguous (:130-212) and the permuted (:215-297) Gaussian
+//                filter, each for both time shifts.
+//   k_v3_second  the second half of the Mansour FFTs and the Gaussian bucket
+//                FFTs.
+//   k_v3_peel    one thread-block cluster (8 or 16 CTAs) per signal runs
+//                alternate_fft's estimate / peel rounds (:784-1088):
+//                bucket estimation spread over the cluster, subtraction of
+//                recovered tones with FP64 atomics, and the bucket-count
+//                fixpoint test, with a bounded number of rounds.
 // The result map is a per-signal open-addressing table in global memory.
 // FP64 throughout: the phase-slope frequency decode needs phase accuracy
-// below pi/n.
+// below pi/n.  On GB300 a warp's FP64 instruction holds its sub-partition's
+// FP64 pipe for 64 to 76 cycles, with one lane active or 32, so these kernels
+// take about as long as their longest chain of FP64 instructions: folds and
+// FFTs are spread over many CTAs, and the phases go through integer
+// arithmetic and a table (phase functions below).
 #include <cooperative_groups.h>
 
 #include "common.cuh"
 #include "engine.h"
+#include "fft.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -33,212 +36,277 @@ __device__ __forceinline__ double2 ld_x(const void *base, int in_type, long i) {
   return make_double2((double)v.x, (double)v.y);
 }
 
+// ----------------------------------------------------------------- phases --
+//
+// cos and sin of an angle held as a fraction of a turn in 64-bit fixed point,
+// and the fraction of a double angle of any size (M. Payne and R. Hanek,
+// "Radian reduction for trigonometric functions", SIGNUM Newsletter 18,
+// 1983): the angle's mantissa times a 128-bit window of 1 / (2 pi), in integer
+// arithmetic, of which the fraction's top 64 bits are kept.  The fraction's
+// nearest 1024th of a turn comes from a table, the rest (under 0.0031 rad)
+// from the Taylor terms that reach 1e-17.  13 FP64 instructions against more
+// than 40 in sincos (and its slow path beyond 1e5 rad, which the comb's phase
+// arguments of up to 2 pi n take); the arguments' own rounding, which the
+// reference's results contain, is untouched.  Largest error against 113-bit
+// arithmetic over 10^6 arguments of 1e-3 to 1e15 rad: 1.13e-16 (a correctly
+// rounded value: 0.56e-16; CUDA states 2 units in the last place, 2.2e-16).
+
+constexpr int TRIG_BITS = 10;  // V3Dev::trig: (cos, sin)(2 pi i / 1024)
+
+__device__ __forceinline__ double2 cis_turn(const double2 *trig, unsigned long long fr) {
+  const unsigned long long up = fr + (1ull << (63 - TRIG_BITS));
+  const double2 t = trig[(int)(up >> (64 - TRIG_BITS))];
+  // the rest, in (-2^53, 2^53] units of 2^-64 turn; as a double through the mantissa of 1.5 2^52
+  const long long rest = (long long)(fr - (up & ~((1ull << (64 - TRIG_BITS)) - 1)));
+  const double x =
+      __dadd_rn(__longlong_as_double(0x4338000000000000ll + (rest >> 2)), -6755399441055744.0) * 1.3624486320346218e-18;
+  const double s = x * x;
+  const double sn = fma(x * s, fma(s, 1.0 / 120, -1.0 / 6), x);  // sin x
+  const double cm = s * fma(s, 1.0 / 24, -0.5);                  // cos x - 1
+  return make_double2(t.x + fma(t.x, cm, -(t.y * sn)), t.y + fma(t.y, cm, t.x * sn));
+}
+
+// The fraction of a turn of `a` radians (|a| < 2^110).
+__device__ __forceinline__ unsigned long long turn_of(double a) {
+  constexpr unsigned long long R0 = 0x28be60db9391054aull, R1 = 0x7f09d5f47d4d3770ull, R2 = 0x36d8a5664f10e410ull;  // 1 / (2 pi)
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+  const int ex = (int)((b >> 52) & 0x7ff);
+  const unsigned long long M = (b & 0xfffffffffffffull) | (1ull << 52);
+  const int e = ex - 1075;  // |a| = M 2^e
+  unsigned long long hi, lo;
+  if (e > 0) {
+    hi = e < 64 ? (R0 << e) | (R1 >> (64 - e)) : R1 << (e - 64);
+    lo = e < 64 ? (R1 << e) | (R2 >> (64 - e)) : R2 << (e - 64);
+  } else if (e > -64) {
+    hi = R0 >> -e;
+    lo = e ? (R1 >> -e) | (R0 << (64 + e)) : R1;
+  } else {
+    hi = 0;
+    lo = e > -128 ? R0 >> (-e - 64) : 0;
+  }
+  const unsigned long long fr = __umul64hi(M, lo) + M * hi;
+  return (long long)b < 0 ? 0ull - fr : fr;
+}
+
+__device__ __forceinline__ double2 cis(const double2 *trig, double a) { return cis_turn(trig, turn_of(a)); }
+
+// e^{i (a + k b)}, the angle not rounded to a double in between.
+__device__ __forceinline__ double2 cis_step(const double2 *trig, double a, int k, double b) {
+  const double kd = (double)k, hi = kd * b, lo = fma(kd, b, -hi);
+  const unsigned long long fr = turn_of(a) + turn_of(hi) + (unsigned long long)__double2ll_rn(lo * 2935890503282001226.0);
+  return cis_turn(trig, fr);
+}
+
+// atan2(y, x).  An FP32 arctangent names the nearest 1024th of a turn, the
+// vector is turned back by it (table), and the remaining angle, under 0.0035
+// rad, is the series of its tangent; the quotient's FP32 reciprocal is
+// corrected to FP64.  About 20 FP64 instructions; largest error over 10^6
+// vectors 3.3e-16 rad (half a unit in the last place of pi is 2.2e-16).
+// Magnitudes outside 2^+-60 take the library function.
+__device__ __forceinline__ double angle_of(const double2 *trig, double y, double x) {
+  const int ey = (__double2hiint(y) >> 20) & 0x7ff, exx = (__double2hiint(x) >> 20) & 0x7ff, m = max(ey, exx);
+  if (m < 1023 - 60 || m > 1023 + 60) return atan2(y, x);
+  const float af = atan2f((float)y, (float)x);
+  const int k = __float2int_rn(af * 162.97466172610083f);  // 1024 / (2 pi)
+  const double2 t = trig[k & 1023];
+  const double u = fma(x, t.x, y * t.y), v = fma(y, t.x, -(x * t.y));
+  const double r = (double)(1.0f / (float)u);
+  const double q0 = v * r, q = fma(fma(-q0, u, v), r, q0);
+  const double s = q * q, d = fma(q * s, fma(s, 0.2, -1.0 / 3), q);
+  const double kd = (double)k;
+  return fma(kd, 0.006135923151542565, fma(kd, 2.391888279584674e-19, d));
+}
+
+// sqrt(a) and 1 / a for positive a of 2^+-60, from FP32 seeds by Newton steps
+// with exact FMA remainders (8 and 6 FP64 instructions); the library's beyond.
+__device__ __forceinline__ bool seedable(double a) {
+  const int e = __double2hiint(a) >> 20;
+  return e > 1023 - 60 && e < 1023 + 60;
+}
+__device__ __forceinline__ double sqrt_of(double a) {
+  if (!seedable(a)) return sqrt(a);
+  const double y = (double)rsqrtf((float)a);
+  double g = a * y, h = 0.5 * y;
+  const double e = fma(-g, h, 0.5);
+  g = fma(g, e, g);
+  h = fma(h, e, h);
+  return fma(fma(-g, g, a), h, g);
+}
+__device__ __forceinline__ double recip_of(double a) {
+  if (!seedable(a)) return 1. / a;
+  const double y = (double)(1.0f / (float)a), r = fma(fma(-a, y, 1.0), y, y);
+  return fma(fma(-a, r, 1.0), r, r);
+}
+
+// True if a component's magnitude is at least 2^e: a bucket none of whose
+// components is, is known to be empty without any FP64 instruction.
+__device__ __forceinline__ bool reaches(double2 v, int e) {
+  const int a = __double2hiint(v.x) & 0x7fffffff, b = __double2hiint(v.y) & 0x7fffffff;
+  return max(a, b) >= ((1023 + e) << 20);
+}
+
+__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {  // a b + c
+  return make_double2(fma(a.x, b.x, fma(-a.y, b.y, c.x)), fma(a.x, b.y, fma(a.y, b.x, c.y)));
+}
+
 // --------------------------------------------------------------- filters --
-
-// Split of the permuted Gaussian fold's phase products into tables:
-// LO = the power of two at or above sqrt(count) entries of step^lo and
-// ceil(count / LO) of shift_0 step^(LO hi), 16 bytes each, in the filter
-// kernel's shared memory.
-__host__ __device__ __forceinline__ int v3_phase_lo(int count) {
-  int lo = 1;
-  while ((long)lo * lo < count) lo *= 2;
-  return lo;
-}
-
-// a^e, e >= 0, by binary powering in FP64: about 2 log2(e) rounded complex
-// products, a relative error of a few 1e-15.
-__device__ __forceinline__ double2 cpow64(double2 a, int e) {
-  double2 r = make_double2(1.0, 0.0);
-  while (e) {
-    if (e & 1) r = cmul<double>(r, a);
-    e >>= 1;
-    if (e) a = cmul<double>(a, a);
-  }
-  return r;
-}
-
-
-template <int PER>
-__global__ void __launch_bounds__(1024) k_v3_filters(V3Dev d, int role0) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2 *buf = (double2 *)smem_raw;
-  const int role = blockIdx.x + role0, slot = blockIdx.y, l = role & 1;
-  const int *rp = d.rparams + (long)slot * d.rp_stride;
-  const unsigned long long mask = (unsigned long long)d.n - 1;
-  const void *x = d.inputs[slot];
-  int N;
-  const double2 *tw;
-  double2 *dst;
-  if (role < 2) {  // Mansour: x[(init_offset + l + i * n/W) mod n]
-    N = d.W;
-    tw = (const double2 *)d.tw_man;
-    dst = (double2 *)d.man + (long)slot * 2 * d.W;
-    const long sigma = d.n / d.W;
-    const long o = rp[3] + l;
-    for (int i = threadIdx.x; i < N; i += blockDim.x)
-      buf[i] = ld_x(x, d.in_type, (long)((unsigned long long)(o + i * sigma) & mask));
-  } else if (role < 4) {  // Gaussian 1: taps over x[init_G_offset + l + t]
-    N = d.B1;
-    tw = (const double2 *)d.tw_g1;
-    dst = (double2 *)d.g1 + (long)slot * 2 * d.B1;
-    const int chunks = d.w1 / d.B1;
-    const long base = (long)rp[4] + l;
-    const double2 *taps = (const double2 *)d.taps1;
-    for (int b = threadIdx.x; b < N; b += blockDim.x) {
-      double2 acc = make_double2(0.0, 0.0);
-      for (int c = 0; c < chunks; c++) {
-        const int t = c * N + b;
-        const double2 xv = ld_x(x, d.in_type, (long)((unsigned long long)(base + t) & mask));
-        acc = cadd<double>(acc, cmul<double>(xv, __ldg(taps + t)));
-      }
-      buf[b] = acc;
-    }
-  } else {  // Gaussian 2 on the permuted, phase-shifted samples
-    N = d.B2;
-    tw = (const double2 *)d.tw_g2;
-    dst = (double2 *)d.g2 + (long)slot * 2 * d.B2;
-    const int chunks = d.w2 / d.B2;
-    const int ig = rp[4], ai = rp[1], bb = rp[2];
-    const double2 *taps = (const double2 *)d.taps2;
-    // permute_fourier (computefourier-3.0.cc:66-87): sample i is
-    // x[(ig + i*ai) mod n] * shift_i with shift_0 = e^{2 pi i ig b / n} and
-    // shift_{i+1} = shift_i * e^{2 pi i ai b / n}, a running product.  Its
-    // two factors are formed here as there (the same FP64 angles, cos and
-    // sin), but the product is not replayed serially: on GB300's FP64 pipe a
-    // one-thread chain of rounded complex multiplications costs about 64
-    // cycles per operation (2945 steps at n = 2^24, k = 1000: 0.58 ms).
-    // Every thread instead forms shift_i = (shift_0 step^(LO hi)) step^lo
-    // from two tables built by binary powering, one sample per thread.  Its
-    // relative error, a few 1e-15, is below the serial chain's own
-    // accumulated rounding (about i * 2^-53) and far inside the 1e-10 value
-    // tolerance against the reference.
-    double2 *P = (double2 *)d.perm + (long)slot * (d.w2 + 2) * 2 + (long)l * (d.w2 + 2);
-    const int count = chunks * N + 1;
-    const int LO = v3_phase_lo(count), HI = (count + LO - 1) / LO;
-    double2 *tab = (double2 *)smem_raw;  // [LO] step^lo, then [HI] shift_0 step^(LO hi)
-    {
-      const double a0 = 2 * kPi * ig * bb / d.n, a1 = 2 * kPi * ai * bb / d.n;
-      const double2 sh0 = make_double2(cos(a0), sin(a0)), st = make_double2(cos(a1), sin(a1));
-      for (int e = threadIdx.x; e < LO + HI; e += blockDim.x)
-        tab[e] = e < LO ? cpow64(st, e) : cmul<double>(sh0, cpow64(cpow64(st, LO), e - LO));
-    }
-    __syncthreads();
-    for (int i = l + threadIdx.x; i < count; i += blockDim.x) {
-      const double2 shift = cmul<double>(tab[LO + i / LO], tab[i % LO]);
-      const long index = (long)(((unsigned long long)ig + (unsigned long long)i * (unsigned)ai) % (unsigned)d.n);
-      P[i - l] = cmul<double>(ld_x(x, d.in_type, index), shift);
-    }
-    __syncthreads();
-    for (int b = threadIdx.x; b < N; b += blockDim.x) {
-      double2 acc = make_double2(0.0, 0.0);
-      for (int c = 0; c < chunks; c++) {
-        const int t = c * N + b;
-        acc = cadd<double>(acc, cmul<double>(P[t], __ldg(taps + t)));
-      }
-      buf[b] = acc;
-    }
-  }
-  __syncthreads();
-  block_fft<double, PER>(buf, N, 31 - __clz(N), tw);
-  for (int i = threadIdx.x; i < N; i += blockDim.x) dst[2 * i + l] = buf[i];
-}
-
-// Mansour comb of width W above the shared-memory FFT: the two samplings go
-// to contiguous arrays (man_tmp[slot][l][i]), are transformed by the
-// global-memory FFT, and are interleaved into man[slot][2 i + l].
-__global__ void k_v3_man_gather(V3Dev d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y, slot = blockIdx.z;
-  if (i >= d.W) return;
-  const int *rp = d.rparams + (long)slot * d.rp_stride;
-  const unsigned long long mask = (unsigned long long)d.n - 1;
-  const long sigma = d.n / d.W, o = rp[3] + l;
-  double2 *a = (double2 *)d.man_tmp + (long)slot * 4 * d.W + (long)l * d.W;
-  a[i] = ld_x(d.inputs[slot], d.in_type, (long)((unsigned long long)(o + i * sigma) & mask));
-}
-
-__global__ void k_v3_man_interleave(V3Dev d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y, slot = blockIdx.z;
-  if (i >= d.W) return;
-  const double2 *a = (const double2 *)d.man_tmp + (long)slot * 4 * d.W + (long)l * d.W;
-  ((double2 *)d.man + (long)slot * 2 * d.W)[2 * i + l] = a[i];
-}
 
 int v3_max_smem_fft() { return 8192; }
 
-// Mansour comb FFT of W points (4096 <= W <= 8192) as eight W/8-point FFTs:
-// the one-CTA FP64 FFT of 8192 points in the filter kernel takes about 280 k
-// cycles on GB300's narrow FP64 pipe, one SM's worth.  CTA r of a (signal,
-// shift) transforms the samples a[8m + r] (m < M = W/8) in shared memory,
-// multiplies entry m by w_W^(r m) and stores Y_r; k_v3_man_combine then
-// forms X[k + M q] = sum_r Y_r[k] w_8^(r q) (a radix-2 FFT of 8 points per
-// k).  The arithmetic differs from the one-CTA Stockham order only in
-// rounding (the v3 results are held to 1e-10 of the reference's).
-constexpr int V3_MAN_SPLIT = 8;
+// The filters of one signal of n = 2^24, k = 1000: 103 us with a CTA per role
+// (96 k cycles for the contiguous Gaussian's alone), 22 us spread like this.
+//
+// Work of k_v3_first per signal, in CTAs of V3_T threads: Mansour tiles of
+// both shifts, groups of buckets of the two Gaussian folds (both shifts, each
+// bucket's taps over several lanes), and blocks of the result table to clear.
+constexpr int V3_T = 128;
+constexpr int V3_S1 = 4, V3_S2 = 8;            // lanes per bucket and shift of the two folds
+constexpr int V3_G1 = V3_T / (2 * V3_S1);      // buckets per CTA
+constexpr int V3_G2 = V3_T / (2 * V3_S2);
+constexpr int V3_CLEAR = 16 * 4 * V3_T;        // table entries cleared per CTA
 
-__global__ void __launch_bounds__(256) k_v3_man_split(V3Dev d) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int M = d.W / V3_MAN_SPLIT;
-  double2 *buf = (double2 *)smem_raw;  // [M]
-  double2 *tws = buf + M;              // [M]: w_M^e = w_W^(8 e)
-  const int r = blockIdx.x, l = blockIdx.y, slot = blockIdx.z;
-  const int *rp = d.rparams + (long)slot * d.rp_stride;
-  const unsigned long long mask = (unsigned long long)d.n - 1;
-  const long sigma = d.n / d.W, o = rp[3] + l;
-  const double2 *tw = (const double2 *)d.tw_man;
-  const void *x = d.inputs[slot];
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    tws[m] = __ldg(tw + V3_MAN_SPLIT * m);
-    buf[m] = ld_x(x, d.in_type, (long)((unsigned long long)(o + (long)(V3_MAN_SPLIT * m + r) * sigma) & mask));
+struct V3Shape {
+  int elems[2];    // Mansour tile entries of the two launches
+  int man[2];      // Mansour CTAs per shift of the two launches
+  int n1, n2, nc;  // Gaussian fold CTAs, table-clearing CTAs
+  int chunks2;
+};
+
+// Buckets [b0, b0 + G) of one Gaussian filter, both shifts: thread = ((bucket
+// - b0) * 2 + shift) * S + part; part p takes taps p, p + S, ... of its bucket.
+template <int G, int S, typename Val>
+__device__ __forceinline__ void v3_fold(int b0, int B, int chunks, const double2 *taps, double2 *dst, Val val) {
+  const int part = threadIdx.x % S, o = threadIdx.x / S, l = o & 1, b = b0 + (o >> 1);
+  double2 acc = make_double2(0.0, 0.0);
+  if (b < B) {
+#pragma unroll 4
+    for (int c = part; c < chunks; c += S) acc = cfma(val(b - b0, c, l), __ldg(taps + (long)c * B + b), acc);
   }
-  __syncthreads();
-  block_fft<double, 1>(buf, M, 31 - __clz(M), tws);
-  double2 *Y = (double2 *)d.man_tmp + (long)slot * 4 * d.W + (long)l * d.W + (long)r * M;
-  for (int m = threadIdx.x; m < M; m += blockDim.x) Y[m] = cmul<double>(buf[m], __ldg(tw + r * m));
+#pragma unroll
+  for (int s = S / 2; s > 0; s >>= 1) {
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, s);
+    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, s);
+  }
+  if (b < B && part == 0) dst[2 * b + l] = acc;
 }
 
-__global__ void __launch_bounds__(128) k_v3_man_combine(V3Dev d) {
-  const int M = d.W / V3_MAN_SPLIT;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x, l = blockIdx.y, slot = blockIdx.z;
-  if (k >= M) return;
-  const double2 *Y = (const double2 *)d.man_tmp + (long)slot * 4 * d.W + (long)l * d.W;
-  const double2 *tw = (const double2 *)d.tw_man;
-  double2 v[V3_MAN_SPLIT];
-  constexpr int br[V3_MAN_SPLIT] = {0, 4, 2, 6, 1, 5, 3, 7};  // bit-reversed r
-#pragma unroll
-  for (int i = 0; i < V3_MAN_SPLIT; i++) v[i] = Y[(long)br[i] * M + k];
-#pragma unroll
-  for (int h = 1; h < V3_MAN_SPLIT; h *= 2) {
-#pragma unroll
-    for (int s0 = 0; s0 < V3_MAN_SPLIT; s0 += 2 * h) {
-#pragma unroll
-      for (int j = 0; j < h; j++) {
-        // w_8^(j 8 / (2 h)) = w_W^(M j 8 / (2 h))
-        const double2 t = j ? cmul<double>(v[s0 + j + h], __ldg(tw + (long)M * j * (V3_MAN_SPLIT / (2 * h))))
-                            : v[s0 + j + h];
-        const double2 u = v[s0 + j];
-        v[s0 + j] = cadd<double>(u, t);
-        v[s0 + j + h] = csub<double>(u, t);
-      }
-    }
+__global__ void __launch_bounds__(V3_T) k_v3_first(V3Dev d, V3Shape sh) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int slot = blockIdx.y;
+  int x = blockIdx.x;
+  const int *rp = d.rparams + (long)slot * d.rp_stride;
+  const unsigned mask = (unsigned)d.n - 1u;
+  const void *in = d.inputs[slot];
+  const int in_type = d.in_type;
+  if (x == 0 && threadIdx.x < CNT_STRIDE) d.counters[slot * CNT_STRIDE + threadIdx.x] = 0;
+  if (x < 2 * sh.man[0]) {  // Mansour: x[(init_offset + l + i * n/W) mod n]
+    const int l = x / sh.man[0], tile = x - l * sh.man[0], W = d.W;
+    const int M = W / fft_m2(W), lc = fft_lc(sh.elems[0], M, W);
+    const unsigned sigma = (unsigned)(d.n / W), o = (unsigned)(rp[3] + l);
+    double2 *dst = (double2 *)d.man_tmp + ((long)slot * 2 + l) * W;
+    fft_tile<double>((double2 *)smem_raw, M, lc, 1, W, tile << lc, floor_log2(W) & 1, (const double2 *)d.tw_man,
+                     [=](int i) { return ld_x(in, in_type, (long)((o + (unsigned)i * sigma) & mask)); },
+                     [=](int i, double2 v) { dst[i] = v; });
+    return;
   }
-  double2 *man = (double2 *)d.man + (long)slot * 2 * d.W;
-#pragma unroll
-  for (int q = 0; q < V3_MAN_SPLIT; q++) man[2 * (k + M * q) + l] = v[q];
+  x -= 2 * sh.man[0];
+  if (x < sh.n1) {  // Gaussian 1: taps over x[init_G_offset + l + t]
+    const int b0 = x * V3_G1, B = d.B1;
+    const unsigned base = (unsigned)rp[4];
+    v3_fold<V3_G1, V3_S1>(b0, B, d.w1 / B, (const double2 *)d.taps1, (double2 *)d.g1 + (long)slot * 2 * B,
+                          [=](int b, int c, int l) {
+                            return ld_x(in, in_type, (long)((base + (unsigned)(c * B + b0 + b + l)) & mask));
+                          });
+    return;
+  }
+  x -= sh.n1;
+  if (x < sh.n2) {
+    // Gaussian 2 on permuted, phase-shifted samples.  permute_fourier
+    // (computefourier-3.0.cc:66-87): sample i is x[(ig + i*ai) mod n] *
+    // shift_i with shift_0 = e^{2 pi i ig b / n} and shift_{i+1} = shift_i *
+    // e^{2 pi i ai b / n}, a running product.  The two angles are formed as
+    // there (the same FP64 products); shift_i = e^{i (a0 + i a1)} directly,
+    // one sample per thread -- replaying the product serially costs about 64
+    // cycles per operation (2945 steps at n = 2^24, k = 1000: 0.58 ms).  Its
+    // error, about 3e-16, is below the serial chain's accumulated rounding
+    // (about i * 2^-53) and far inside the 1e-10 value tolerance.
+    const int b0 = x * V3_G2, B = d.B2, chunks = sh.chunks2, G = min(V3_G2, B - b0);
+    const unsigned ig = (unsigned)rp[4], ai = (unsigned)rp[1];
+    const int bb = rp[2];
+    const double a0 = 2 * kPi * rp[4] * bb / d.n, a1 = 2 * kPi * rp[1] * bb / d.n;
+    const double2 *trig = (const double2 *)d.trig;
+    double2 *P = (double2 *)smem_raw;  // [chunk][G + 1]: the shifts use samples b and b + 1
+    for (int t = threadIdx.x; t < chunks * (V3_G2 + 1); t += V3_T) {
+      const int c = t / (V3_G2 + 1), k = t - c * (V3_G2 + 1);
+      if (k > G) continue;
+      const int i = c * B + b0 + k;
+      P[t] = cfma(ld_x(in, in_type, (long)((ig + (unsigned)i * ai) & mask)), cis_step(trig, a0, i, a1),
+                  make_double2(0.0, 0.0));
+    }
+    __syncthreads();
+    v3_fold<V3_G2, V3_S2>(b0, B, chunks, (const double2 *)d.taps2, (double2 *)d.g2 + (long)slot * 2 * B,
+                          [=](int b, int c, int l) { return P[c * (V3_G2 + 1) + b + l]; });
+    return;
+  }
+  x -= sh.n2;
+  int4 *keys = (int4 *)(d.map_keys + (long)slot * d.table_cap) + (long)x * (V3_CLEAR / 4);
+  for (int t = threadIdx.x; t < V3_CLEAR / 4 && (long)x * V3_CLEAR + 4 * t < d.table_cap; t += V3_T)
+    keys[t] = make_int4(-1, -1, -1, -1);
+}
+
+// blockDim.x >= V3_T: a quarter of the longest Gaussian bucket FFT (at most
+// 1024, PER butterflies per thread).
+template <int PER>
+__global__ void __launch_bounds__(1024) k_v3_second(V3Dev d, V3Shape sh) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int slot = blockIdx.y;
+  int x = blockIdx.x;
+  if (x < 2 * sh.man[1]) {
+    const int l = x / sh.man[1], tile = x - l * sh.man[1], W = d.W, M = fft_m2(W), lc = fft_lc(sh.elems[1], M, W);
+    const double2 *src = (const double2 *)d.man_tmp + ((long)slot * 2 + l) * W;
+    double2 *dst = (double2 *)d.man + (long)slot * 2 * W;
+    fft_tile<double>((double2 *)smem_raw, M, lc, W / M, W, tile << lc, false, (const double2 *)d.tw_man,
+                     [=](int i) { return src[i]; }, [=](int i, double2 v) { dst[2 * i + l] = v; });
+    return;
+  }
+  x -= 2 * sh.man[1];
+  const int l = x & 1, B = x < 2 ? d.B1 : d.B2;
+  double2 *buf = (double2 *)smem_raw, *g = (x < 2 ? (double2 *)d.g1 : (double2 *)d.g2) + (long)slot * 2 * B;
+  for (int i = threadIdx.x; i < B; i += blockDim.x) buf[i] = g[2 * i + l];
+  __syncthreads();
+  block_fft<double, PER>(buf, B, floor_log2(B), (const double2 *)(x < 2 ? d.tw_g1 : d.tw_g2));
+  for (int i = threadIdx.x; i < B; i += blockDim.x) g[2 * i + l] = buf[i];
 }
 
 // ------------------------------------------------------------------ peel --
+//
+// A request's rounds run each piece of this kernel a few times, so its time
+// is latency: chains of FP64 instructions (about 100 from a bucket's values
+// to the subtraction of its tone), L2 round trips and cluster barriers.  What
+// was taken out of the chains, with the kernel's time for one signal of n =
+// 2^24, k = 1000 (6 rounds) and for 16 of n = 2^18, k = 100: library atan2 /
+// sincos and 8 CTAs 202 / 208 us; table phases and 16 CTAs 148 / 168; no
+// divisions for constants in every warp (8 warps a sub-partition, 64 cycles
+// an instruction) and lists by exponent 104 / 114; tones peeled by the CTA
+// that found them, from shared memory, and the barrier after reading the
+// buckets split around the estimates' arithmetic 83 / 101.
 
+// State of a signal's rounds, the same for every thread of a CTA (shared
+// memory).
 struct PeelCtx {
-  const V3Dev *d;
-  int n, n1;
+  V3Dev d;
+  int n1, lw, a, ai, b, io, ig, aG, shift, tmask, rank, nb;
   double2 *man, *g1, *g2;
   int *tkey;
   double2 *tval;
   int *list;
-  int tmask;
   int *est_f;
   double2 *est_v;
-  int a, ai, b, io, ig, aG, shift;
+  int *counters;
+  double slope[2], off[2];  // 2 pi ig / n and 2 pi a ig / n; the comb offsets io and io + 1
+  // counters of the cluster (the first CTA's shared memory)
+  int *count, *err;
+  double2 trig[1 << TRIG_BITS];  // V3Dev::trig: a cluster barrier drops what L1 holds
 };
 
 __device__ __forceinline__ double2 win_at(const double2 *win, int half, int n, int dist, int *err) {
@@ -252,80 +320,57 @@ __device__ __forceinline__ double2 win_at(const double2 *win, int half, int n, i
 
 __device__ __forceinline__ int wrapmul(int x, int y) { return (int)((unsigned)x * (unsigned)y); }
 
-// Subtract a recovered tone from the three nearest buckets of both shifts
-// of a Gaussian filter (computefourier-3.0.cc:354-463).
-__device__ void update_gauss(const PeelCtx &c, double2 *SAMP, const double2 *win, int half, int B,
-                             int key, double2 v, int offset, int step, int l, int *err) {
-  const int n = c.n, n1 = c.n1;
-  const unsigned q = n / B;
-  // key / q with q a power of two: the product with 1 / q is the same double
-  const int h = (int)(key * (1. / q) + 0.5) % B;
-  const int dist1 = (int)(((unsigned)h * q - (unsigned)key + (unsigned)n) & (unsigned)n1);
-  const int dist2 = (int)(((unsigned)dist1 + (unsigned)n + q) & (unsigned)n1);
-  const int dist3 = (int)(((unsigned)dist1 + 2u * (unsigned)n - q) & (unsigned)n1);
-  // shift l of the two: time offset `offset` (l = 0) or `offset + step` (l = 1)
-  const int ko = wrapmul(key, (int)((unsigned)offset + (l ? (unsigned)step : 0u))) % n;
-  const double PI2_DIV_N = 2 * kPi / n;
-  double sn, cs;
-  sincos(PI2_DIV_N * ko, &sn, &cs);
-  const double2 vl = cmul<double>(v, make_double2(cs, sn));
-  const int dists[3] = {dist1, dist2, dist3};
-  const int bks[3] = {h, (h + 1) % B, (h + B - 1) % B};
-#pragma unroll
-  for (int qd = 0; qd < 3; qd++) {
-    const double2 f = win_at(win, half, n, dists[qd], err);
-    const double2 r = cmul<double>(vl, f);
-    double *p = (double *)&SAMP[2 * bks[qd] + l];
-    atomicAdd(p, -r.x);
-    atomicAdd(p + 1, -r.y);
-  }
-}
-
-// (computefourier-3.0.cc:300-351), shift l of the two
-__device__ void update_mansour(const PeelCtx &c, int key, double2 v, int l) {
-  const int W = c.d->W;
-  const int h = key & (W - 1);
-  const double PI2_OVER_N = 2 * kPi / c.n;
-  double s, co;
-  sincos(PI2_OVER_N * key * (double)(c.io + l), &s, &co);
-  const double rr = (double)W * (v.x * co - v.y * s);
-  const double ri = (double)W * (v.x * s + v.y * co);
-  double *p = (double *)&c.man[2 * h + l];
-  atomicAdd(p, -rr);
-  atomicAdd(p + 1, -ri);
-}
-
 // Subtraction of a recovered tone from one filter's buckets of one shift:
 // part = 2 * filter + shift, filter 0 the permuted Gaussian, 1 the
-// contiguous Gaussian, 2 the Mansour comb.  The six parts of a tone are
-// independent (atomic subtractions), so they are separate work items:
-// their FP64 chains (one sincos each) run on different sub-partitions.
-__device__ void update_part(const PeelCtx &c, int key, double2 v, int part, int *err) {
-  const V3Dev &d = *c.d;
+// contiguous Gaussian (the three nearest buckets, computefourier-3.0.cc:
+// 354-463), 2 the Mansour comb (:300-351).  The six parts of a tone are
+// independent (atomic subtractions), so they are separate work items: their
+// FP64 chains run on different sub-partitions.
+__device__ __forceinline__ void update_part(const PeelCtx &c, int key, double2 v, int part) {
+  const V3Dev &d = c.d;
   const int l = part & 1;
-  if (part < 2) {
-    const int k2 = (int)((((long long)key * c.ai) % c.n + c.shift) % c.n);
-    update_gauss(c, c.g2, (const double2 *)d.win2, d.win2_half, d.B2, k2, v, c.aG, 1, l, err);
-  } else if (part < 4) {
-    update_gauss(c, c.g1, (const double2 *)d.win1, d.win1_half, d.B1, key, v, c.ig, 1, l, err);
+  const double2 zero = make_double2(0.0, 0.0);
+  if (part < 4) {
+    const bool perm = part < 2;
+    const int B = perm ? d.B2 : d.B1, half = perm ? d.win2_half : d.win1_half;
+    const double2 *win = (const double2 *)(perm ? d.win2 : d.win1);
+    double2 *samp = perm ? c.g2 : c.g1;
+    const unsigned f = perm ? ((unsigned)key * (unsigned)c.ai + (unsigned)c.shift) & (unsigned)c.n1 : (unsigned)key;
+    const int lq = d.logn - floor_log2(B);
+    const unsigned q = 1u << lq;
+    const int h = (int)(((f + (q >> 1)) >> lq) & (unsigned)(B - 1));  // (int)(f / q + 0.5)
+    const unsigned dist = (unsigned)h * q - f;
+    // shift l: time offset `offset` + l; the phase 2 pi ko / n is the integer
+    // ko mod n of n-ths of a turn
+    const unsigned ko = (f * ((unsigned)(perm ? c.aG : c.ig) + (unsigned)l)) & (unsigned)c.n1;
+    const double2 vl = cfma(v, cis_turn(c.trig, (unsigned long long)ko << (64 - d.logn)), zero);
+#pragma unroll 1
+    for (int qd = -1; qd < 2; qd++) {
+      const double2 r = cfma(vl, win_at(win, half, d.n, (int)((dist + (unsigned)qd * q) & (unsigned)c.n1), c.err), zero);
+      double *p = (double *)&samp[2 * ((h + qd) & (B - 1)) + l];
+      atomicAdd(p, -r.x);
+      atomicAdd(p + 1, -r.y);
+    }
   } else {
-    update_mansour(c, key, v, l);
+    const double2 r = cfma(v, cis(c.trig, d.pi2_over_n * key * c.off[l]), zero);
+    double *p = (double *)&c.man[2 * (key & (d.W - 1)) + l];
+    atomicAdd(p, -(d.w_dbl * r.x));
+    atomicAdd(p + 1, -(d.w_dbl * r.y));
   }
 }
 
 // Result map: key -> accumulated value; returns nothing, keys of one round
 // are distinct so the value update has a single writer.
-__device__ void map_add(const PeelCtx &c, int key, double2 v, bool assign, int *count, int cap,
-                        int *err) {
+__device__ __forceinline__ void map_add(const PeelCtx &c, int key, double2 v, bool assign) {
   unsigned h = ((unsigned)key * 2654435761u) & (unsigned)c.tmask;
   for (int probe = 0; probe <= c.tmask; probe++) {
     const int cur = atomicCAS(&c.tkey[h], -1, key);
     if (cur == -1) {
-      const int idx = atomicAdd(count, 1);
-      if (idx < cap)
+      const int idx = atomicAdd(c.count, 1);
+      if (idx < c.d.map_cap)
         c.list[idx] = (int)h;
       else
-        atomicOr(err, ERR_V3_CAP);
+        atomicOr(c.err, ERR_V3_CAP);
       c.tval[h] = v;
       return;
     }
@@ -340,17 +385,16 @@ __device__ void map_add(const PeelCtx &c, int key, double2 v, bool assign, int *
     }
     h = (h + 1) & (unsigned)c.tmask;
   }
-  atomicOr(err, ERR_V3_CAP);
+  atomicOr(c.err, ERR_V3_CAP);
 }
 
-// The estimation loops below visit every bucket, but only buckets that pass
-// the reference's zero-bucket check do FP64 work (atan2, sincos, sqrt) --
-// and on GB300 a warp's FP64 instruction occupies its SM sub-partition's
-// narrow FP64 pipe for tens of cycles whether one lane or 32 are active.
-// So each CTA first lists its passing buckets in shared memory (the cheap
-// check), then deals the list out one per lane over warps of all four
-// sub-partitions: the FP64 work of a phase costs about one warp's chain
-// per sub-partition instead of one per warp that holds a passing bucket.
+// The estimation loops below visit every bucket, but FP64 work is done only
+// on listed ones: a warp's FP64 instruction occupies its SM sub-partition's
+// FP64 pipe for 64 cycles and more whether one lane or 32 are active.  So each
+// CTA lists the buckets that are not empty by their exponents alone, deals
+// the list out one per lane over warps of all four sub-partitions, keeps the
+// entries that pass the reference's tests in a second list, and deals those
+// out again: an item per angle and one per magnitude, then one per value.
 constexpr int V3_LIST = 1024;  // list entries per CTA and pass (= threads per CTA)
 
 // Position in the list of thread `tid` of a 1024-thread CTA: consecutive
@@ -359,156 +403,126 @@ __device__ __forceinline__ int v3_spread(int tid) {
   return ((tid >> 7) << 7) | ((tid & 31) << 2) | ((tid >> 5) & 3);
 }
 
-// Per-CTA shared scratch of the estimation loops: the list of passing
-// buckets and, per (entry, shift), the phase and one more quantity.  Each
-// passing bucket is two work items in a first step -- the atan2 of one
-// shift each, plus sqrt(c0) or 1 / c0 -- and one in a second step, so its
-// FP64 chain is split over two sub-partitions.
+// Per-CTA shared scratch of the estimation loops, and the tones that the CTA
+// found in the current phase (beyond V3_LIST in est_f / est_v, which have
+// room for one tone per bucket that the CTA visits).
 struct EstScratch {
-  int list[V3_LIST];
-  int cnt;
-  double ang[2 * V3_LIST], aux[2 * V3_LIST];
+  int raw[V3_LIST], list[V3_LIST], key[V3_LIST];
+  int nraw, cnt, tones;
+  double c0[V3_LIST], ang[2 * V3_LIST], mag[V3_LIST];
+  double2 s[2 * V3_LIST], val[V3_LIST];
 };
 
-// Lists this CTA's buckets among [base + t0] (one per thread) that pass
-// `pass`; every thread of the CTA calls it.  Returns the count.
-__device__ __forceinline__ int est_list(EstScratch &x, int bk, bool pass) {
-  if (threadIdx.x == 0) x.cnt = 0;
-  __syncthreads();
-  if (pass) x.list[atomicAdd(&x.cnt, 1)] = bk;
-  __syncthreads();
-  return x.cnt;
-}
-
-// estimate_freq_mansour_loops2 (computefourier-3.0.cc:642-776)
-__device__ void est_mansour(const PeelCtx &c, int *nfound, int cap, int *err, int t0, int tstride, EstScratch &x) {
-  const int W = c.d->W, n = c.n;
-  const double PI2 = 2 * kPi, N_OVER_PI2 = n / PI2, PI2_OVER_N = PI2 / n;
-  const unsigned FREQ_MASK = ((unsigned)(n - 1) & ~((unsigned)W - 1));
-  const double NORM = 1. / W, NORM2 = NORM * NORM;
-  for (int base = 0; base < W; base += tstride) {
-    const int bk0 = base + t0;
-    bool pass = false;
-    if (bk0 < W) {
-      const double2 s0 = c.man[2 * bk0], s1 = c.man[2 * bk0 + 1];
-      const double c0 = (s0.x * s0.x + s0.y * s0.y) * NORM2;
-      const double c1 = (s1.x * s1.x + s1.y * s1.y) * NORM2;
-      pass = c0 + c1 > 1e-8;
-    }
-    const int cnt = est_list(x, bk0, pass);
-    for (int w = v3_spread(threadIdx.x); w < 2 * cnt; w += V3_LIST) {
-      const int bk = x.list[w >> 1], l = w & 1;
-      const double2 sl = c.man[2 * bk + l];
-      x.ang[w] = atan2(sl.y * NORM, sl.x * NORM);
-      const double2 s0 = c.man[2 * bk];
-      const double c0 = (s0.x * s0.x + s0.y * s0.y) * NORM2;
-      x.aux[w] = l ? 1. / c0 : sqrt(c0);
-    }
-    __syncthreads();
-    for (int e = v3_spread(threadIdx.x); e < cnt; e += V3_LIST) {
-      const int bk = x.list[e];
-      const double2 s1 = c.man[2 * bk + 1];
-      const double c1 = (s1.x * s1.x + s1.y * s1.y) * NORM2;
-      const double s0x = c.man[2 * bk].x, s0y = c.man[2 * bk].y;
-      const double c0 = (s0x * s0x + s0y * s0y) * NORM2;
-      const double d0 = x.ang[2 * e], d1 = x.ang[2 * e + 1];
-      const double bb = (c1 * x.aux[2 * e + 1]) - 1;
-      if ((bb * bb < n * 1e-10) && (c0 > 0.01)) {
-        const int freq1 = (int)__double2ll_rn((d1 - d0) * N_OVER_PI2);
-        const int freq3 = (int)((unsigned)freq1 & FREQ_MASK) | bk;
-        const double ph = d0 - PI2_OVER_N * wrapmul(freq3, c.io);
-        const double ab = x.aux[2 * e];
-        double sn, co;
-        sincos(ph, &sn, &co);
-        const int i = atomicAdd(nfound, 1);
-        if (i < cap) {
-          c.est_f[i] = freq3;
-          c.est_v[i] = make_double2(ab * co, ab * sn);
-        } else {
-          atomicOr(err, ERR_V3_CAP);
-        }
-      }
-    }
-    __syncthreads();  // the scratch is reused by the next pass
+__device__ __forceinline__ void tone_put(const PeelCtx &c, EstScratch &x, int key, double2 v) {
+  const int i = atomicAdd(&x.tones, 1);
+  if (i < V3_LIST) {
+    x.key[i] = key;
+    x.val[i] = v;
+  } else {
+    c.est_f[i - V3_LIST] = key;
+    c.est_v[i - V3_LIST] = v;
   }
 }
+__device__ __forceinline__ int tone_key(const PeelCtx &c, const EstScratch &x, int i) {
+  return i < V3_LIST ? x.key[i] : c.est_f[i - V3_LIST];
+}
+__device__ __forceinline__ double2 tone_val(const PeelCtx &c, const EstScratch &x, int i) {
+  return i < V3_LIST ? x.val[i] : c.est_v[i - V3_LIST];
+}
 
-// estimate_freq_gauss_loops2 (computefourier-3.0.cc:484-640)
-__device__ void est_gauss(const PeelCtx &c, const double2 *SAMP, int B, const double2 *win,
-                          int half, int a, int b, int *nfound, int cap, int *err, int t0, int tstride,
-                          EstScratch &x) {
-  const int n = c.n;
-  const unsigned n1 = n - 1, B1 = B - 1;
-  const double PI2 = 2 * kPi, N_OVER_PI2 = n / PI2;
-  const double PI2_A_OFFSET_OVER_N = PI2 * a * c.ig / n;
-  const double BUCKETS_OVER_N = (double)B / n;
-  const double INV_N = 1. / n;  // n is a power of two: the product equals the quotient
-  const unsigned q = n / B;
-  for (int base = 0; base < B; base += tstride) {
-    const int bk0 = base + t0;
-    bool pass = false;
-    if (bk0 < B) {
-      const double2 s0 = SAMP[2 * bk0], s1 = SAMP[2 * bk0 + 1];
-      const double c0 = s0.x * s0.x + s0.y * s0.y;
-      const double c1 = s1.x * s1.x + s1.y * s1.y;
-      pass = c0 + c1 > 1e-8;
+// Finds this CTA's tones of one filter.  stage 0: estimate_freq_mansour_loops2
+// (computefourier-3.0.cc:642-776) on the comb; 1, 2:
+// estimate_freq_gauss_loops2 (:484-640) on the contiguous and the permuted
+// Gaussian buckets.  Every thread of the CTA calls it.  The cluster barrier's
+// first half (arrive) comes once the CTA has read its last bucket; the caller
+// waits for the second half before it changes any bucket.
+__device__ __noinline__ void estimate(const PeelCtx &c, int stage, EstScratch &x) {
+  const V3Dev &d = c.d;
+  const int gt = v3_spread(threadIdx.x) * c.nb + c.rank, T = V3_LIST * c.nb, t = v3_spread(threadIdx.x);
+  const bool comb = stage == 0, perm = stage == 2;
+  const double2 *s = comb ? c.man : perm ? c.g2 : c.g1;
+  const int B = comb ? d.W : perm ? d.B2 : d.B1, lw = comb ? c.lw : 0;
+  const double norm2 = comb ? d.inv_w2 : 1.0, tol = comb ? d.tol_man : d.tol_gauss;
+  const unsigned n1 = (unsigned)c.n1;
+  if (threadIdx.x == 0) x.tones = 0;
+#pragma unroll 1
+  for (int base = 0; base < B; base += T) {
+    // not empty: c0 + c1 > 1e-8 needs a component of at least 5e-5
+    if (threadIdx.x == 0) x.nraw = x.cnt = 0;
+    __syncthreads();
+    const int bk0 = base + gt;
+    if (bk0 < B && (reaches(s[2 * bk0], lw - 15) || reaches(s[2 * bk0 + 1], lw - 15)))
+      x.raw[atomicAdd(&x.nraw, 1)] = bk0;
+    __syncthreads();
+    // c0 + c1 > 1e-8, c0 > 0.01 and (c1 / c0 - 1)^2 < tol
+    if (t < x.nraw) {
+      const int bk = x.raw[t];
+      const double2 s0 = s[2 * bk], s1 = s[2 * bk + 1];
+      const double c0 = fma(s0.x, s0.x, s0.y * s0.y) * norm2, c1 = fma(s1.x, s1.x, s1.y * s1.y) * norm2;
+      const double b = c1 - c0;
+      if (c0 + c1 > 1e-8 && c0 > 0.01 && b * b < tol * (c0 * c0)) {
+        const int i = atomicAdd(&x.cnt, 1);
+        x.list[i] = bk;
+        x.c0[i] = c0;
+        x.s[2 * i] = s0;
+        x.s[2 * i + 1] = s1;
+      }
     }
-    const int cnt = est_list(x, bk0, pass);
-    for (int w = v3_spread(threadIdx.x); w < 2 * cnt; w += V3_LIST) {
-      const int bk = x.list[w >> 1], l = w & 1;
-      const double2 sl = SAMP[2 * bk + l];
-      x.ang[w] = atan2(sl.y, sl.x);
-      const double2 s0 = SAMP[2 * bk];
-      const double c0 = s0.x * s0.x + s0.y * s0.y;
-      if (l) {
-        const double c1 = sl.x * sl.x + sl.y * sl.y;
-        x.aux[w] = c1 / c0 - 1;
+    __syncthreads();
+    if (base + T >= B) cg::this_cluster().barrier_arrive();
+    const int cnt = x.cnt, m0 = (2 * cnt + 127) & ~127;  // magnitudes in warps of their own
+#pragma unroll 1
+    for (int w = t; w < m0 + cnt; w += V3_LIST) {
+      if (w < 2 * cnt)
+        x.ang[w] = angle_of(c.trig, x.s[w].y, x.s[w].x);  // the scale does not change the angle
+      else if (w >= m0)
+        x.mag[w - m0] = sqrt_of(x.c0[w - m0]);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int e = t; e < cnt; e += V3_LIST) {
+      const double d0 = x.ang[2 * e], ab = x.mag[e];
+      const int fr = (int)__double2ll_rn((x.ang[2 * e + 1] - d0) * d.n_over_pi2);
+      const int bk = x.list[e];
+      unsigned freq, dist = 0;
+      double ph;
+      if (comb) {
+        freq = ((unsigned)fr & n1 & ~((unsigned)B - 1u)) | (unsigned)bk;
+        ph = d0 - d.pi2_over_n * wrapmul((int)freq, c.io);
       } else {
-        x.aux[w] = sqrt(c0);
+        freq = (unsigned)(fr + d.n) & n1;
+        const int lq = d.logn - floor_log2(B);
+        const unsigned q = 1u << lq, down = freq >> lq, rest = 2u * (freq & (q - 1u));
+        // freq / q rounded to nearest, ties to even
+        const unsigned hashed = (down + (rest > q || (rest == q && (down & 1u)))) & ((unsigned)B - 1u);
+        if (hashed != (unsigned)bk) continue;
+        dist = (hashed * q - freq) & n1;
+        ph = d0 - c.slope[perm] * (int)freq;
       }
-    }
-    __syncthreads();
-    for (int e = v3_spread(threadIdx.x); e < cnt; e += V3_LIST) {
-      const int bk = x.list[e];
-      const double2 s0 = SAMP[2 * bk];
-      const double c0 = s0.x * s0.x + s0.y * s0.y;
-      const double d0 = x.ang[2 * e], d1 = x.ang[2 * e + 1];
-      const double eb = x.aux[2 * e + 1];
-      const double err2 = (eb * eb) * INV_N;
-      if ((err2 < 1e-12) && (c0 > 0.01)) {
-        const int freq = (int)((unsigned)((int)__double2ll_rn(N_OVER_PI2 * (d1 - d0)) + n) & n1);
-        const unsigned hashed = (unsigned)__double2ll_rn(freq * BUCKETS_OVER_N) & B1;
-        if (hashed == (unsigned)bk) {
-          const double ph = d0 - PI2_A_OFFSET_OVER_N * freq;
-          const double r = x.aux[2 * e];
-          double sn, co;
-          sincos(ph, &sn, &co);
-          const double mr = r * co, mi = r * sn;
-          const int dist = (int)((hashed * q - (unsigned)freq + (unsigned)n) & n1);
-          const double2 f = win_at(win, half, n, dist, err);
-          const double den = f.x * f.x + f.y * f.y;
-          const double2 v = make_double2((mr * f.x + mi * f.y) / den, (mi * f.x - mr * f.y) / den);
-          const int fo = (int)((unsigned)((int)(((long long)freq * a) % n) - b + n) & n1);
-          const int i = atomicAdd(nfound, 1);
-          if (i < cap) {
-            c.est_f[i] = fo;
-            c.est_v[i] = v;
-          } else {
-            atomicOr(err, ERR_V3_CAP);
-          }
-        }
+      // the window's value is asked for before the phase is worked out
+      const double2 f = comb ? make_double2(1.0, 0.0)
+                             : win_at((const double2 *)(perm ? d.win2 : d.win1), perm ? d.win2_half : d.win1_half, d.n,
+                                      (int)dist, c.err);
+      const double2 w = cis(c.trig, ph);
+      double2 v = make_double2(ab * w.x, ab * w.y);
+      if (!comb) {  // divided by the window
+        const double den = fma(f.x, f.x, f.y * f.y), inv = recip_of(den);
+        const double2 num = make_double2(fma(v.x, f.x, v.y * f.y), fma(v.y, f.x, -(v.x * f.y)));
+        const double2 q0 = make_double2(num.x * inv, num.y * inv);  // corrected by the remainders
+        v = make_double2(fma(fma(-q0.x, den, num.x), inv, q0.x), fma(fma(-q0.y, den, num.y), inv, q0.y));
+        if (perm) freq = (freq * (unsigned)c.a - (unsigned)c.b) & n1;
       }
+      tone_put(c, x, (int)freq, v);
     }
-    __syncthreads();  // the scratch is reused by the next pass
+    __syncthreads();  // the tones are complete, and the lists free for the next pass
   }
 }
 
-__device__ __forceinline__ void trace_rec(const V3Dev &d, int slot, int *cnt, int round, int stage, int key,
-                                          double2 v) {
-  if (slot != 0 || !d.trace) return;
-  const int i = atomicAdd(&cnt[CNT_TRACE], 1);
-  if (i < d.trace_cap) {
-    double *t = d.trace + 5 * (long)i;
+__device__ __forceinline__ void trace_rec(const PeelCtx &c, int round, int stage, int key, double2 v) {
+  if (!c.d.trace) return;
+  const int i = atomicAdd(&c.counters[CNT_TRACE], 1);
+  if (i < c.d.trace_cap) {
+    double *t = c.d.trace + 5 * (long)i;
     t[0] = round;
     t[1] = stage;
     t[2] = key;
@@ -517,173 +531,174 @@ __device__ __forceinline__ void trace_rec(const V3Dev &d, int slot, int *cnt, in
   }
 }
 
-// One thread-block cluster of V3_CLUSTER CTAs per signal runs the
-// estimate / peel rounds: every loop over buckets, estimates and map
-// entries is spread over the cluster's threads, and each block-wide
-// barrier of the round structure is a cluster barrier (release / acquire
-// at cluster scope, so the global-memory bucket arrays and the map written
-// before it are visible after it).  The round's counters live in the
-// shared memory of the cluster's first CTA and are updated through
-// distributed shared memory.  Control flow is uniform across the cluster:
-// every branch is taken on values read after a barrier.
-constexpr int V3_CLUSTER = 8;
+// Peels parts p0 .. p0 + np of `mine` tones: the CTA's estimates, or (known)
+// the entries rank, rank + nb, ... of the result map.  A warp takes one part
+// of 32 tones, so the two forms of update_part do not meet in a warp; new
+// estimates go to the map (add: to what it holds, else in its place) as a
+// part of their own.
+__device__ __noinline__ void subtract(const PeelCtx &c, const EstScratch &x, int mine, int p0, int np, bool known,
+                                      bool to_map, bool assign, int round, int stage) {
+  const int parts = np + (to_map ? 1 : 0), warps = parts * ((mine + 31) >> 5);
+#pragma unroll 1
+  for (int u = threadIdx.x >> 5; u < warps; u += V3_LIST / 32) {
+    const int part = u % parts, i = (u / parts) * 32 + (threadIdx.x & 31);
+    if (i >= mine) continue;
+    const int h = known ? c.list[i * c.nb + c.rank] : 0;
+    const int key = known ? c.tkey[h] : tone_key(c, x, i);
+    const double2 v = known ? c.tval[h] : tone_val(c, x, i);
+    if (part < np) {
+      update_part(c, key, v, p0 + part);
+    } else {
+      trace_rec(c, round, stage, key, v);
+      map_add(c, key, v, assign);
+    }
+  }
+}
 
+// One thread-block cluster (8 or 16 CTAs) per signal runs the estimate /
+// peel rounds: every loop over buckets, estimates and map entries is spread
+// over the cluster's threads, and each block-wide barrier of the round
+// structure is a cluster barrier (release / acquire at cluster scope, so the
+// global-memory bucket arrays and the map written before it are visible
+// after it).  The round's counters live in the shared memory of the
+// cluster's first CTA and are updated through distributed shared memory; a
+// counter that a check adds to was cleared by the one before, so clearing
+// needs no barrier of its own.  A CTA peels the tones it found itself, from its
+// own shared memory: no estimate crosses L2, and the barrier between reading
+// the buckets and changing them runs beside the estimates' arithmetic.
+// Control flow is uniform across the cluster: every branch is taken on values
+// read after a barrier.
 struct PeelShared {
-  int found, count, err, cnt[3], prev[3], stop;
+  int found, count, err, cnt[2][3];
 };
 
-__global__ void __cluster_dims__(V3_CLUSTER, 1, 1) __launch_bounds__(1024) k_v3_peel(V3Dev d) {
-  __shared__ PeelShared sh_local;
-  cg::cluster_group cl = cg::this_cluster();
-  const int rank = (int)cl.block_rank();
-  PeelShared *S = cl.map_shared_rank(&sh_local, 0);
-  const int slot = blockIdx.x / V3_CLUSTER;
-  const int *rp = d.rparams + (long)slot * d.rp_stride;
+struct PeelMem {
   PeelCtx c;
-  c.d = &d;
-  c.n = d.n;
-  c.n1 = d.n - 1;
-  c.man = (double2 *)d.man + (long)slot * 2 * d.W;
-  c.g1 = (double2 *)d.g1 + (long)slot * 2 * d.B1;
-  c.g2 = (double2 *)d.g2 + (long)slot * 2 * d.B2;
-  c.tkey = d.map_keys + (long)slot * d.table_cap;
-  c.tval = (double2 *)d.map_vals + (long)slot * d.table_cap;
-  c.list = d.map_table + (long)slot * d.map_cap;
-  c.tmask = d.table_cap - 1;
-  c.est_f = d.est_f + (long)slot * d.est_cap;
-  c.est_v = (double2 *)d.est_v + (long)slot * d.est_cap;
-  c.a = rp[0];
-  c.ai = rp[1];
-  c.b = rp[2];
-  c.io = rp[3];
-  c.ig = rp[4];
-  c.aG = wrapmul(c.a, c.ig);
-  c.shift = ((wrapmul(c.ai, c.b) % d.n) + d.n) % d.n;
-  int *cnt = d.counters + slot * CNT_STRIDE;
-  // The cluster's threads; work item i of a loop over the cluster goes to
-  // CTA i mod 8 and, within it, to consecutive sub-partitions and lanes
-  // (v3_spread), so a short loop spreads its FP64 work over all 32
-  // sub-partitions of the cluster's SMs.
-  const int T = blockDim.x * V3_CLUSTER;
-  const int gt = v3_spread(threadIdx.x) * V3_CLUSTER + rank;
-  __shared__ EstScratch est_x;
-  const bool lead = rank == 0 && threadIdx.x == 0;
-  if (lead) {
-    S->found = 0;
-    S->count = 0;
-    S->err = 0;
-    S->stop = 0;
-    for (int i = 0; i < 3; i++) S->prev[i] = 0;
+  PeelShared sh;
+  EstScratch x;
+};
+
+__global__ void __launch_bounds__(V3_LIST) k_v3_peel(V3Dev dev) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  PeelMem &mem = *(PeelMem *)smem_raw;
+  PeelCtx &c = mem.c;
+  PeelShared &sh_local = mem.sh;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), nb = (int)cl.num_blocks();
+  PeelShared *S = cl.map_shared_rank(&sh_local, 0);
+  const int slot = blockIdx.x / nb;
+  const int *rp = dev.rparams + (long)slot * dev.rp_stride;
+  if (rank == 0 && threadIdx.x < sizeof(PeelShared) / sizeof(int)) ((int *)&sh_local)[threadIdx.x] = 0;
+  if (threadIdx.x == 0) {
+    c.d = dev;
+    if (slot) c.d.trace = nullptr;
+    c.n1 = dev.n - 1;
+    c.lw = floor_log2(dev.W);
+    c.man = (double2 *)dev.man + (long)slot * 2 * dev.W;
+    c.g1 = (double2 *)dev.g1 + (long)slot * 2 * dev.B1;
+    c.g2 = (double2 *)dev.g2 + (long)slot * 2 * dev.B2;
+    c.tkey = dev.map_keys + (long)slot * dev.table_cap;
+    c.tval = (double2 *)dev.map_vals + (long)slot * dev.table_cap;
+    c.list = dev.map_table + (long)slot * dev.map_cap;
+    c.tmask = dev.table_cap - 1;
+    // this CTA's share of the spill arrays: a tone per bucket it visits
+    const long share = (dev.est_cap - 16 * V3_LIST) / nb + V3_LIST;
+    c.est_f = dev.est_f + (long)slot * dev.est_cap + rank * share;
+    c.est_v = (double2 *)dev.est_v + (long)slot * dev.est_cap + rank * share;
+    c.counters = dev.counters + slot * CNT_STRIDE;
+    c.a = rp[0];
+    c.ai = rp[1];
+    c.b = rp[2];
+    c.io = rp[3];
+    c.ig = rp[4];
+    c.aG = wrapmul(c.a, c.ig);
+    c.shift = ((wrapmul(c.ai, c.b) % dev.n) + dev.n) % dev.n;
+    c.rank = rank;
+    c.nb = nb;
+    c.count = &S->count;
+    c.err = &S->err;
   }
+  if (threadIdx.x >= 32 && threadIdx.x < 34) {
+    // the reference's products; n is a power of two: times 1 / n equals the quotient
+    const int i = threadIdx.x - 32;
+    c.slope[i] = 2 * kPi * (i ? rp[0] : 1) * rp[4] * dev.inv_n;
+    c.off[i] = (double)(rp[3] + i);
+  }
+  for (int i = threadIdx.x; i < (1 << TRIG_BITS); i += V3_LIST) c.trig[i] = __ldg((const double2 *)dev.trig + i);
+  const int T = V3_LIST * nb, gt = v3_spread(threadIdx.x) * nb + rank;
+  const bool lead = rank == 0 && threadIdx.x == 0;
   cl.sync();
 
   // ---- Mansour estimate; first tones are assigned, their buckets cleared
-  est_mansour(c, &S->found, d.est_cap, &S->err, gt, T, est_x);
-  cl.sync();
-  int F = min(S->found, d.est_cap);
-  for (int i = gt; i < F; i += T) {
-    trace_rec(d, slot, cnt, -2, 0, c.est_f[i], c.est_v[i]);
-    map_add(c, c.est_f[i], c.est_v[i], true, &S->count, d.map_cap, &S->err);
-    const int bk = c.est_f[i] % d.W;
+  estimate(c, 0, mem.x);
+  const int first = mem.x.tones;  // the CTA's
+  if (threadIdx.x == 0 && first) atomicAdd(&S->found, first);
+  cl.barrier_wait();
+  for (int i = threadIdx.x; i < first; i += V3_LIST) {
+    const int bk = tone_key(c, mem.x, i) & (dev.W - 1);
     c.man[2 * bk] = make_double2(0.0, 0.0);
     c.man[2 * bk + 1] = make_double2(0.0, 0.0);
   }
+  // ---- first Gaussian filter: peel the known tones, estimate, peel
+  subtract(c, mem.x, first, 2, 2, false, true, true, -2, 0);
   cl.sync();
-  if (F == d.k) {  // the reference returns before writing its output (:859-860)
+  if (S->found == dev.k) {  // the reference returns before writing its output (:859-860)
     if (lead) {
-      cnt[CNT_OUT] = 0;
-      if (d.out_count) d.out_count[slot] = 0;
-      cnt[CNT_V3] = -1;
+      c.counters[CNT_OUT] = 0;
+      if (dev.out_count) dev.out_count[slot] = 0;
+      c.counters[CNT_V3] = -1;
     }
     cl.sync();     // the first CTA's shared memory outlives every reader
     return;
   }
-
-  // ---- first Gaussian filter: peel the known tones, estimate, peel
-  int M = min(S->count, d.map_cap);
-  for (int w = gt; w < 2 * M; w += T) {  // items (tone, shift)
-    const int h = c.list[w >> 1];
-    update_part(c, c.tkey[h], c.tval[h], 2 + (w & 1), &S->err);
-  }
-  if (lead) S->found = 0;
-  cl.sync();
-  est_gauss(c, c.g1, d.B1, (const double2 *)d.win1, d.win1_half, 1, 0, &S->found, d.est_cap, &S->err, gt, T,
-            est_x);
-  cl.sync();
-  F = min(S->found, d.est_cap);
-  for (int w = gt; w < 4 * F; w += T) {  // items (tone, part 2..5)
-    const int i = w >> 2;
-    if (!(w & 3)) {
-      trace_rec(d, slot, cnt, -1, 1, c.est_f[i], c.est_v[i]);
-      map_add(c, c.est_f[i], c.est_v[i], false, &S->count, d.map_cap, &S->err);
-    }
-    update_part(c, c.est_f[i], c.est_v[i], 2 + (w & 3), &S->err);
-  }
+  estimate(c, 1, mem.x);
+  cl.barrier_wait();
+  subtract(c, mem.x, mem.x.tones, 2, 4, false, true, false, -1, 1);
   cl.sync();
 
   // ---- second (permuted) Gaussian filter: peel every known tone
-  M = min(S->count, d.map_cap);
-  for (int w = gt; w < 2 * M; w += T) {  // items (tone, shift)
-    const int h = c.list[w >> 1];
-    update_part(c, c.tkey[h], c.tval[h], w & 1, &S->err);
-  }
+  subtract(c, mem.x, (min(S->count, dev.map_cap) - rank + nb - 1) / nb, 0, 2, true, false, false, 0, 0);
   cl.sync();
 
   // ---- round robin: G2, then Mansour, G1, G2, ... until the counts of
   //      non-empty buckets repeat after a G2 round (:959-1076)
-  int stage = 2, rounds = 0;
+  int stage = 2, rounds = 0, checks = 0, prev[3] = {0, 0, 0};
   for (;;) {
-    if (lead) S->found = 0;
-    cl.sync();
-    if (stage == 0)
-      est_mansour(c, &S->found, d.est_cap, &S->err, gt, T, est_x);
-    else if (stage == 1)
-      est_gauss(c, c.g1, d.B1, (const double2 *)d.win1, d.win1_half, 1, 0, &S->found, d.est_cap, &S->err, gt, T,
-                est_x);
-    else
-      est_gauss(c, c.g2, d.B2, (const double2 *)d.win2, d.win2_half, c.a, c.b, &S->found, d.est_cap, &S->err,
-                gt, T, est_x);
-    cl.sync();
-    F = min(S->found, d.est_cap);
-    for (int w = gt; w < 6 * F; w += T) {  // items (tone, part)
-      const int i = w / 6, part = w - 6 * i;
-      if (part == 0) {
-        trace_rec(d, slot, cnt, rounds, stage, c.est_f[i], c.est_v[i]);
-        map_add(c, c.est_f[i], c.est_v[i], false, &S->count, d.map_cap, &S->err);
-      }
-      update_part(c, c.est_f[i], c.est_v[i], part, &S->err);
-    }
-    if (stage == 2 && rounds >= 1 && lead) S->cnt[0] = S->cnt[1] = S->cnt[2] = 0;
+    estimate(c, stage, mem.x);
+    cl.barrier_wait();
+    subtract(c, mem.x, mem.x.tones, 0, 6, false, true, false, rounds, stage);
     cl.sync();
     if (stage == 2 && rounds >= 1) {
-      int cm = 0, c1 = 0, c2 = 0;
-      for (int j = gt; j < d.B1; j += T) {
-        const double2 v = c.g1[j];
-        c1 += (v.x * v.x + v.y * v.y > 1e-6);
-      }
-      for (int j = gt; j < d.B2; j += T) {
-        const double2 v = c.g2[j];
-        c2 += (v.x * v.x + v.y * v.y > 1e-6);
-      }
-      const double inv_w = 1. / d.W;  // W is a power of two: the products equal the quotients
-      for (int j = gt; j < d.W; j += T) {
-        const double2 v = c.man[2 * j];
-        const double re = v.x * inv_w, im = v.y * inv_w;
-        cm += (re * re + im * im > 1e-6);
-      }
-      if (cm) atomicAdd(&S->cnt[0], cm);
-      if (c1) atomicAdd(&S->cnt[1], c1);
-      if (c2) atomicAdd(&S->cnt[2], c2);
-      cl.sync();
+      int *cn = S->cnt[checks & 1];
       if (lead) {
-        S->stop = (S->cnt[0] == S->prev[0] && S->cnt[1] == S->prev[1] && S->cnt[2] == S->prev[2]);
-        for (int i = 0; i < 3; i++) S->prev[i] = S->cnt[i];
+        int *other = S->cnt[~checks & 1];
+        other[0] = other[1] = other[2] = 0;
+      }
+      checks++;
+#pragma unroll 1
+      for (int i = 0; i < 3; i++) {  // comb, contiguous, permuted
+        const double2 *s = i == 0 ? c.man : i == 1 ? c.g1 : c.g2;
+        const int B = i == 0 ? dev.W : i == 1 ? dev.B1 : dev.B2, st = i == 0 ? 2 : 1;
+        const double norm2 = i == 0 ? dev.inv_w2 : 1.0;  // W is a power of two: exact scaling
+        int k = 0;
+        for (int j = gt; j < B; j += T) {
+          const double2 v = s[st * j];
+          // |v|^2 > 1e-6 needs a component of at least 7e-4
+          if (reaches(v, (i == 0 ? c.lw : 0) - 11)) k += ((v.x * v.x + v.y * v.y) * norm2 > 1e-6);
+        }
+        if (k) atomicAdd(&cn[i], k);
       }
       cl.sync();
-      if (S->stop) break;
+      bool same = true;
+      for (int i = 0; i < 3; i++) {
+        const int v = cn[i];
+        same = same && v == prev[i];
+        prev[i] = v;
+      }
+      if (same) break;
     }
     rounds++;
-    if (rounds > d.max_passes) {
+    if (rounds > dev.max_passes) {
       if (lead) atomicOr(&S->err, ERR_V3_NOCONVERGE);
       break;
     }
@@ -692,77 +707,111 @@ __global__ void __cluster_dims__(V3_CLUSTER, 1, 1) __launch_bounds__(1024) k_v3_
   cl.sync();
 
   // ---- output: every key of the map with its accumulated value
-  M = min(S->count, d.map_cap);
-  const int outn = min(M, d.out_cap);
+  const int M = min(S->count, dev.map_cap), outn = min(M, dev.out_cap);
   for (int i = gt; i < outn; i += T) {
     const int h = c.list[i];
-    d.out_idx[(long)slot * d.out_stride + i] = c.tkey[h];
-    ((double2 *)d.out_val)[(long)slot * d.out_stride + i] = c.tval[h];
+    dev.out_idx[(long)slot * dev.out_stride + i] = c.tkey[h];
+    ((double2 *)dev.out_val)[(long)slot * dev.out_stride + i] = c.tval[h];
   }
   if (lead) {
-    cnt[CNT_OUT] = outn;
-    if (d.out_count) d.out_count[slot] = outn;
-    cnt[CNT_V3] = rounds;
-    cnt[CNT_ERR] |= S->err | (M > d.out_cap ? ERR_OUT_OVERFLOW : 0);
+    c.counters[CNT_OUT] = outn;
+    if (dev.out_count) dev.out_count[slot] = outn;
+    c.counters[CNT_V3] = rounds;
+    c.counters[CNT_ERR] |= S->err | (M > dev.out_cap ? ERR_OUT_OVERFLOW : 0);
   }
   cl.sync();       // the first CTA's shared memory outlives every reader
 }
 
 // ---------------------------------------------------------------- launch --
 
+// CTAs per cluster of the peel kernel: 16 (beyond the portable 8, so only
+// where the device says that it can hold such clusters) for few signals,
+// whose rounds then have twice the FP64 pipes; 8 once 16 would leave signals
+// waiting for one another.
+static cudaError_t v3_cluster(int nslots, int &nb) {
+  static std::mutex mu;
+  static std::map<int, int> held;  // device -> clusters of 16 at once
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e) return e;
+  std::lock_guard<std::mutex> g(mu);
+  auto it = held.find(dev);
+  if (it == held.end()) {
+    int n = 0;
+    if ((e = set_smem(k_v3_peel, sizeof(PeelMem)))) return e;
+    if (cudaFuncSetAttribute(k_v3_peel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = 16;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3(16);
+      cfg.blockDim = dim3(V3_LIST);
+      cfg.dynamicSmemBytes = sizeof(PeelMem);
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&n, k_v3_peel, &cfg) != cudaSuccess) n = 0;
+    }
+    cudaGetLastError();
+    it = held.emplace(dev, n).first;
+  }
+  nb = nslots <= it->second / 2 ? 16 : 8;
+  return cudaSuccess;
+}
+
+static cudaError_t v3_peel(const V3Dev &d, int nslots, cudaStream_t s) {
+  int nb = 8;
+  cudaError_t e = v3_cluster(nslots, nb);
+  if (e) return e;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = nb;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(nslots * nb);
+  cfg.blockDim = dim3(V3_LIST);
+  cfg.dynamicSmemBytes = sizeof(PeelMem);
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_v3_peel, d);
+}
+
 cudaError_t v3_run(const V3Dev &d, int nslots, cudaStream_t s, StageEvents *se) {
   cudaError_t e;
-  if ((e = cudaMemsetAsync(d.counters, 0, sizeof(int) * CNT_STRIDE * nslots, s))) return e;
-  if ((e = cudaMemsetAsync(d.map_keys, 0xFF, sizeof(int) * (size_t)d.table_cap * nslots, s))) return e;
-  int Nmax = d.B1 > d.B2 ? d.B1 : d.B2;
-  if (!d.large_man && d.W > Nmax) Nmax = d.W;
-  int T = Nmax / 4;
-  if (T > 1024) T = 1024;
-  if (T < 32) T = 32;
-  const int per = (Nmax / 4 + T - 1) / T;
-  const int count2 = (d.w2 / d.B2) * d.B2 + 1, lo2 = v3_phase_lo(count2);
-  const size_t sm = std::max((size_t)Nmax * sizeof(double2), sizeof(double2) * (size_t)(lo2 + (count2 + lo2 - 1) / lo2));
   mark(se, s);
-  int role0 = 0;
-  if (!d.large_man && v3_man_split(d.W)) {
-    const int M = d.W / V3_MAN_SPLIT;
-    const size_t msm = 2 * sizeof(double2) * (size_t)M;
-    if ((e = set_smem(k_v3_man_split, msm))) return e;
-    k_v3_man_split<<<dim3(V3_MAN_SPLIT, 2, nslots), 256, msm, s>>>(d);
-    if ((e = cudaGetLastError())) return e;
-    k_v3_man_combine<<<dim3((M + 127) / 128, 2, nslots), 128, 0, s>>>(d);
-    if ((e = cudaGetLastError())) return e;
-    note_launches(2);
-    role0 = 2;
-  } else if (d.large_man) {
-    const dim3 g((d.W + 255) / 256, 2, nslots);
-    k_v3_man_gather<<<g, 256, 0, s>>>(d);
-    if ((e = cudaGetLastError())) return e;
-    double2 *a = (double2 *)d.man_tmp;
-    if ((e = global_fft_c128(a, a + 2L * d.W, d.W, 2, d.W, 4L * d.W, nslots, d.tw_man, s))) return e;
-    k_v3_man_interleave<<<g, 256, 0, s>>>(d);
-    if ((e = cudaGetLastError())) return e;
-    note_launches(2);
-    role0 = 2;
-  }
-  dim3 grid(6 - role0, nslots);
-  switch (per) {
-    case 1:
-      if ((e = set_smem(k_v3_filters<1>, sm))) return e;
-      k_v3_filters<1><<<grid, T, sm, s>>>(d, role0);
-      break;
-    case 2:
-      if ((e = set_smem(k_v3_filters<2>, sm))) return e;
-      k_v3_filters<2><<<grid, T, sm, s>>>(d, role0);
-      break;
-    default:
-      return cudaErrorInvalidValue;
+  const int Bmax = std::max(d.B1, d.B2), m2 = fft_m2(d.W);
+  V3Shape sh;
+  sh.elems[0] = sh.elems[1] = 4 * V3_T;  // W is at most 2^17: tiles of up to 512 rows
+  if (d.W / m2 > sh.elems[0] || m2 > sh.elems[1]) return cudaErrorInvalidValue;
+  sh.man[0] = fft_ctas(sh.elems[0], d.W / m2, d.W);
+  sh.man[1] = fft_ctas(sh.elems[1], m2, d.W);
+  sh.n1 = (d.B1 + V3_G1 - 1) / V3_G1;
+  sh.n2 = (d.B2 + V3_G2 - 1) / V3_G2;
+  sh.nc = (d.table_cap + V3_CLEAR - 1) / V3_CLEAR;
+  sh.chunks2 = d.w2 / d.B2;
+  const size_t tile = sizeof(double2) * (size_t)sh.elems[0];
+  const size_t sa = std::max(tile, sizeof(double2) * (size_t)sh.chunks2 * (V3_G2 + 1));
+  const size_t sb = std::max(tile, sizeof(double2) * (size_t)Bmax);
+  if ((e = set_smem(k_v3_first, sa))) return e;
+  k_v3_first<<<dim3(2 * sh.man[0] + sh.n1 + sh.n2 + sh.nc, nslots), V3_T, sa, s>>>(d, sh);
+  if ((e = cudaGetLastError())) return e;
+  const dim3 grid(2 * sh.man[1] + 4, nslots);
+  const int T = std::min(1024, std::max(V3_T, Bmax / 4));
+  if (Bmax / 4 <= 1024) {
+    if ((e = set_smem(k_v3_second<1>, sb))) return e;
+    k_v3_second<1><<<grid, T, sb, s>>>(d, sh);
+  } else if (Bmax / 4 <= 2048) {
+    if ((e = set_smem(k_v3_second<2>, sb))) return e;
+    k_v3_second<2><<<grid, T, sb, s>>>(d, sh);
+  } else {
+    return cudaErrorInvalidValue;
   }
   if ((e = cudaGetLastError())) return e;
   mark(se, s);
-  k_v3_peel<<<nslots * V3_CLUSTER, 1024, 0, s>>>(d);
+  if ((e = v3_peel(d, nslots, s))) return e;
   mark(se, s);
-  note_launches(2);
+  note_launches(3);
   return cudaGetLastError();
 }
 
