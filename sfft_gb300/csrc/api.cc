@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -142,6 +143,8 @@ struct PlanImpl {
   int *h_rp = nullptr;
   const void **h_in = nullptr;
   int staged_slots = 0;
+  int *h_cnt = nullptr;  // page-locked copy of the slots' counters
+  int h_cnt_slots = 0;
   // stage timing (sfft_profile): event sets of launches not yet harvested
   bool profiling = false;
   std::vector<sfft::StageEvents *> free_sets;
@@ -153,6 +156,7 @@ struct PlanImpl {
     for (auto *e : pending) destroy(e);
     if (h_rp) cudaFreeHost(h_rp);
     if (h_in) cudaFreeHost((void *)h_in);
+    if (h_cnt) cudaFreeHost(h_cnt);
   }
   static void destroy(sfft::StageEvents *e) {
     for (int i = 0; i < 8; i++) cudaEventDestroy(e->ev[i]);
@@ -670,7 +674,8 @@ void shift_view(PlanImpl &P, sfft::V3Dev &d, int base, bool own_out) {
 }
 
 bool launch(PlanImpl &P, int num, const void *const *in_dev, int in_type, cudaStream_t s,
-            const OutTarget *tgt = nullptr, int base = 0, const unsigned *seeds = nullptr) {
+            const OutTarget *tgt = nullptr, int base = 0, const unsigned *seeds = nullptr,
+            cudaEvent_t input_read = nullptr) {
   std::vector<int> rp((size_t)P.rp_stride * num);
   for (int i = 0; i < num; i++) {
     unsigned ep = 0;
@@ -711,7 +716,7 @@ bool launch(PlanImpl &P, int num, const void *const *in_dev, int in_type, cudaSt
       d.out_count = tgt->count;
       d.out_stride = tgt->stride;
     }
-    ok = cuda_ok(sfft::v12_run(d, num, s, se), "v1/v2 launch");
+    ok = cuda_ok(sfft::v12_run(d, num, s, se, input_read), "v1/v2 launch");
   } else {
     sfft::V3Dev d = v3_view(P);
     shift_view(P, d, base, tgt == nullptr);
@@ -722,7 +727,7 @@ bool launch(PlanImpl &P, int num, const void *const *in_dev, int in_type, cudaSt
       d.out_count = tgt->count;
       d.out_stride = tgt->stride;
     }
-    ok = cuda_ok(sfft::v3_run(d, num, s, se), "v3 launch");
+    ok = cuda_ok(sfft::v3_run(d, num, s, se, input_read), "v3 launch");
   }
   if (se) P.pending.push_back(se);
   return ok;
@@ -766,47 +771,94 @@ std::set<void *> g_pinned;
 
 PlanImpl *impl(sfft_plan *p) { return p ? (PlanImpl *)p->data : nullptr; }
 
-// Runs `num` (<= slots) transforms whose inputs are host or device
-// pointers and writes dense n-point outputs (host or device).
-bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out) {
+// Whether the input and output arrays (nb bytes each) of device pointers
+// overlap anywhere, an in-place transform among them.
+bool in_out_overlap(const std::vector<const void *> &in, const std::vector<void *> &out, size_t nb) {
+  std::vector<std::pair<uintptr_t, int>> v;
+  for (const void *p : in) v.emplace_back((uintptr_t)p, 0);
+  for (void *p : out) v.emplace_back((uintptr_t)p, 1);
+  std::sort(v.begin(), v.end());
+  // the nearest array of the other kind below each array decides
+  uintptr_t last[2] = {0, 0};
+  bool seen[2] = {false, false};
+  for (const auto &e : v) {
+    const int o = 1 - e.second;
+    if (seen[o] && last[o] + nb > e.first) return true;
+    last[e.second] = e.first;
+    seen[e.second] = true;
+  }
+  return false;
+}
+
+// Page-locked room for the counters of `num` slots.
+bool ensure_host_counters(PlanImpl &P, int num) {
+  if (P.h_cnt_slots >= num) return true;
+  if (P.h_cnt) cudaFreeHost(P.h_cnt);
+  P.h_cnt = nullptr;
+  P.h_cnt_slots = 0;
+  if (!cuda_ok(cudaMallocHost((void **)&P.h_cnt, sizeof(int) * sfft::CNT_STRIDE * (size_t)num), "counters")) return false;
+  P.h_cnt_slots = num;
+  return true;
+}
+
+// Runs `num` (<= slots) transforms whose inputs are host or device pointers
+// (in_dev / out_dev: which) and writes dense n-point outputs (host or
+// device).  The outputs are cleared by one kernel on copy_out beside the
+// transform, so that 16 n bytes a signal are written while its kernels wait
+// for FP64 and for each other; where an output overlaps an input, after the
+// transform.  v3 clears from the end of its filters on (its peeling clusters
+// need whole SMs first), v1 / v2 likewise from the end of the fold when the
+// inputs are larger than L2, whose gathers need the memory themselves (one
+// signal of 2^24 points: 161 us, from the start on 168), else at once (64
+// signals of 2^16 points: 472 us, from the end of the fold on 480).
+// One memset per output took 41 us for 2^24 points after a v3 transform of 110
+// us, and 64 calls for 64 outputs of 2^16 points.
+bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out, const char *in_dev, const char *out_dev) {
   cudaStream_t s = P.stream;
   const size_t nb = sizeof(double) * 2 * (size_t)P.n;
   std::vector<const void *> dev_in(num);
+  std::vector<void *> dense(num);
   bool need_in_stage = false, need_out_stage = false;
   for (int i = 0; i < num; i++) {
-    if (!is_device_ptr(in[i])) need_in_stage = true;
-    if (!is_device_ptr(out[i])) need_out_stage = true;
+    need_in_stage |= !in_dev[i];
+    need_out_stage |= !out_dev[i];
   }
   if (need_in_stage && !P.in_stage.ensure(nb * P.slots)) return false;
   if (need_out_stage && !P.dense_stage.ensure(nb * P.slots)) return false;
+  if (!ensure_host_counters(P, num)) return false;
   for (int i = 0; i < num; i++) {
-    if (is_device_ptr(in[i])) {
-      dev_in[i] = in[i];
-    } else {
-      void *dst = (char *)P.in_stage.p + nb * i;
-      if (!cuda_ok(cudaMemcpyAsync(dst, in[i], nb, cudaMemcpyHostToDevice, s), "input copy")) return false;
-      dev_in[i] = dst;
-    }
+    dev_in[i] = in_dev[i] ? (const void *)in[i] : (const void *)((char *)P.in_stage.p + nb * i);
+    dense[i] = out_dev[i] ? (void *)out[i] : (void *)((char *)P.dense_stage.p + nb * i);
+    if (!in_dev[i] &&
+        !cuda_ok(cudaMemcpyAsync((void *)dev_in[i], in[i], nb, cudaMemcpyHostToDevice, s), "input copy"))
+      return false;
   }
-  if (!launch(P, num, dev_in.data(), sfft::IN_C128, s)) return false;
-  std::vector<void *> dense(num);
-  for (int i = 0; i < num; i++) {
-    dense[i] = is_device_ptr(out[i]) ? (void *)out[i] : (char *)P.dense_stage.p + nb * i;
-    if (!cuda_ok(cudaMemsetAsync(dense[i], 0, nb, s), "output clear")) return false;
-  }
-  if (!cuda_ok(cudaMemcpyAsync(P.dense_ptrs.p, dense.data(), sizeof(void *) * num, cudaMemcpyHostToDevice, s),
-               "pointer upload"))
+  const bool beside = !in_out_overlap(dev_in, dense, nb);
+  const bool late = beside && (P.version == 2 || nb * num > (96u << 20));
+  cudaStream_t zs = beside ? P.copy_out : s;
+  if (!launch(P, num, dev_in.data(), sfft::IN_C128, s, nullptr, 0, nullptr, late ? P.ev_comp[0] : nullptr))
+    return false;
+  if (late && !cuda_ok(cudaStreamWaitEvent(zs, P.ev_comp[0], 0), "wait")) return false;
+  if (!cuda_ok(cudaMemcpyAsync(P.dense_ptrs.p, dense.data(), sizeof(void *) * num, cudaMemcpyHostToDevice, zs),
+               "pointer upload") ||
+      !cuda_ok(sfft::clear_dense((void *const *)P.dense_ptrs.p, P.n, num, zs), "output clear"))
+    return false;
+  if (beside && (!cuda_ok(cudaEventRecord(P.ev_out[0], zs), "event") ||
+                 !cuda_ok(cudaStreamWaitEvent(s, P.ev_out[0], 0), "wait")))
     return false;
   if (!cuda_ok(sfft::scatter_dense(P.out_idx.as<int>(), P.out_val.p, P.version < 2 ? P.prec : sfft::PREC_FP64,
                                    P.counters.as<int>(), P.out_cap, (void *const *)P.dense_ptrs.p, num, s),
                "scatter"))
     return false;
   for (int i = 0; i < num; i++)
-    if (!is_device_ptr(out[i]) &&
-        !cuda_ok(cudaMemcpyAsync(out[i], dense[i], nb, cudaMemcpyDeviceToHost, s), "output copy"))
+    if (!out_dev[i] && !cuda_ok(cudaMemcpyAsync(out[i], dense[i], nb, cudaMemcpyDeviceToHost, s), "output copy"))
       return false;
-  if (!cuda_ok(cudaStreamSynchronize(s), "exec")) return false;
-  return check_device_errors(P, num);
+  if (!cuda_ok(cudaMemcpyAsync(P.h_cnt, P.counters.p, sizeof(int) * sfft::CNT_STRIDE * (size_t)num,
+                               cudaMemcpyDeviceToHost, s),
+               "counters") ||
+      !cuda_ok(cudaStreamSynchronize(s), "exec"))
+    return false;
+  return check_counts(P.h_cnt, num);
 }
 
 // sfft_exec_many on host buffers: chunk c's input copies (copy_in), its
@@ -1251,7 +1303,10 @@ static sfft_plan *make_plan_impl(int n, int k, enum sfft_version version, const 
         !upload_twiddles(P->tw_c, p.W_Man, sfft::PREC_FP64) || !upload_trig(P->trig))
       return nullptr;
   }
-  if (!cuda_ok(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking), "stream")) return nullptr;
+  // above the copy streams, on which outputs are cleared beside the transform
+  int least = 0, greatest = 0;
+  cudaDeviceGetStreamPriorityRange(&least, &greatest);
+  if (!cuda_ok(cudaStreamCreateWithPriority(&P->stream, cudaStreamNonBlocking, greatest), "stream")) return nullptr;
   if (!cuda_ok(cudaEventCreateWithFlags(&P->done, cudaEventDisableTiming), "event")) return nullptr;
   if (!cuda_ok(cudaStreamCreateWithFlags(&P->copy_in, cudaStreamNonBlocking), "stream") ||
       !cuda_ok(cudaStreamCreateWithFlags(&P->copy_out, cudaStreamNonBlocking), "stream"))
@@ -1363,9 +1418,13 @@ void sfft_exec_many(sfft_plan *plan, int num, complex_t **in, complex_t **out) {
   cudaSetDevice(P->device);
   g_err.clear();
   const int chunk = std::max(1, std::min(P->max_batch, num));
+  std::vector<char> in_dev(num), out_dev(num);
   bool all_host = num > 1;
-  for (int i = 0; i < num && all_host; i++)
-    if (is_device_ptr(in[i]) || is_device_ptr(out[i])) all_host = false;
+  for (int i = 0; i < num; i++) {
+    in_dev[i] = is_device_ptr(in[i]);
+    out_dev[i] = is_device_ptr(out[i]);
+    if (in_dev[i] || out_dev[i]) all_host = false;
+  }
   if (all_host) {  // about 32 chunks: copies overlap the transforms with little fill and drain
     exec_dense_pipelined(*P, num, in, out, std::max(1, std::min(chunk, (num + 31) / 32)));
     return;
@@ -1373,7 +1432,7 @@ void sfft_exec_many(sfft_plan *plan, int num, complex_t **in, complex_t **out) {
   if (!ensure_slots(*P, chunk)) return;
   for (int i = 0; i < num; i += chunk) {
     const int m = std::min(chunk, num - i);
-    if (!exec_dense_chunk(*P, m, in + i, out + i)) return;
+    if (!exec_dense_chunk(*P, m, in + i, out + i, &in_dev[i], &out_dev[i])) return;
   }
 }
 

@@ -78,12 +78,16 @@ struct V12Dev {
 };
 
 // Launches the whole v1/v2 pipeline for `nslots` signals on `stream`.
-cudaError_t v12_run(const V12Dev &d, int nslots, cudaStream_t stream, StageEvents *se = nullptr);
-// Scatters the sparse result of each slot into dense n-point complex128
-// outputs (device array of per-slot pointers, already zeroed).
+// input_read (optional) is recorded once no later kernel reads the inputs.
+cudaError_t v12_run(const V12Dev &d, int nslots, cudaStream_t stream, StageEvents *se = nullptr,
+                    cudaEvent_t input_read = nullptr);
+// Zeroes `nslots` dense outputs of n complex128 values.
+cudaError_t clear_dense(void *const *dense, int n, int nslots, cudaStream_t stream);
 // Device-to-device copy of `count` ints by a kernel (stream-ordered, no copy
 // engine involved).
 cudaError_t copy_ints(const int *src, int *dst, int count, cudaStream_t s);
+// Scatters the sparse result of each slot into dense n-point complex128
+// outputs (device array of per-slot pointers, already zeroed).
 cudaError_t scatter_dense(const int *out_idx, const void *out_val, int prec, const int *counters,
                           int out_cap, void *const *dense, int nslots, cudaStream_t stream);
 
@@ -175,7 +179,9 @@ struct V3Dev {
   int in_type;
 };
 
-cudaError_t v3_run(const V3Dev &d, int nslots, cudaStream_t stream, StageEvents *se = nullptr);
+// input_read (optional) is recorded once no later kernel reads the inputs.
+cudaError_t v3_run(const V3Dev &d, int nslots, cudaStream_t stream, StageEvents *se = nullptr,
+                   cudaEvent_t input_read = nullptr);
 // Largest Gaussian bucket FFT of the v3 filter kernels (one CTA).
 int v3_max_smem_fft();
 // Batched complex128 FFTs of length N in global memory (the same stages as

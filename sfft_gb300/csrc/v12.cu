@@ -1588,6 +1588,17 @@ __global__ void __launch_bounds__(EC_THREADS, 3) k_estimate_comb64(V12Dev d) {
 
 // ---------------------------------------------------------------- scatter --
 
+// 16 stores of 16 bytes per thread: 64 KB a block.
+constexpr int CLEAR_PER = 16;
+
+__global__ void __launch_bounds__(256) k_clear_dense(void *const *dense, int n) {
+  double2 *o = (double2 *)dense[blockIdx.y];
+  const long i0 = (long)blockIdx.x * (256 * CLEAR_PER) + threadIdx.x;
+#pragma unroll
+  for (int u = 0; u < CLEAR_PER; u++)
+    if (i0 + 256 * u < n) __stcs(o + i0 + 256 * u, make_double2(0.0, 0.0));  // L2 stays the transform's
+}
+
 template <typename R>
 __global__ void k_scatter_dense(const int *out_idx, const c2_t<R> *out_val, const int *counters,
                                 int out_cap, void *const *dense) {
@@ -1784,7 +1795,7 @@ static cudaError_t launch_estimate(const V12Dev &d, int nslots, cudaStream_t s) 
 }
 
 template <typename R, typename In>
-static cudaError_t run_typed(const V12Dev &d, int nslots, cudaStream_t s, StageEvents *se) {
+static cudaError_t run_typed(const V12Dev &d, int nslots, cudaStream_t s, StageEvents *se, cudaEvent_t input_read) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(d.counters, 0, sizeof(int) * CNT_STRIDE * nslots, s))) return e;
   mark(se, s);
@@ -1802,6 +1813,7 @@ static cudaError_t run_typed(const V12Dev &d, int nslots, cudaStream_t s, StageE
   }
   if ((e = cudaGetLastError())) return e;
   mark(se, s);
+  if (input_read && (e = cudaEventRecord(input_read, s))) return e;
   if ((e = launch_bucket<R>(d, nslots, s))) return e;
   {
     const size_t sm = vote_smem(d);
@@ -2148,12 +2160,12 @@ cudaError_t global_fft_c128(void *a, void *b, int N, int narr, long arr_stride, 
                             s);
 }
 
-cudaError_t v12_run(const V12Dev &d, int nslots, cudaStream_t s, StageEvents *se) {
+cudaError_t v12_run(const V12Dev &d, int nslots, cudaStream_t s, StageEvents *se, cudaEvent_t input_read) {
   if (d.prec == PREC_FP64)
-    return d.in_type == IN_C128 ? run_typed<double, double2>(d, nslots, s, se)
-                                : run_typed<double, float2>(d, nslots, s, se);
-  return d.in_type == IN_C128 ? run_typed<float, double2>(d, nslots, s, se)
-                              : run_typed<float, float2>(d, nslots, s, se);
+    return d.in_type == IN_C128 ? run_typed<double, double2>(d, nslots, s, se, input_read)
+                                : run_typed<double, float2>(d, nslots, s, se, input_read);
+  return d.in_type == IN_C128 ? run_typed<float, double2>(d, nslots, s, se, input_read)
+                              : run_typed<float, float2>(d, nslots, s, se, input_read);
 }
 
 __global__ void k_copy_ints(const int *src, int *dst, int count) {
@@ -2164,6 +2176,12 @@ __global__ void k_copy_ints(const int *src, int *dst, int count) {
 cudaError_t copy_ints(const int *src, int *dst, int count, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   k_copy_ints<<<(count + 255) / 256, 256, 0, s>>>(src, dst, count);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t clear_dense(void *const *dense, int n, int nslots, cudaStream_t s) {
+  k_clear_dense<<<dim3((unsigned)((n + 256L * CLEAR_PER - 1) / (256L * CLEAR_PER)), nslots), 256, 0, s>>>(dense, n);
   note_launches(1);
   return cudaGetLastError();
 }

@@ -777,7 +777,7 @@ static cudaError_t v3_peel(const V3Dev &d, int nslots, cudaStream_t s) {
   return cudaLaunchKernelEx(&cfg, k_v3_peel, d);
 }
 
-cudaError_t v3_run(const V3Dev &d, int nslots, cudaStream_t s, StageEvents *se) {
+cudaError_t v3_run(const V3Dev &d, int nslots, cudaStream_t s, StageEvents *se, cudaEvent_t input_read) {
   cudaError_t e;
   mark(se, s);
   const int Bmax = std::max(d.B1, d.B2), m2 = fft_m2(d.W);
@@ -809,6 +809,7 @@ cudaError_t v3_run(const V3Dev &d, int nslots, cudaStream_t s, StageEvents *se) 
   }
   if ((e = cudaGetLastError())) return e;
   mark(se, s);
+  if (input_read && (e = cudaEventRecord(input_read, s))) return e;
   if ((e = v3_peel(d, nslots, s))) return e;
   mark(se, s);
   note_launches(3);
