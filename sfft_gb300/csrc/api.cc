@@ -1264,7 +1264,7 @@ static sfft_plan *make_plan_impl(int n, int k, enum sfft_version version, const 
     P->large_b = (p.B_loc > mx || p.B_est > mx);
     P->large_c = (P->version == 1 && p.W_Comb > mx);
     P->many_b = P->large_b || sfft::v12_many_ctas(P->prec, std::max(p.B_loc, p.B_est));
-    P->many_c = P->large_c || (P->version == 1 && sfft::v12_many_ctas(P->prec, p.W_Comb));
+    P->many_c = P->large_c || (P->version == 1 && sfft::v12_many_ctas_comb(P->prec, p.W_Comb));
     if (p.B_loc > (1 << 20) || p.B_est > (1 << 20) || p.W_Comb > (1 << 22)) {
       set_err("bucket or comb FFT longer than 2^20 points");
       return nullptr;

@@ -93,14 +93,19 @@ cudaError_t scatter_dense(const int *out_idx, const void *out_val, int prec, con
 
 // Maximum bucket-FFT length held in one CTA's shared memory.
 int v12_max_fft(int prec);
-// Whether FFTs of N points run over many CTAs: every one beyond a CTA's
-// shared memory, and FP64 ones from 1024 points on (see fft.cuh).  Below, a
-// one-CTA FP64 FFT already gives each sub-partition at most one warp of
+// Whether bucket FFTs of N points run over many CTAs: every one beyond a
+// CTA's shared memory, and FP64 ones from 1024 points on (see fft.cuh).  Below,
+// a one-CTA FP64 FFT already gives each sub-partition at most one warp of
 // butterflies, so more CTAs would only add launches.  Measured in FP64,
 // 4096-point buckets of 8 signals (160 FFTs) with their voting: 168 us in one
 // CTA each, 106 us over many; 16384-point combs: 174 us stage by stage
 // through global memory, 50 us.
 inline bool v12_many_ctas(int prec, int N) { return N > v12_max_fft(prec) || (prec == PREC_FP64 && N >= 1024); }
+// The same for comb FFTs, a few per signal, which would leave most SMs idle in
+// one CTA each: FP32 ones from 1024 points on too (one signal's six combs of
+// 8192 points 29 us in one CTA each, 22 us over many; 13 signals' 26 combs of
+// 16384 points 43 and 35 us; 32 combs of 2048 points 20 and 17 us).
+inline bool v12_many_ctas_comb(int prec, int W) { return v12_many_ctas(prec, W) || W >= 1024; }
 
 // ------------------------------------------- persistent uneven executor --
 // One persistent kernel runs the whole v2 pipeline of several FP32 plans

@@ -291,12 +291,15 @@ __host__ __device__ __forceinline__ int fft_ctas(int elems, int M, int N) { retu
 //
 // A histogram over the range the keys span (not over fixed digits: powers of
 // one signal share their leading bits) leaves few keys in the cutoff's bin,
-// which are listed and ranked against each other, so the keys are read about
-// four times whatever their width; a fuller bin is split again.  Together
-// with the FFT shapes above, against one histogram per 8 bits and radix-4
-// stages: the bucket and vote stage of 32 FP32 signals (640 FFTs of 4096
-// points) 120 -> 78 us, one FP32 comb of 16384 points 91 -> 45 us, the bucket
-// stage of one FP64 signal of 2^24 points 212 -> 60 us.
+// which are listed and ranked against each other; a fuller bin is split
+// again.  Each thread keeps the leading 32 bits of its keys in registers (S of
+// them; S = 0: too many keys, read again from where they are) and goes back
+// for a whole 64-bit key only where those decide nothing.  Against one
+// histogram per 8 bits over keys in shared memory (and together with the FFT
+// shapes above): the bucket and vote stage of 32 FP32 signals (640 FFTs of 4096
+// points) 120 -> 78 us, the bucket stage of one FP64 signal of 2^24 points 212
+// -> 60 us.  Registers instead of shared memory: 160 lists of 4096 64-bit keys
+// 12.8 -> 9.2 us, three of 16384 20.7 -> 13.9 us.
 constexpr int SEL_BINS = 1024, SEL_CAP = 256;
 
 template <typename K>
@@ -307,115 +310,200 @@ struct SelShared {
   int a[32], b[32], bin, rem, cnt, n;
 };
 
-// keyat(i): the key of entry i.  out[0..num) (optional) receives the indices; bits
-// (optional) receives one bit per entry, ceil(N / 32) words.  Every thread
-// calls; blockDim.x is a multiple of 32, at most 1024.  Ends with a barrier.
-template <typename K, typename KeyAt>
+// The histogram's bin that holds rank `rem` (cum <= rem < cum + count) into
+// s.bin, s.rem (rank within it) and s.cnt.  Ends with a barrier.
+template <typename K>
+__device__ __forceinline__ void select_bin(SelShared<K> &s, int bins, int rem) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int T = blockDim.x, t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const int per = T >= bins ? 1 : bins / T;
+  int sum = 0;
+  if (t * per < bins)
+    for (int q = 0; q < per; q++) sum += s.hist[t * per + q];
+  int inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(FULL, inc, o);
+    if (lane >= o) inc += x;
+  }
+  if (lane == 31) s.a[wid] = inc;
+  __syncthreads();
+  int cum = __reduce_add_sync(FULL, lane < wid ? s.a[lane] : 0) + inc - sum;
+  if (rem >= cum && rem < cum + sum)
+    for (int q = 0; q < per; q++) {
+      const int c = s.hist[t * per + q];
+      if (rem >= cum && rem < cum + c) {
+        s.bin = t * per + q;
+        s.rem = rem - cum;
+        s.cnt = c;
+      }
+      cum += c;
+    }
+  __syncthreads();
+}
+
+// keyat(i): the key of entry i.  out[0..num) (optional) receives the indices;
+// bits (optional) one bit per entry, ceil(N / 32) words.  Every thread calls;
+// blockDim.x is a multiple of 32, at most 1024; S = 0 or ceil(N / 32) groups
+// of 32 entries are at most S per warp.  Ends with a barrier.
+template <typename K, int S, typename KeyAt>
 __device__ __forceinline__ void block_select(KeyAt keyat, int N, int num, int *__restrict__ out,
                                              unsigned *__restrict__ bits, SelShared<K> &s) {
-  constexpr int BITS = sizeof(K) * 8;
-  const int T = blockDim.x, t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = T >> 5;
+  constexpr bool WIDE = sizeof(K) == 8;
+  constexpr unsigned FULL = 0xffffffffu;
+  const int t = threadIdx.x, T = blockDim.x, lane = t & 31, wid = t >> 5, nw = T >> 5;
   // about two keys per bin, so that short lists do not pay for 1024 bins
   const int lbins = min(10, max(5, floor_log2(N) - 1)), bins = 1 << lbins;
-  constexpr unsigned FULL = 0xffffffffu;
-  unsigned lo32 = FULL, hi32 = 0;
-#pragma unroll 4
-  for (int i = t; i < N; i += T) {
-    const unsigned h = (unsigned)(keyat(i) >> (BITS - 32));
-    lo32 = min(lo32, h);
-    hi32 = max(hi32, h);
+  // each warp owns consecutive groups of 32 entries
+  const int groups = (N + 31) >> 5, per = (groups + nw - 1) / nw, g0 = min(groups, wid * per);
+  const int mine = min(per, groups - g0), SN = S ? S : mine;
+  auto at = [&](int g) { return ((g0 + g) << 5) + lane; };
+  auto top = [&](int i) -> unsigned {
+    if constexpr (WIDE)
+      return (unsigned)(keyat(i) >> 32);
+    else
+      return keyat(i);
+  };
+  unsigned H[S ? S : 1];
+  unsigned lo = FULL, hi = 0;
+#pragma unroll
+  for (int g = 0; g < (S ? S : 0); g++) {
+    const bool in = g < mine && at(g) < N;
+    H[g] = in ? top(at(g)) : 0u;
+    lo = min(lo, in ? H[g] : FULL);
+    hi = max(hi, H[g]);
   }
-  lo32 = __reduce_min_sync(FULL, lo32);
-  hi32 = __reduce_max_sync(FULL, hi32);
+  auto lead = [&](int g) -> unsigned {
+    if constexpr (S != 0)
+      return H[g];
+    else
+      return at(g) < N ? top(at(g)) : 0u;
+  };
+  if constexpr (S == 0) {
+#pragma unroll 4
+    for (int g = 0; g < mine; g++)
+      if (at(g) < N) {
+        const unsigned h = top(at(g));
+        lo = min(lo, h);
+        hi = max(hi, h);
+      }
+  }
+  lo = __reduce_min_sync(FULL, lo);
+  hi = __reduce_max_sync(FULL, hi);
   if (lane == 0) {
-    s.lo[wid] = lo32;
-    s.hi[wid] = hi32;
+    s.lo[wid] = lo;
+    s.hi[wid] = hi;
   }
   for (int i = t; i < bins; i += T) s.hist[i] = 0;
   if (t == 0) s.n = 0;
   __syncthreads();
-  lo32 = __reduce_min_sync(FULL, lane < nw ? s.lo[lane] : FULL);
-  hi32 = __reduce_max_sync(FULL, lane < nw ? s.hi[lane] : 0u);
-  K lo = (K)lo32 << (BITS - 32);  // the cutoff lies in [lo, lo + 2^w)
-  int w = BITS - __clz(hi32 - lo32);
-  int rem = N - num - 1;  // its rank among the keys there
-  K cut;
+  lo = __reduce_min_sync(FULL, lane < nw ? s.lo[lane] : FULL);
+  hi = __reduce_max_sync(FULL, lane < nw ? s.hi[lane] : 0u);
+  int w = 32 - __clz(hi - lo);  // the cutoff's leading bits lie in [lo, lo + 2^w)
+  int rem = N - num - 1;        // its rank among the keys there
+  bool listed = false;
   for (;;) {
     const int sh = max(0, w - lbins);
-#pragma unroll 4
-    for (int i = t; i < N; i += T) {
-      const K d = keyat(i) - lo;  // keys below lo wrap to the top
-      if (w >= BITS || (d >> (w & (BITS - 1))) == 0) atomicAdd(&s.hist[(int)(d >> sh)], 1);
-    }
-    __syncthreads();
-    // the bin with cum <= rem < cum + count
-    const int per = T >= bins ? 1 : bins / T;
-    int sum = 0;
-    if (t * per < bins)
-      for (int q = 0; q < per; q++) sum += s.hist[t * per + q];
-    int inc = sum;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int x = __shfl_up_sync(FULL, inc, o);
-      if (lane >= o) inc += x;
+    for (int g = 0; g < SN; g++) {
+      const unsigned d = lead(g) - lo;  // keys below lo wrap to the top
+      if (g < mine && at(g) < N && (w >= 32 || (d >> (w & 31)) == 0)) atomicAdd(&s.hist[d >> sh], 1);
     }
-    if (lane == 31) s.a[wid] = inc;
     __syncthreads();
-    int wb = lane < wid ? s.a[lane] : 0;
-    wb = __reduce_add_sync(FULL, wb);
-    int cum = wb + inc - sum;
-    if (rem >= cum && rem < cum + sum)
-      for (int q = 0; q < per; q++) {
-        const int c = s.hist[t * per + q];
-        if (rem >= cum && rem < cum + c) {
-          s.bin = t * per + q;
-          s.rem = rem - cum;
-          s.cnt = c;
-        }
-        cum += c;
-      }
-    __syncthreads();
-    lo += (K)s.bin << sh;
-    rem = s.rem;
+    select_bin(s, bins, rem);
+    lo += (unsigned)s.bin << sh;
     w = sh;
-    const int cnt = s.cnt;
-    if (w == 0) {
-      cut = lo;
-      break;
-    }
-    if (cnt <= SEL_CAP) {
-#pragma unroll 4
-      for (int i = t; i < N; i += T) {
-        const K k = keyat(i);
-        if (((k - lo) >> w) == 0) s.list[atomicAdd(&s.n, 1)] = k;
-      }
-      __syncthreads();
-      for (int e = t; e < cnt; e += T) {
-        const K k = s.list[e];
-        int r = 0;
-        for (int u = 0; u < cnt; u++) {
-          const K x = s.list[u];
-          r += x < k || (x == k && u < e);
-        }
-        if (r == rem) s.cut = k;
-      }
-      __syncthreads();
-      cut = s.cut;
-      break;
-    }
+    rem = s.rem;
+    listed = s.cnt <= SEL_CAP && (WIDE || w > 0);
+    if (listed || w == 0) break;
     for (int i = t; i < bins; i += T) s.hist[i] = 0;
     __syncthreads();
   }
-  // ordered compaction: each warp owns consecutive groups of 32 entries
-  const int groups = (N + 31) >> 5, per = (groups + nw - 1) / nw;
-  const int g0 = min(groups, wid * per), g1 = min(groups, g0 + per);
+  K cut = (K)lo;
+  if constexpr (WIDE) {
+    // more than SEL_CAP keys share the leading bits: the same on the others
+    unsigned lo2 = 0;
+    int w2 = 32;
+    while (!listed && w2 > 0) {
+      for (int i = t; i < bins; i += T) s.hist[i] = 0;
+      __syncthreads();
+      const int sh = max(0, w2 - lbins);
+#pragma unroll
+      for (int g = 0; g < SN; g++)
+        if (g < mine && at(g) < N && lead(g) == lo) {
+          const unsigned d = (unsigned)keyat(at(g)) - lo2;
+          if (w2 >= 32 || (d >> (w2 & 31)) == 0) atomicAdd(&s.hist[d >> sh], 1);
+        }
+      __syncthreads();
+      select_bin(s, bins, rem);
+      lo2 += (unsigned)s.bin << sh;
+      w2 = sh;
+      rem = s.rem;
+      if (s.cnt <= SEL_CAP && w2 > 0) break;
+    }
+    cut = ((K)lo << 32) | lo2;
+    if (!listed && w2 > 0) {  // list the keys of [cut, cut + 2^w2)
+#pragma unroll
+      for (int g = 0; g < SN; g++)
+        if (g < mine && at(g) < N && lead(g) == lo) {
+          const K k = keyat(at(g));
+          if (((k - cut) >> w2) == 0) s.list[atomicAdd(&s.n, 1)] = k;
+        }
+      listed = true;
+      w = -1;
+    }
+  }
+  if (listed) {
+    if (w >= 0) {
+#pragma unroll
+      for (int g = 0; g < SN; g++)
+        if (g < mine && at(g) < N && ((lead(g) - lo) >> w) == 0) {
+          const int p = atomicAdd(&s.n, 1);
+          if constexpr (WIDE)
+            s.list[p] = keyat(at(g));
+          else
+            s.list[p] = lead(g);
+        }
+    }
+    __syncthreads();
+    const int cnt = s.cnt;
+    for (int e = t; e < cnt; e += T) {
+      const K k = s.list[e];
+      int r = 0;
+      for (int u = 0; u < cnt; u++) {
+        const K x = s.list[u];
+        r += x < k || (x == k && u < e);
+      }
+      if (r == rem) s.cut = k;
+    }
+    __syncthreads();
+    cut = s.cut;
+  }
+  // ordered compaction
+  auto place = [&](int g, bool &gt, bool &eq) {
+    const bool in = g < mine && at(g) < N;
+    const unsigned h = lead(g);
+    if constexpr (WIDE) {
+      const unsigned c = (unsigned)(cut >> 32);
+      gt = in && h > c;
+      eq = false;
+      if (in && h == c) {
+        const unsigned l = (unsigned)keyat(at(g));
+        gt = l > (unsigned)cut;
+        eq = l == (unsigned)cut;
+      }
+    } else {
+      gt = in && h > cut;
+      eq = in && h == cut;
+    }
+  };
   int ngt = 0, neq = 0;
-#pragma unroll 4
-  for (int g = g0; g < g1; g++) {
-    const int i = g * 32 + lane;
-    const K k = i < N ? keyat(i) : 0;
-    ngt += __popc(__ballot_sync(FULL, i < N && k > cut));
-    neq += __popc(__ballot_sync(FULL, i < N && k == cut));
+#pragma unroll
+  for (int g = 0; g < SN; g++) {
+    bool gt, eq;
+    place(g, gt, eq);
+    ngt += __popc(__ballot_sync(FULL, gt));
+    neq += __popc(__ballot_sync(FULL, eq));
   }
   if (lane == 0) {
     s.a[wid] = ngt;
@@ -426,17 +514,18 @@ __device__ __forceinline__ void block_select(KeyAt keyat, int N, int num, int *_
   const int need = max(0, num - __reduce_add_sync(FULL, ca));  // entries equal to the cutoff to take
   int bgt = __reduce_add_sync(FULL, lane < wid ? ca : 0), beq = __reduce_add_sync(FULL, lane < wid ? cb : 0);
   const unsigned below = (1u << lane) - 1u;
-  for (int g = g0; g < g1; g++) {
-    const int i = g * 32 + lane;
-    const K k = i < N ? keyat(i) : 0;
-    const unsigned mg = __ballot_sync(FULL, i < N && k > cut), me = __ballot_sync(FULL, i < N && k == cut);
+#pragma unroll
+  for (int g = 0; g < SN; g++) {
+    bool gt, eq;
+    place(g, gt, eq);
+    const unsigned mg = __ballot_sync(FULL, gt), me = __ballot_sync(FULL, eq);
     const int pe = beq + __popc(me & below);
-    const bool take = ((mg >> lane) & 1u) || (((me >> lane) & 1u) && pe < need);
     const int pos = bgt + __popc(mg & below) + min(pe, need);
-    if (out && take && pos < num) out[pos] = i;
+    const bool take = (gt || (eq && pe < need)) && pos < num;
+    if (out && take) out[pos] = at(g);
     if (bits) {
-      const unsigned m = __ballot_sync(FULL, take && pos < num);
-      if (lane == 0) bits[g] = m;
+      const unsigned m = __ballot_sync(FULL, take);
+      if (lane == 0 && g < mine) bits[g0 + g] = m;
     }
     bgt += __popc(mg);
     beq += __popc(me);

@@ -268,7 +268,7 @@ long estimate_bytes(const PlanKey &key, int slots, int tune) {
     const long out = std::min(W, f[4] * num) * (key.n / std::max(W, 1L)) + 8L * num * key.n / f[0];
     // FFTs over many CTAs keep a second array and the selection keys
     const long xtra = sfft::v12_many_ctas(key.prec, (int)std::max(f[0], f[2])) ? xs * (cs + cs / 2) : 0;
-    const long ctra = key.version == 1 && sfft::v12_many_ctas(key.prec, (int)W) ? f[4] * W * (cs + cs / 2) : 0;
+    const long ctra = key.version == 1 && sfft::v12_many_ctas_comb(key.prec, (int)W) ? f[4] * W * (cs + cs / 2) : 0;
     const long per = xs * (cs + 8) + xtra + ctra + 4L * key.n + L * num * 4 + W * (4 + f[4] / 8 + 1) + out * (cs + 4) + 4096;
     const long cst = (f[8] + f[9]) * cs + 2L * key.n / f[0] * 32 + (f[0] + f[2] + W) * cs;
     return cst + per * slots;

@@ -212,11 +212,11 @@ struct OneCta<double> {
 
 // Residues of one comb sampling: one bit plane per sampling (plain stores,
 // nothing to clear); a single sampling's residues are the list itself.
-template <typename K, typename KeyAt>
+template <typename K, int S, typename KeyAt>
 __device__ __forceinline__ void comb_select(const V12Dev &d, int c, int slot, KeyAt keyat, SelShared<K> &ss) {
   const int W = d.W, words = (W + 31) >> 5;
   const bool one = d.comb_loops == 1;
-  block_select<K>(keyat, W, d.num, one ? d.comb_list + (long)slot * W : nullptr,
+  block_select<K, S>(keyat, W, d.num, one ? d.comb_list + (long)slot * W : nullptr,
                   d.comb_bits + ((long)slot * d.comb_loops + c) * words, ss);
   if (one && threadIdx.x == 0) d.counters[slot * CNT_STRIDE + CNT_COMB] = d.num;
 }
@@ -275,7 +275,7 @@ __device__ __forceinline__ void comb_block(const V12Dev &d, int c, int slot, uns
   const long sigma = d.n / W;
   const In *x = (const In *)d.inputs[slot] + rp[2 * d.L + c];
   f.template fft<PER>(W, (const c2_t<R> *)d.tw_comb, [=](int i) { return cvt_in<R>(__ldg(x + i * sigma)); });
-  comb_select<key_t<R>>(d, c, slot, [&](int i) { return f.key(i); }, ss);
+  comb_select<key_t<R>, 16>(d, c, slot, [&](int i) { return f.key(i); }, ss);
 }
 
 template <typename R, int PER, typename In>
@@ -561,7 +561,7 @@ __device__ __forceinline__ void bucket_block(const V12Dev &d, int j, int slot, u
     xs[p] = v;
     if (xs32) xs32[p] = make_float2((float)v.x, (float)v.y);
   }
-  block_select<key_t<R>>([&](int i) { return f.key(i); }, B, d.num, d.J + ((long)slot * d.L + j) * d.num,
+  block_select<key_t<R>, 16>([&](int i) { return f.key(i); }, B, d.num, d.J + ((long)slot * d.L + j) * d.num,
                          sel_plane(d, slot, j), ss);
 }
 
@@ -619,27 +619,16 @@ __global__ void __launch_bounds__(1024) k_bucket_b(V12Dev d, int elems, int nloc
               });
 }
 
-// Selection of loop j from its keys (in shared memory up to SEL_KEYS bytes).
-constexpr int SEL_KEYS = 128 * 1024;
-
-template <typename R>
+// Selection of loop j from its keys: S of them per thread (S = 0: any number).
+template <typename R, int S>
 __global__ void __launch_bounds__(1024) k_bucket_select(V12Dev d) {
-  extern __shared__ __align__(16) unsigned char smem[];
   using K = key_t<R>;
   __shared__ SelShared<K> ss;
   const int j = blockIdx.x, slot = blockIdx.y;
   const LoopSpan l = loop_span(d, j);
   const K *pw = (const K *)d.pw + (long)slot * d.xs_size + l.off;
-  int *J = d.J + ((long)slot * d.L + j) * d.num;
-  if (l.B * sizeof(K) <= SEL_KEYS) {
-    K *keys = (K *)smem;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < l.B; i += blockDim.x) keys[i] = pw[i];
-    __syncthreads();
-    block_select<K>([=](int i) { return keys[i]; }, l.B, d.num, J, sel_plane(d, slot, j), ss);
-  } else {
-    block_select<K>([=](int i) { return pw[i]; }, l.B, d.num, J, sel_plane(d, slot, j), ss);
-  }
+  block_select<K, S>([=](int i) { return pw[i]; }, l.B, d.num, d.J + ((long)slot * d.L + j) * d.num,
+                     sel_plane(d, slot, j), ss);
 }
 
 template <typename R, typename In>
@@ -666,22 +655,13 @@ __global__ void __launch_bounds__(1024) k_comb_b(V12Dev d, int elems) {
               [=](int i) { return src[i]; }, [=](int i, c2_t<R> v) { pw[i] = pkey(cabs2<R>(v)); });
 }
 
-template <typename R>
+template <typename R, int S>
 __global__ void __launch_bounds__(1024) k_comb_select(V12Dev d) {
-  extern __shared__ __align__(16) unsigned char smem[];
   using K = key_t<R>;
   __shared__ SelShared<K> ss;
   const int c = blockIdx.x, slot = blockIdx.y, W = d.W;
   const K *pw = (const K *)d.comb_pw + ((long)slot * d.comb_loops + c) * W;
-  if (W * sizeof(K) <= SEL_KEYS) {
-    K *keys = (K *)smem;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < W; i += blockDim.x) keys[i] = pw[i];
-    __syncthreads();
-    comb_select<K>(d, c, slot, [=](int i) { return keys[i]; }, ss);
-  } else {
-    comb_select<K>(d, c, slot, [=](int i) { return pw[i]; }, ss);
-  }
+  comb_select<K, S>(d, c, slot, [=](int i) { return pw[i]; }, ss);
   comb_last_list(d, slot);
 }
 
@@ -1618,7 +1598,7 @@ int v12_max_fft(int prec) { return prec == PREC_FP64 ? 8192 : 16384; }
 // Butterflies per thread and radix-4 stage of an FP64 one-CTA FFT.
 static int one_cta_per(int N) { return std::max(1, N / 4 / 1024); }
 
-// Threads of a selection over N keys: about eight per thread.
+// Threads of a selection over N keys: eight per thread, more beyond 8192 keys.
 static int select_threads(int N) { return std::min(1024, std::max(128, N / 8)); }
 
 template <typename R, typename In>
@@ -1628,13 +1608,18 @@ static cudaError_t launch_comb(const V12Dev &d, int nslots, cudaStream_t s) {
     const int W = d.W, m2 = fft_m2(W);
     const FftShape f = fft_shape2(W, W, sizeof(c2_t<R>));
     const size_t sa = sizeof(c2_t<R>) * f.elems[0], sb = sizeof(c2_t<R>) * f.elems[1];
-    const size_t sk = (size_t)W * sizeof(key_t<R>) <= SEL_KEYS ? (size_t)W * sizeof(key_t<R>) : 0;
-    if ((e = set_smem(k_comb_a<R, In>, sa)) || (e = set_smem(k_comb_b<R>, sb)) || (e = set_smem(k_comb_select<R>, sk)))
-      return e;
+    if ((e = set_smem(k_comb_a<R, In>, sa)) || (e = set_smem(k_comb_b<R>, sb))) return e;
     k_comb_a<R, In><<<dim3(fft_ctas(f.elems[0], W / m2, W), d.comb_loops, nslots), f.elems[0] / 4, sa, s>>>(
         d, f.elems[0]);
     k_comb_b<R><<<dim3(fft_ctas(f.elems[1], m2, W), d.comb_loops, nslots), f.elems[1] / 4, sb, s>>>(d, f.elems[1]);
-    k_comb_select<R><<<dim3(d.comb_loops, nslots), select_threads(W), sk, s>>>(d);
+    const dim3 grid(d.comb_loops, nslots);
+    const int T = select_threads(W);
+    if (W <= 8 * 1024)
+      k_comb_select<R, 8><<<grid, T, 0, s>>>(d);
+    else if (W <= 16 * 1024)
+      k_comb_select<R, 16><<<grid, T, 0, s>>>(d);
+    else
+      k_comb_select<R, 0><<<grid, T, 0, s>>>(d);
     note_launches(3);
     return cudaGetLastError();
   }
@@ -1667,18 +1652,21 @@ static cudaError_t launch_bucket(const V12Dev &d, int nslots, cudaStream_t s) {
   const int Bmax = d.B_loc > d.B_est ? d.B_loc : d.B_est;
   if (d.pw) {
     const FftShape f = fft_shape2(d.B_loc, d.B_est, sizeof(c2_t<R>));
-    const size_t kl = (size_t)d.B_loc * sizeof(key_t<R>), ke = (size_t)d.B_est * sizeof(key_t<R>);
     const size_t sa = sizeof(c2_t<R>) * f.elems[0], sb = sizeof(c2_t<R>) * f.elems[1];
-    const size_t sk = std::max(kl <= SEL_KEYS ? kl : 0, ke <= SEL_KEYS ? ke : 0);
-    if ((e = set_smem(k_bucket_a<R>, sa)) || (e = set_smem(k_bucket_b<R>, sb)) ||
-        (e = set_smem(k_bucket_select<R>, sk)))
-      return e;
+    if ((e = set_smem(k_bucket_a<R>, sa)) || (e = set_smem(k_bucket_b<R>, sb))) return e;
     const int ml = fft_m2(d.B_loc), me = fft_m2(d.B_est);
     const int al = fft_ctas(f.elems[0], d.B_loc / ml, d.B_loc), ae = fft_ctas(f.elems[0], d.B_est / me, d.B_est);
     const int bl = fft_ctas(f.elems[1], ml, d.B_loc), be = fft_ctas(f.elems[1], me, d.B_est);
     k_bucket_a<R><<<dim3(d.L_loc * al + d.L_est * ae, nslots), f.elems[0] / 4, sa, s>>>(d, f.elems[0], al, ae);
     k_bucket_b<R><<<dim3(d.L_loc * bl + d.L_est * be, nslots), f.elems[1] / 4, sb, s>>>(d, f.elems[1], bl, be);
-    k_bucket_select<R><<<dim3(d.L, nslots), select_threads(Bmax), sk, s>>>(d);
+    const dim3 grid(d.L, nslots);
+    const int T = select_threads(Bmax);
+    if (Bmax <= 8 * 1024)
+      k_bucket_select<R, 8><<<grid, T, 0, s>>>(d);
+    else if (Bmax <= 16 * 1024)
+      k_bucket_select<R, 16><<<grid, T, 0, s>>>(d);
+    else
+      k_bucket_select<R, 0><<<grid, T, 0, s>>>(d);
     note_launches(2);  // the third is counted with the stage kernels
     return cudaGetLastError();
   }
