@@ -303,7 +303,8 @@ bool upload_v12_window(DBuf &b, const std::vector<double> &freq, int n, int q, i
       w[4 * m] = c;
       w[4 * m + 1] = dd;
       w[4 * m + 2] = c * c + dd * dd;  // same rounding as the reference's hadd
-      w[4 * m + 3] = 0.0;
+      // its reciprocal where the estimator may divide by it (see div_by), else 0
+      w[4 * m + 3] = w[4 * m + 2] > 0x1p-100 && w[4 * m + 2] < 0x1p100 ? 1.0 / w[4 * m + 2] : 0.0;
     }
     return b.upload(w);
   }
@@ -1621,7 +1622,10 @@ long sfft_debug_fetch(sfft_plan *plan, int what, void *dst, long cap) {
       case 9: {  // FP64 (c, d, c^2 + d^2, 0) doubles, FP32 conj(h)/|h|^2 floats
         const long q = P->n / (what == 8 ? p.B_loc : p.B_est);
         const DBuf &w = what == 8 ? P->win_a : P->win_b;
-        return P->prec == sfft::PREC_FP64 ? fetch(w.p, 4 * q, 8) : fetch(w.p, 2 * q, 4);
+        if (P->prec != sfft::PREC_FP64) return fetch(w.p, 2 * q, 4);
+        const long c = fetch(w.p, 4 * q, 8);
+        for (long m = 0; c > 0 && m < q; m++) ((double *)dst)[4 * m + 3] = 0.0;  // the device keeps a reciprocal there
+        return c;
       }
       default:
         break;

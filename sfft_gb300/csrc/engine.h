@@ -42,7 +42,7 @@ struct V12Dev {
   long xs_size;      // per slot, complex entries
   // plan constants
   const void *taps_loc, *taps_est;  // w complex (double2 or float2)
-  const void *win_loc, *win_est;    // q entries: FP64 double4 (c, d, c^2+d^2, 0); FP32 float2 (g)
+  const void *win_loc, *win_est;    // q entries: FP64 double4 (c, d, c^2+d^2, its reciprocal or 0); FP32 float2 (g)
   const void *tw_loc, *tw_est, *tw_comb;  // twiddle tables (double2 or float2)
   const void *win32_loc, *win32_est;  // FP64 plans: float2 g = conj-scaled window for bounds
   // per-slot workspace
