@@ -82,21 +82,14 @@ struct DBuf {
   }
 };
 
-int gcd_ref(int a, int b) { return (a % b == 0) ? b : gcd_ref(b, a % b); }  // src/utils.cc:41-46
-
-int mod_inverse_ref(int a, int n) {  // src/utils.cc:85-101
-  int i = n, v = 0, d = 1;
-  while (a > 0) {
-    int t = i / a, x = a;
-    a = i % x;
-    i = x;
-    x = d;
-    d = v - t * x;
-    v = x;
-  }
-  v %= n;
-  if (v < 0) v = (v + n) % n;
-  return v;
+// a^-1 mod n for odd a, n a power of two up to 2^30: the value of
+// src/utils.cc:85-101 (Euclid's algorithm, a dozen divisions; the inverse in
+// [0, n) is unique) by Newton's iteration, which doubles the correct low bits
+// -- 5 from the start value, then 10, 20, 40.
+int mod_inverse_pow2(int a, int n) {
+  unsigned x = (3u * (unsigned)a) ^ 2u;
+  for (int i = 0; i < 3; i++) x *= 2u - (unsigned)a * x;
+  return (int)(x & ((unsigned)n - 1u));
 }
 
 int ilog2(long v) {
@@ -458,11 +451,11 @@ void draw_params(const PlanImpl &P, int *rp, unsigned epoch, Rng &g) {
   const int n = P.n;
   if (P.version < 2) {
     const int L = L12(P);
-    for (int i = 0; i < L; i++) {  // src/computefourier-1.0-2.0.cc:465-474
+    for (int i = 0; i < L; i++) {  // src/computefourier-1.0-2.0.cc:465-474; gcd(a, n) = 1: a is odd
       int a = 0;
-      while (gcd_ref(a, n) != 1) a = (int)(g.rnd() % n);
+      while (!(a & 1)) a = (int)(g.rnd() & (n - 1));
       rp[i] = a;
-      rp[L + i] = mod_inverse_ref(a, n);
+      rp[L + i] = mod_inverse_pow2(a, n);
     }
     for (int c = 0; c < P.p12.Comb_loops; c++) {  // :62, once per Comb_Filt call
       if (P.version == 1) {
@@ -475,9 +468,9 @@ void draw_params(const PlanImpl &P, int *rp, unsigned epoch, Rng &g) {
     rp[2 * L + P.p12.Comb_loops] = (int)epoch;
   } else {  // src/computefourier-3.0.cc:800-810
     int a = 0;
-    while (gcd_ref(a, n) != 1) a = (int)(g.rnd() % n);
+    while (!(a & 1)) a = (int)(g.rnd() & (n - 1));
     rp[0] = a;
-    rp[1] = mod_inverse_ref(a, n);
+    rp[1] = mod_inverse_pow2(a, n);
     rp[2] = (int)(g.rnd() % n);
     rp[3] = (int)(unsigned)std::floor(g.d48() * n);
     rp[4] = (int)(unsigned)std::floor(g.d48() * n);
