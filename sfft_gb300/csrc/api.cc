@@ -688,15 +688,10 @@ bool launch(PlanImpl &P, int num, const void *const *in_dev, int in_type, cudaSt
     draw_params(P, &rp[(size_t)i * P.rp_stride], ep, g);
   }
   if (base == 0) P.last_rp.assign(rp.begin(), rp.begin() + P.rp_stride);
-  // pageable sources: the runtime stages them before returning
-  if (!cuda_ok(cudaMemcpyAsync(P.rparams.as<int>() + (size_t)base * P.rp_stride, rp.data(), sizeof(int) * rp.size(),
-                               cudaMemcpyHostToDevice, s),
+  if (!cuda_ok(sfft::setup_slots(rp.data(), P.rp_stride, in_dev, num, P.rparams.as<int>() + (size_t)base * P.rp_stride,
+                                 (const void **)P.inputs.p + base,
+                                 P.version < 2 ? P.counters.as<int>() + (size_t)base * sfft::CNT_STRIDE : nullptr, s),
                "params upload"))
-    return false;
-  std::vector<const void *> ptrs(in_dev, in_dev + num);
-  if (!cuda_ok(cudaMemcpyAsync((const void **)P.inputs.p + base, ptrs.data(), sizeof(void *) * num,
-                               cudaMemcpyHostToDevice, s),
-               "pointer upload"))
     return false;
   sfft::StageEvents *se = P.profiling ? P.take_set() : nullptr;
   bool ok;
@@ -1084,11 +1079,12 @@ bool plan_staged_view(sfft_plan *plan, int num, int in_type, int *out_idx, void 
 
 // Per call of the persistent executor, capturable: the staged draws and
 // input pointers go to the device, the counters of `num`
-// slots are cleared (what v12_run does before its first kernel).
+// slots are cleared (what setup_slots does for other launches).
 bool plan_persist_prepare(sfft_plan *plan, int num, cudaStream_t s) {
   PlanImpl *P = impl(plan);
   if (!P || P->version > 1 || num > P->staged_slots) return false;
   std::lock_guard<std::mutex> g(P->mu);
+  // copies and a memset, no kernel: a batch of the executor is one launch
   return cuda_ok(cudaMemcpyAsync(P->rparams.p, P->h_rp, sizeof(int) * (size_t)P->rp_stride * num,
                                  cudaMemcpyHostToDevice, s),
                  "params upload") &&
@@ -1104,11 +1100,9 @@ bool plan_launch_staged(sfft_plan *plan, int num, int in_type, int *out_idx, voi
   PlanImpl *P = impl(plan);
   if (!P || num > P->staged_slots) return false;
   std::lock_guard<std::mutex> g(P->mu);
-  if (!cuda_ok(cudaMemcpyAsync(P->rparams.p, P->h_rp, sizeof(int) * (size_t)P->rp_stride * num,
-                               cudaMemcpyHostToDevice, s),
-               "params upload") ||
-      !cuda_ok(cudaMemcpyAsync(P->inputs.p, P->h_in, sizeof(void *) * num, cudaMemcpyHostToDevice, s),
-               "pointer upload"))
+  if (!cuda_ok(sfft::setup_slots_staged(P->h_rp, P->rp_stride, P->h_in, num, P->rparams.as<int>(),
+                                        (const void **)P->inputs.p, P->counters.as<int>(), s),
+               "params upload"))
     return false;
   if (P->version < 2) {
     sfft::V12Dev d = v12_view(*P);

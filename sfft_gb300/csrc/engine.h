@@ -77,7 +77,17 @@ struct V12Dev {
   int in_type;
 };
 
-// Launches the whole v1/v2 pipeline for `nslots` signals on `stream`.
+// What a launch of `num` slots starts from, on the stream: its draws
+// (rp_stride ints per slot) and input pointers on the device, its counters
+// cleared (cnt null: v3, whose first kernel clears them).  The staged form
+// reads page-locked memory when it runs.
+cudaError_t setup_slots(const int *h_rp, int rp_stride, const void *const *h_in, int num, int *rp, const void **in,
+                        int *cnt, cudaStream_t s);
+cudaError_t setup_slots_staged(const int *h_rp, int rp_stride, const void *const *h_in, int num, int *rp,
+                               const void **in, int *cnt, cudaStream_t s);
+
+// Launches the whole v1/v2 pipeline for `nslots` signals on `stream`, after
+// setup_slots.
 // input_read (optional) is recorded once no later kernel reads the inputs.
 cudaError_t v12_run(const V12Dev &d, int nslots, cudaStream_t stream, StageEvents *se = nullptr,
                     cudaEvent_t input_read = nullptr);

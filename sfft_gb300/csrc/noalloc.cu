@@ -154,8 +154,8 @@ extern "C" long sfft_exec_noalloc(sfft_plan *plan, const void *d_in, int in_type
   int rp[2 * SFFT_NOALLOC_MAX_LOOPS + 16];
   plan_draw(plan, rp, g_epoch[dev]);
   const void *in_ptr = d_in;
-  if (cudaMemcpyAsync(base + o_rp, rp, sizeof(int) * rp_stride, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-      cudaMemcpyAsync(base + o_in, &in_ptr, sizeof(void *), cudaMemcpyHostToDevice, s) != cudaSuccess) {
+  if (setup_slots(rp, rp_stride, &in_ptr, 1, (int *)(base + o_rp), (const void **)(base + o_in), (int *)(base + o_cnt), s) !=
+      cudaSuccess) {
     cudaGetLastError();
     set_last_error("sfft_exec_noalloc: parameter upload failed");
     return -1;

@@ -1860,7 +1860,6 @@ static cudaError_t launch_estimate(const V12Dev &d, int nslots, cudaStream_t s) 
 template <typename R, typename In>
 static cudaError_t run_typed(const V12Dev &d, int nslots, cudaStream_t s, StageEvents *se, cudaEvent_t input_read) {
   cudaError_t e;
-  if ((e = cudaMemsetAsync(d.counters, 0, sizeof(int) * CNT_STRIDE * nslots, s))) return e;
   mark(se, s);
   if (d.version == 1) {
     if ((e = launch_comb<R, In>(d, nslots, s))) return e;
@@ -2229,6 +2228,38 @@ cudaError_t v12_run(const V12Dev &d, int nslots, cudaStream_t s, StageEvents *se
                                 : run_typed<double, float2>(d, nslots, s, se, input_read);
   return d.in_type == IN_C128 ? run_typed<float, double2>(d, nslots, s, se, input_read)
                               : run_typed<float, float2>(d, nslots, s, se, input_read);
+}
+
+// ------------------------------------------------------------------ setup --
+
+// The draws and input pointers of a launch captured in a graph, read from
+// page-locked host memory when the graph runs, and the cleared counters: one
+// node where two copies and a memset were three (24 uneven signals, 15
+// branches: 340 -> 321 us a pass).  A direct launch keeps the copies: with its
+// draws as kernel arguments it was no faster (four voted signals of n = 2^22,
+// k = 500: 207 -> 210 us).
+__global__ void __launch_bounds__(256) k_setup_staged(const int *h_rp, const void *const *h_in, int nrp, int *rp, int nin,
+                                                      const void **in, int ncnt, int *cnt) {
+  for (int i = threadIdx.x; i < nrp; i += 256) rp[i] = h_rp[i];
+  for (int i = threadIdx.x; i < nin; i += 256) in[i] = h_in[i];
+  for (int i = threadIdx.x; i < ncnt; i += 256) cnt[i] = 0;
+}
+
+// From pageable memory, which the runtime stages before it returns.
+cudaError_t setup_slots(const int *h_rp, int rp_stride, const void *const *h_in, int num, int *rp, const void **in,
+                        int *cnt, cudaStream_t s) {
+  cudaError_t e;
+  if ((e = cudaMemcpyAsync(rp, h_rp, sizeof(int) * (size_t)rp_stride * num, cudaMemcpyHostToDevice, s)) ||
+      (e = cudaMemcpyAsync(in, h_in, sizeof(void *) * (size_t)num, cudaMemcpyHostToDevice, s)))
+    return e;
+  return cnt ? cudaMemsetAsync(cnt, 0, sizeof(int) * CNT_STRIDE * (size_t)num, s) : cudaSuccess;
+}
+
+cudaError_t setup_slots_staged(const int *h_rp, int rp_stride, const void *const *h_in, int num, int *rp,
+                               const void **in, int *cnt, cudaStream_t s) {
+  k_setup_staged<<<1, 256, 0, s>>>(h_rp, h_in, rp_stride * num, rp, num, in, CNT_STRIDE * num, cnt);
+  note_launches(1);
+  return cudaGetLastError();
 }
 
 __global__ void k_copy_ints(const int *src, int *dst, int count) {
