@@ -43,13 +43,19 @@ int plan_device(sfft_plan *plan);
 void set_last_error(const char *m);
 }  // namespace sfft
 
+// Plans are accepted by the first figure; the second is room beside it for
+// what the kernels of an accepted plan keep per loop instead of once: the
+// selected buckets' bits (at most 65536 / 8 bytes) and the planes of a second
+// to eighth comb loop (at most 2^14 / 8 bytes each, longer combs being
+// refused).
 #define SFFT_NOALLOC_SCRATCH_BYTES (4u << 20)
+#define SFFT_NOALLOC_LOOP_BYTES (64u << 10)
 #define SFFT_NOALLOC_MAX_N (1 << 18)
 #define SFFT_NOALLOC_MAX_XS 65536L
 #define SFFT_NOALLOC_MAX_LOOPS 32
 #define SFFT_NOALLOC_MAX_DEVICES 64
 
-static __device__ __align__(256) unsigned char g_noalloc_scratch[SFFT_NOALLOC_SCRATCH_BYTES];
+static __device__ __align__(256) unsigned char g_noalloc_scratch[SFFT_NOALLOC_SCRATCH_BYTES + SFFT_NOALLOC_LOOP_BYTES];
 
 namespace {
 
@@ -102,16 +108,17 @@ extern "C" long sfft_exec_noalloc(sfft_plan *plan, const void *d_in, int in_type
   if (d.prec == PREC_FP64) off += up256(8 * (size_t)d.xs_size);
   const size_t o_J = off;
   off += up256(sizeof(int) * (size_t)L * d.num);
-  const size_t o_sel = off;
-  off += up256(sizeof(unsigned) * (size_t)d.L_loc * ((d.B_loc + 31) / 32));
   const size_t o_hits = off;
   off += up256(sizeof(int) * (size_t)hit_cap);
-  const size_t o_bits = off;
-  off += up256(sizeof(unsigned) * (size_t)d.comb_loops * ((d.W + 31) / 32));
   const size_t o_list = off;
   off += up256(sizeof(int) * (size_t)d.W);
+  const size_t o_bits = off;
+  const size_t plane = sizeof(unsigned) * (size_t)((d.W + 31) / 32);
+  off += up256(plane);
+  const size_t o_sel = d.version == 1 ? o_bits + up256(plane * (size_t)d.comb_loops) : off;
+  const size_t end = o_sel + up256(sizeof(unsigned) * (size_t)d.L_loc * ((d.B_loc + 31) / 32));
   if (d.large_buckets || d.large_comb || d.n > SFFT_NOALLOC_MAX_N || d.xs_size > SFFT_NOALLOC_MAX_XS || L > SFFT_NOALLOC_MAX_LOOPS ||
-      off > SFFT_NOALLOC_SCRATCH_BYTES) {
+      off > SFFT_NOALLOC_SCRATCH_BYTES || end > SFFT_NOALLOC_SCRATCH_BYTES + SFFT_NOALLOC_LOOP_BYTES) {
     set_last_error("sfft_exec_noalloc: plan exceeds the 4 MiB static scratch (limits: n <= 2^18, "
                    "at most 65536 bucket samples, at most 32 loops)");
     return -1;

@@ -46,7 +46,7 @@ __device__ __forceinline__ int dlog2(unsigned v) { return 31 - __clz(v); }
 // ------------------------------------------------------------------ fold --
 
 template <typename R, typename In>
-__global__ void __launch_bounds__(256) k_fold(V12Dev d) {
+__global__ void __launch_bounds__(256, 4) k_fold(V12Dev d) {
   const int slot = blockIdx.y;
   const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= d.xs_size) return;
@@ -74,11 +74,14 @@ __global__ void __launch_bounds__(256) k_fold(V12Dev d) {
   c2_t<R> acc;
   acc.x = 0;
   acc.y = 0;
-  // gathers issued 8 at a time, summed in increasing tap order
-  for (int t0 = b; t0 < w; t0 += 8 * B) {
-    c2_t<R> xv[8], hv[8];
+  // Gathers issued 4 at a time, summed in increasing tap order.  Four blocks
+  // an SM with 4 gathers each keep the FP64 pipes busier than two with 8,
+  // which need 102 registers a thread (one signal of 2^13 points 14.9 ->
+  // 12.9 us, of 2^20 24.8 -> 19.9, 64 of 2^16 234.5 -> 232.7).
+  for (int t0 = b; t0 < w; t0 += 4 * B) {
+    c2_t<R> xv[4], hv[4];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
+    for (int u = 0; u < 4; u++) {
       const int t = t0 + u * B;
       if (t < w) {
         const unsigned long long idx = ((unsigned long long)t * ai) & mask;
@@ -87,7 +90,7 @@ __global__ void __launch_bounds__(256) k_fold(V12Dev d) {
       }
     }
 #pragma unroll
-    for (int u = 0; u < 8; u++)
+    for (int u = 0; u < 4; u++)
       if (t0 + u * B < w) acc = cadd<R>(acc, cmul<R>(xv[u], hv[u]));
   }
   ((c2_t<R> *)d.xs)[(long)slot * d.xs_size + g] = acc;
@@ -1870,8 +1873,14 @@ static cudaError_t run_typed(const V12Dev &d, int nslots, cudaStream_t s, StageE
     dim3 fg((unsigned)((d.xs_size * S + 255) / 256), nslots);
     k_fold_split<In, S><<<fg, 256, 0, s>>>(d);
   } else {
-    dim3 fg((unsigned)((d.xs_size + 255) / 256), nslots);
-    k_fold<R, In><<<fg, 256, 0, s>>>(d);
+    // FP64: a bucket's taps are one chain of instructions that each hold an
+    // FP64 pipe, so few buckets go out in blocks of two warps, over as many
+    // SMs as there are; from four warps to a pipe on the block's size decides
+    // nothing (one signal of 2^13 points 17.5 us in blocks of eight warps, 12.0 in
+    // blocks of two; of 2^20 points 19.4 and 13.9)
+    const int T = d.xs_size * nslots <= (long)sm_count() * 4 * 4 * 32 ? 64 : 256;
+    dim3 fg((unsigned)((d.xs_size + T - 1) / T), nslots);
+    k_fold<R, In><<<fg, T, 0, s>>>(d);
   }
   if ((e = cudaGetLastError())) return e;
   mark(se, s);
