@@ -196,7 +196,7 @@ int xs_perm_of(const PlanImpl &P) {
   if (P.version != 1 || P.voted || P.large_b || p.W_Comb <= 0) return 0;
   const long ql = P.n / p.B_loc, qe = P.n / p.B_est, R = P.n / p.W_Comb;
   if (p.W_Comb % ql || p.W_Comb % qe || R < 32) return 0;
-  return ilog2(std::min<long>(R, 256));
+  return ilog2(std::min<long>(R, sfft::EC_GROUP_MAX));
 }
 
 // Position of bucket b of a loop of B buckets in the grouped layout.

@@ -31,6 +31,11 @@ enum ErrBits { ERR_HIT_OVERFLOW = 1, ERR_OUT_OVERFLOW = 2, ERR_V3_NOCONVERGE = 4
                ERR_WAIT_TIMEOUT = 16 };
 
 // ---------------------------------------------------------------- v1/v2 --
+
+// Most candidates that share a run of buckets (V12Dev::xs_perm): a CTA of
+// the estimation by comb residue.
+constexpr int EC_GROUP_MAX = 128;
+
 struct V12Dev {
   int version;  // 0 = v1, 1 = v2
   int prec;

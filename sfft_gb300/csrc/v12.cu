@@ -1278,11 +1278,17 @@ __global__ void __launch_bounds__(128, est64_blocks(LN)) k_estimate64(V12Dev d, 
 // reads its candidate's value of every loop from shared memory -- lanes i
 // of a warp read entries (rot + i ai) mod G, distinct mod 16, so without
 // bank conflicts -- and takes the lower medians.  Several CTAs per SM
-// overlap one CTA's copies with the others' arithmetic.  Output position
-// h = residue index * R + group * G + i; the output is a set, so its order
-// is free.
+// overlap one CTA's copies with the others' arithmetic.  Output positions:
+// residue by residue, see ec_place.
 
-constexpr int EC_THREADS = 256;            // candidates per CTA of k_estimate_comb32
+// Candidates, and threads, per CTA.  A CTA waits for its copies, then
+// computes; many small CTAs an SM keep some of them computing.  32 FP32
+// signals of 2^22 points, k = 100, by threads x CTAs per SM: 256 x 4 353 us,
+// 128 x 8 348, 128 x 9 (56 registers) 330, 128 x 10 (48) 356, 64 x 16 384,
+// 64 x 18 370; 8 FP64 signals: 256 x 4 180, 128 x 7 167, 128 x 8 166,
+// 128 x 9 179, 64 x 16 171 (before ec_place interleaved their stores, which
+// costs 2 and 6 us of that).  Groups are at most this long (xs_perm_of).
+constexpr int EC_THREADS = EC_GROUP_MAX;
 constexpr int EC_MAXL = 32;
 constexpr long EC_WAIT_POLLS = 1L << 22;
 
@@ -1340,6 +1346,20 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned b
                : "memory");
 }
 
+// The output lists a residue's R candidates as if groups were of min(R, 2
+// EC_GROUP_MAX): position (grp' , i') holds rep = grp' + i' S'.  Where R is
+// larger than a group, two neighbouring groups interleave in one such stretch:
+// unit v of a residue is the group grp = v / 2 + (v odd ? S / 2 : 0), and its
+// candidate i stands at 2 i + (v odd) of the pair's places.
+__device__ __forceinline__ int ec_group(unsigned v, int lr, int lg) {
+  const int p = lr > lg;
+  return (int)((v >> p) + ((v & (unsigned)p) << (lr - lg - p)));
+}
+__device__ __forceinline__ long ec_place(long hb, int i, int lr, int lg) {  // hb: first position of unit v's run
+  const int p = lr > lg;
+  return (hb & ~((1L << (lg + p)) - 1)) + ((i << p) | ((int)(hb >> lg) & p));
+}
+
 // Staging of candidates [h0, h0 + NTH) of a slot (total: the slot's candidate
 // count, a multiple of G, so a group is wholly live or wholly past the end;
 // nothing is done when h0 >= total): one thread per (group, loop) writes the group's
@@ -1369,7 +1389,7 @@ __device__ __forceinline__ int ec_stage(const V12Dev &d, int slot, long h0, long
     j = threadIdx.x - u * L;
     const unsigned h = (unsigned)h0 + ((unsigned)u << lg), ridx = h >> lr;
     res = d.comb_list[(long)slot * d.W + min(ridx, (unsigned)d.W - 1u)];
-    grp = (int)((h & ((1u << lr) - 1u)) >> lg);
+    grp = ec_group((h & ((1u << lr) - 1u)) >> lg, lr, lg);
     ai = (unsigned)d.rparams[(long)slot * d.rp_stride + L + j];
   }
   const int live = (int)min((long)units, (total - h0) >> lg);
@@ -1428,7 +1448,7 @@ __device__ __forceinline__ int ec_stage(const V12Dev &d, int slot, long h0, long
 // The staging area's start in dynamic shared memory: runs of 8 G bytes at
 // multiples of 8 G, so that a run's base and an offset within it combine by OR
 // (one logic operation with the modulus).
-constexpr int EC_ALIGN = 2048;  // 8 * 256 bytes, the longest run
+constexpr int EC_ALIGN = 8 * EC_GROUP_MAX;  // bytes of the longest run
 __device__ __forceinline__ float2 *ec_area(void *dyn) {
   return (float2 *)((unsigned char *)dyn + (-smem_u32(dyn) & (EC_ALIGN - 1u)));
 }
@@ -1467,14 +1487,14 @@ __device__ __forceinline__ void ec32_values(const V12Dev &d, const float2 *seg, 
 }
 
 // Lower medians of the values and the output entry of candidate i of
-// group (res, grp), position h0 + threadIdx.x of the slot's output.
+// group (res, grp).
 template <int LN, bool EXACT>
 __device__ __forceinline__ void ec32_finish(const V12Dev &d, int slot, long h0, int res, int grp, int i,
                                             float (&re)[LN], float (&im)[LN]) {
   const int Lr = EXACT ? LN : d.L;
   const float mre = lower_median<LN, EXACT>(re, Lr), mim = lower_median<LN, EXACT>(im, Lr);
-  const int lw = dlog2((unsigned)d.W), ls = dlog2((unsigned)d.n) - lw - d.xs_perm;  // S = n / W / G = 2^ls
-  const long o = (long)slot * d.out_stride + h0 + threadIdx.x;
+  const int lg = d.xs_perm, lw = dlog2((unsigned)d.W), lr = dlog2((unsigned)d.n) - lw, ls = lr - lg;  // S = 2^ls
+  const long o = (long)slot * d.out_stride + ec_place(h0 + threadIdx.x - i, i, lr, lg);
   d.out_idx[o] = (int)((((unsigned)grp + ((unsigned)i << ls)) << lw) + (unsigned)res);
   ((float2 *)d.out_val)[o] = make_float2(mre, mim);
 }
@@ -1557,7 +1577,7 @@ __device__ __forceinline__ int ec_proven(const float (&key)[LN], int Lr, const E
 // the warp, one loop per lane (by one thread it took 20 us, which a single
 // signal waited for: 31 -> 10 us at one signal of 2^20 points, 310 -> 265 us
 // at 8 of 2^22).  There, the proof by sums instead of counts, the corrected
-// quotient instead of IEEE division and four CTAs per SM instead of three
+// quotient instead of IEEE division and 1024 threads per SM instead of 768
 // took it from 262 to 184 us, the shorter staging chain to 178.
 template <int LN, bool EXACT, int NTH>
 __device__ __forceinline__ void ec64_block(const V12Dev &d, int slot, long h0, long total, float2 *seg,
@@ -1612,8 +1632,8 @@ __device__ __forceinline__ void ec64_block(const V12Dev &d, int slot, long h0, l
       atomicAdd(&d.counters[slot * CNT_STRIDE + CNT_EXACT], 1);
     }
   }
-  const int lw = dlog2((unsigned)d.W), ls = dlog2((unsigned)d.n) - lw - lg;
-  const long o = (long)slot * d.out_stride + h0 + threadIdx.x;
+  const int lw = dlog2((unsigned)d.W), lr = dlog2((unsigned)d.n) - lw, ls = lr - lg;
+  const long o = (long)slot * d.out_stride + ec_place(h0 + threadIdx.x - i, i, lr, lg);
   d.out_idx[o] = (int)((((unsigned)sh.grp[u] + ((unsigned)i << ls)) << lw) + (unsigned)sh.res[u]);
   ((double2 *)d.out_val)[o] = res;
 }
@@ -1624,7 +1644,7 @@ __device__ __forceinline__ long ec_total(const V12Dev &d, int slot) {
 }
 
 template <int LN, bool EXACT>
-__global__ void __launch_bounds__(EC_THREADS, 4) k_estimate_comb32(V12Dev d) {
+__global__ void __launch_bounds__(EC_THREADS, 9) k_estimate_comb32(V12Dev d) {
   extern __shared__ __align__(128) float2 seg[];   // [loop][EC_THREADS]
   __shared__ EcShared<EC_THREADS> sh;
   const int slot = blockIdx.y;
@@ -1634,7 +1654,7 @@ __global__ void __launch_bounds__(EC_THREADS, 4) k_estimate_comb32(V12Dev d) {
 }
 
 template <int LN, bool EXACT>
-__global__ void __launch_bounds__(EC_THREADS, 4) k_estimate_comb64(V12Dev d) {
+__global__ void __launch_bounds__(EC_THREADS, 8) k_estimate_comb64(V12Dev d) {
   extern __shared__ __align__(128) float2 seg64[];   // [loop][EC_THREADS]
   __shared__ EcShared<EC_THREADS> sh;
   __shared__ int2 srcmw[(EC_THREADS / 32) * EC_MAXL];
