@@ -802,8 +802,20 @@ bool ensure_host_counters(PlanImpl &P, int num) {
 // signals of 2^16 points: 472 us, from the end of the fold on 480).
 // One memset per output took 41 us for 2^24 points after a v3 transform of 110
 // us, and 64 calls for 64 outputs of 2^16 points.
+// Work that is already queued on the plan's stream (a batch with a NULL stream,
+// or what a program put on sfft_plan_stream) may use the same buffers, so the
+// clearing comes after it; an idle stream, the usual case, costs one query.
 bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out, const char *in_dev, const char *out_dev) {
   cudaStream_t s = P.stream;
+  struct Drain {  // a failed call leaves nothing writing to the caller's buffers
+    PlanImpl &P;
+    bool done = false;
+    ~Drain() {
+      if (done) return;
+      cudaStreamSynchronize(P.copy_out);
+      cudaStreamSynchronize(P.stream);
+    }
+  } drain{P};
   const size_t nb = sizeof(double) * 2 * (size_t)P.n;
   std::vector<const void *> dev_in(num);
   std::vector<void *> dense(num);
@@ -815,6 +827,11 @@ bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out, con
   if (need_in_stage && !P.in_stage.ensure(nb * P.slots)) return false;
   if (need_out_stage && !P.dense_stage.ensure(nb * P.slots)) return false;
   if (!ensure_host_counters(P, num)) return false;
+  const cudaError_t idle = cudaStreamQuery(s);
+  cudaGetLastError();
+  if (idle != cudaSuccess && (!cuda_ok(cudaEventRecord(P.ev_in[0], s), "event") ||
+                              !cuda_ok(cudaStreamWaitEvent(P.copy_out, P.ev_in[0], 0), "wait")))
+    return false;
   for (int i = 0; i < num; i++) {
     dev_in[i] = in_dev[i] ? (const void *)in[i] : (const void *)((char *)P.in_stage.p + nb * i);
     dense[i] = out_dev[i] ? (void *)out[i] : (void *)((char *)P.dense_stage.p + nb * i);
@@ -847,6 +864,7 @@ bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out, con
                "counters") ||
       !cuda_ok(cudaStreamSynchronize(s), "exec"))
     return false;
+  drain.done = true;
   return check_counts(P.h_cnt, num);
 }
 

@@ -1,0 +1,117 @@
+"""The order of the streams' work, on the CPU: the library's host sources run
+over a CUDA runtime that keeps, for every operation, what is ordered before it
+(fake_cuda/runtime.cc).  Work that a program queued on the plan's stream, or
+an asynchronous batch on a stream of its own, comes before what a later call
+does to the same buffers."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from sfft_gb300 import _lib, build
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SHAPES = [(0, 1 << 13, 50), (1, 1 << 14, 50), (2, 1 << 13, 16)]   # version, n, k
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    src = [os.path.join(HERE, "fake_cuda", "runtime.cc")]
+    src += [os.path.join(build.CSRC, f) for f in ("api.cc", "host_plan.cc", "tune.cc")]
+    subprocess.check_call(["g++", "-O1", "-fPIC", "-std=c++17", "-fopenmp", "-shared", "-Wl,-Bsymbolic", "-o", so] + src +
+                          ["-I" + os.path.join(build._cuda_home(), "include"), "-I" + os.path.join(build.ROOT, "include"),
+                           "-I" + build.CSRC])
+    L = ctypes.CDLL(so)
+    vp, cl = ctypes.c_void_p, ctypes.c_long
+    for f in (L.sfft_make_plan_ex, L.sfft_plan_stream):
+        f.restype = vp
+    for f in (L.sfft_output_capacity, L.sfft_exec_sparse):
+        f.restype = cl
+    L.sfft_last_error.restype = L.fake_name.restype = ctypes.c_char_p
+    return L
+
+
+class Plan:
+    def __init__(self, L, version, n, k, max_batch=4):
+        self.L, self.n = L, n
+        self.p = vp(L.sfft_make_plan_ex(n, k, version, 0, ctypes.byref(_lib.Options(0, -1, max_batch))))
+        assert self.p, L.sfft_last_error()
+        self.cap = L.sfft_output_capacity(self.p)
+        self.bufs = []
+
+    def device(self, nbytes):
+        p = ctypes.c_void_p()
+        assert self.L.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(nbytes)) == 0
+        ctypes.memset(p, 0, nbytes)
+        self.bufs.append(p)
+        return p
+
+    def signals(self, m=1):
+        return (ctypes.c_void_p * m)(*[self.device(16 * self.n).value for _ in range(m)])
+
+    def batch(self, m=2, stream=None):
+        """An asynchronous batch; its transforms in the log."""
+        at = self.L.fake_ops()
+        r = self.L.sfft_exec_batch_ex(self.p, m, self.signals(m), 0, None, self.device(4 * m * self.cap),
+                                      self.device(16 * m * self.cap), self.device(4 * m), ctypes.c_long(self.cap),
+                                      ctypes.c_void_p(stream))
+        return r, self.ops(at, "transform")
+
+    def ops(self, at, *names):
+        return [i for i in range(at, self.L.fake_ops()) if self.L.fake_name(i).decode() in names]
+
+    def free(self):
+        self.L.sfft_free_plan(self.p)
+        for b in self.bufs:
+            self.L.cudaFree(b)
+
+
+vp = ctypes.c_void_p
+
+
+@pytest.fixture(params=SHAPES, ids=["v1", "v2", "v3"])
+def plan(fake, request):
+    p = Plan(fake, *request.param)
+    yield p
+    p.free()
+
+
+@pytest.mark.parametrize("m", [1, 5])   # one launch, and two
+def test_outputs_are_cleared_after_work_on_the_plans_stream(fake, plan, m):
+    """A batch with a NULL stream, or a copy queued on sfft_plan_stream, may
+    still read the buffers that a dense call then writes."""
+    before = plan.batch()[1]
+    before.append(fake.fake_ops())
+    fake.fake_work(vp(fake.sfft_plan_stream(plan.p)))
+    at = fake.fake_ops()
+    ins, outs = plan.signals(m), plan.signals(m)
+    fake.sfft_exec_many(plan.p, m, ins, outs)
+    assert fake.sfft_last_error() == b""
+    clears = plan.ops(at, "clear")
+    assert clears
+    for c in clears:
+        assert all(fake.fake_before(b, c) for b in before)
+
+
+def test_clearing_does_not_wait_for_the_calls_own_input_copies(fake, plan):
+    """On an idle plan the outputs are cleared beside the copies of host inputs
+    (v1 / v2; v3 clears after its filters)."""
+    x = np.zeros(plan.n, dtype=np.complex128)
+    at = fake.fake_ops()
+    fake.sfft_exec_many(plan.p, 1, (vp * 1)(x.ctypes.data), plan.signals(1))
+    copy, clear = plan.ops(at, "to device")[0], plan.ops(at, "clear")[0]
+    if plan.p and ctypes.cast(plan.p, ctypes.POINTER(_lib.Plan)).contents.version != 2:
+        assert not fake.fake_before(copy, clear)
+
+
+def test_nothing_is_written_after_a_failed_call_returned(fake, plan):
+    at = fake.fake_ops()
+    fake.fake_fail(b"scatter")
+    fake.sfft_exec_many(plan.p, 1, plan.signals(1), plan.signals(1))
+    fake.fake_fail(b"")
+    assert fake.sfft_last_error() != b""
+    clears = plan.ops(at, "clear")
+    assert clears and all(fake.fake_waited(c) for c in clears)
