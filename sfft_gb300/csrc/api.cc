@@ -112,7 +112,8 @@ struct PlanImpl {
   sfft::V12Params p12;
   sfft::V3Params p3;
   cudaStream_t stream = nullptr;
-  cudaEvent_t done = nullptr;
+  cudaEvent_t done = nullptr;     // recorded after each asynchronous batch
+  bool batch_elsewhere = false;   // one of them ran on a stream of its caller
   // host-buffer pipeline of sfft_exec_many: copies in / out on their own streams
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
   cudaEvent_t ev_in[2] = {nullptr, nullptr}, ev_comp[2] = {nullptr, nullptr}, ev_out[2] = {nullptr, nullptr};
@@ -759,6 +760,14 @@ std::mutex g_alloc_mu;
 std::set<void *> g_pinned;
 
 PlanImpl *impl(sfft_plan *p) { return p ? (PlanImpl *)p->data : nullptr; }
+
+// Asynchronous batches run on their caller's stream with the plan's workspace:
+// whatever runs on the plan's stream next comes after the last of them.
+bool after_batches(PlanImpl &P) {
+  if (P.batch_elsewhere && !cuda_ok(cudaStreamWaitEvent(P.stream, P.done, 0), "event wait")) return false;
+  P.batch_elsewhere = false;
+  return true;
+}
 
 // Whether the input and output arrays (nb bytes each) of device pointers
 // overlap anywhere, an in-place transform among them.
@@ -1423,6 +1432,7 @@ void sfft_exec_many(sfft_plan *plan, int num, complex_t **in, complex_t **out) {
   std::lock_guard<std::mutex> g(P->mu);
   cudaSetDevice(P->device);
   g_err.clear();
+  if (!after_batches(*P)) return;
   const int chunk = std::max(1, std::min(P->max_batch, num));
   std::vector<char> in_dev(num), out_dev(num);
   bool all_host = num > 1;
@@ -1451,6 +1461,7 @@ long sfft_exec_sparse(sfft_plan *plan, const complex_t *in, int *out_idx, comple
   std::lock_guard<std::mutex> g(P->mu);
   cudaSetDevice(P->device);
   g_err.clear();
+  if (!after_batches(*P)) return -1;
   cudaStream_t s = P->stream;
   const size_t nb = sizeof(double) * 2 * (size_t)P->n;
   const void *dev_in = in;
@@ -1505,6 +1516,7 @@ int sfft_exec_many_sparse(sfft_plan *plan, int num, const complex_t *const *in, 
   std::lock_guard<std::mutex> g(P->mu);
   cudaSetDevice(P->device);
   g_err.clear();
+  if (!after_batches(*P)) return -1;
   const int chunk = std::max(1, std::min(P->max_batch, (num + 31) / 32));  // about 32 pipelined chunks
   return exec_sparse_pipelined(*P, num, in, out_idx, out_val, out_count, out_stride, chunk) ? 0 : -1;
 }
@@ -1532,14 +1544,20 @@ int sfft_exec_batch_ex(sfft_plan *plan, int num, const void *const *in, int in_t
   if (!ensure_slots(*P, std::min(num, std::max(1, P->max_batch)))) return -1;
   if (!cuda_ok(cudaStreamWaitEvent(s, P->done, 0), "event wait")) return -1;
   const size_t cs = (P->version < 2 && P->prec == sfft::PREC_FP32) ? 8 : 16;
-  for (int i0 = 0; i0 < num; i0 += P->slots) {
+  bool good = true;
+  for (int i0 = 0; good && i0 < num; i0 += P->slots) {
     const int m = std::min(P->slots, num - i0);
     // results go straight into the caller's strided buffers
     OutTarget t{out_idx + (size_t)i0 * out_stride, (char *)out_val + cs * (size_t)i0 * out_stride, out_count + i0,
                 out_stride};
-    if (!launch(*P, m, in + i0, in_type, s, &t, 0, seeds ? seeds + i0 : nullptr)) return -1;
+    good = launch(*P, m, in + i0, in_type, s, &t, 0, seeds ? seeds + i0 : nullptr);
   }
-  return cuda_ok(cudaEventRecord(P->done, s), "event") ? 0 : -1;
+  // also after a failure: what was launched before it is still running
+  const cudaError_t e = cudaEventRecord(P->done, s);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;  // nothing runs where the batch is only captured
+  if (s != P->stream && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+    P->batch_elsewhere = true;
+  return good && cuda_ok(e, "event") ? 0 : -1;
 }
 
 int sfft_sync(sfft_plan *plan) {

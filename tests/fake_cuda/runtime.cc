@@ -37,6 +37,7 @@ Set host;                     // what the host has waited for
 std::map<char *, size_t> mem;
 size_t limit_bytes = (size_t)-1;
 std::string failing;
+int passes = 0;  // operations of that name that still succeed
 long next_handle = 0x1000;
 
 void merge(Set &a, const Set &b) {
@@ -47,7 +48,7 @@ void merge(Set &a, const Set &b) {
 
 cudaError_t op(const char *name, const void *s, bool whole = true) {
   std::lock_guard<std::recursive_mutex> g(mu);
-  if (failing == name) return cudaErrorUnknown;
+  if (failing == name && passes-- <= 0) return cudaErrorUnknown;
   Set &st = streams[(long)s];
   merge(st, host);
   const size_t i = ops.size();
@@ -79,7 +80,8 @@ int fake_before(int a, int b) { return a < (int)ops[b].before.size() && ops[b].b
 int fake_waited(int a) { return a < (int)host.size() && host[a]; }
 void fake_work(void *stream) { op("work", stream); }
 void fake_limit(size_t bytes) { limit_bytes = bytes; }
-void fake_fail(const char *name) { failing = name; }
+void fake_fail_after(const char *name, int count) { failing = name, passes = count; }
+void fake_fail(const char *name) { fake_fail_after(name, 0); }
 
 // --------------------------------------------------------- the runtime --
 
@@ -149,6 +151,9 @@ cudaError_t cudaStreamQuery(cudaStream_t s) {
     if (st[i] && !fake_waited((int)i)) return cudaErrorNotReady;
   return cudaSuccess;
 }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus *st) {
+  return *st = cudaStreamCaptureStatusNone, cudaSuccess;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
   std::lock_guard<std::recursive_mutex> g(mu);
   merge(streams[(long)s], events[(long)e]);
@@ -202,7 +207,9 @@ cudaError_t v3_run(const V3Dev &d, int nslots, cudaStream_t s, StageEvents *, cu
   return e;
 }
 cudaError_t clear_dense(void *const *, int, int, cudaStream_t s) { return op("clear", s); }
-cudaError_t copy_ints(const int *, int *, int, cudaStream_t s) { return op("copy", s); }
+cudaError_t copy_ints(const int *src, int *dst, int count, cudaStream_t s) {
+  return cudaMemcpyAsync(dst, src, sizeof(int) * count, cudaMemcpyDeviceToDevice, s);
+}
 cudaError_t scatter_dense(const int *, const void *, int, const int *, int, void *const *, int, cudaStream_t s) {
   return op("scatter", s);
 }

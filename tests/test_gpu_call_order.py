@@ -89,3 +89,30 @@ def test_dense_output_over_a_queued_batchs_input(env, version, n, k, batch):
         c.close(c.dense(c.y[0], x[s]), dense)
         c.same(c.lists(), want)
     c.L.sfft_free_plan(c.plan)
+
+
+@pytest.mark.parametrize("version,n,k,batch", SHAPES)
+def test_calls_after_a_batch_on_another_stream(env, version, n, k, batch):
+    """The plan's workspace is the batch's until it ran."""
+    c = Calls(env, version, n, k, batch)
+    c.batch(c.x)
+    want = c.lists()
+    dense = c.dense(c.y[0], c.torch.full_like(c.y[0], 3))
+    host = c.y[0].cpu().numpy()
+    st = c.torch.cuda.Stream()
+    hi, hv = np.empty(c.cap, np.int32), np.empty(c.cap, np.complex128)
+    for sparse in (False, True):
+        c.cnt.zero_()
+        c.torch.cuda.synchronize()
+        c.batch(c.x, st.cuda_stream)
+        if sparse:
+            c.O.seed_libc(9)
+            m = c.L.sfft_exec_sparse(c.plan, host.ctypes.data, hi.ctypes.data, hv.ctypes.data, c.cap)
+            assert m >= 0, c.last_error()
+            got = np.zeros_like(dense)
+            got[hi[:m]] = hv[:m]
+            c.close(got, dense)
+        else:
+            c.close(c.dense(c.y[0], c.torch.full_like(c.y[0], 3)), dense)
+        c.same(c.lists(), want)
+    c.L.sfft_free_plan(c.plan)

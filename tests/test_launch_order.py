@@ -115,3 +115,56 @@ def test_nothing_is_written_after_a_failed_call_returned(fake, plan):
     assert fake.sfft_last_error() != b""
     clears = plan.ops(at, "clear")
     assert clears and all(fake.fake_waited(c) for c in clears)
+
+
+def _dense(p):
+    p.L.sfft_exec_many(p.p, 1, p.signals(1), p.signals(1))
+
+
+def _dense_host(p):
+    x = np.zeros((3, p.n), dtype=np.complex128)
+    a = (vp * 3)(*[v.ctypes.data for v in x])
+    p.L.sfft_exec_many(p.p, 3, a, a)
+
+
+def _sparse(p):
+    assert p.L.sfft_exec_sparse(p.p, p.device(16 * p.n), p.device(4 * p.cap), p.device(16 * p.cap),
+                                ctypes.c_long(p.cap)) == 0
+
+
+def _many_sparse(p):
+    cnt = (ctypes.c_int * 2)()
+    assert p.L.sfft_exec_many_sparse(p.p, 2, p.signals(2), p.device(8 * p.cap), p.device(32 * p.cap), cnt,
+                                     ctypes.c_long(p.cap)) == 0
+
+
+@pytest.mark.parametrize("call", [_dense, _dense_host, _sparse, _many_sparse])
+def test_calls_come_after_batches_on_other_streams(fake, plan, call):
+    """The plan's draws, buckets and lists belong to the batch until it ran."""
+    st = vp()
+    assert fake.cudaStreamCreateWithFlags(ctypes.byref(st), 1) == 0
+    plan.batch(4)                                   # the workspace has its size: nothing below waits for an allocation
+    fake.cudaDeviceSynchronize()
+    r, batch = plan.batch(2, st.value)
+    assert r == 0 and batch
+    at = fake.fake_ops()
+    call(plan)
+    assert fake.sfft_last_error() == b""
+    later = plan.ops(at, "setup", "transform")
+    assert later
+    for i in later:
+        assert all(fake.fake_before(b, i) for b in batch)
+
+
+def test_calls_come_after_the_part_of_a_failed_batch(fake, plan):
+    st = vp()
+    assert fake.cudaStreamCreateWithFlags(ctypes.byref(st), 1) == 0
+    plan.batch(4)
+    fake.cudaDeviceSynchronize()
+    fake.fake_fail_after(b"transform", 1)           # five signals are two launches of at most four
+    r, batch = plan.batch(5, st.value)
+    fake.fake_fail(b"")
+    assert r == -1 and len(batch) == 1
+    at = fake.fake_ops()
+    _dense(plan)
+    assert fake.fake_before(batch[0], plan.ops(at, "setup")[0])
