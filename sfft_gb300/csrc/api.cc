@@ -335,6 +335,7 @@ bool upload_taps(DBuf &b, const std::vector<double> &t, int prec) {
 bool ensure_slots(PlanImpl &P, int want) {
   if (want <= P.slots) return true;
   const size_t S = (size_t)want;
+  P.slots = 0;  // until every buffer is there: one that could not grow is gone
   const size_t cs = P.prec == sfft::PREC_FP64 ? 16 : 8;
   if (!P.counters.ensure(sizeof(int) * sfft::CNT_STRIDE * S)) return false;
   if (!P.inputs.ensure(sizeof(void *) * S) || !P.dense_ptrs.ensure(sizeof(void *) * S)) return false;
@@ -1461,7 +1462,7 @@ long sfft_exec_sparse(sfft_plan *plan, const complex_t *in, int *out_idx, comple
   std::lock_guard<std::mutex> g(P->mu);
   cudaSetDevice(P->device);
   g_err.clear();
-  if (!after_batches(*P)) return -1;
+  if (!after_batches(*P) || !ensure_slots(*P, 1)) return -1;
   cudaStream_t s = P->stream;
   const size_t nb = sizeof(double) * 2 * (size_t)P->n;
   const void *dev_in = in;

@@ -1,8 +1,8 @@
-"""The order of the streams' work, on the CPU: the library's host sources run
-over a CUDA runtime that keeps, for every operation, what is ordered before it
+"""What the library's host code launches, on the CPU: its sources run over a
+CUDA runtime that keeps, for every operation, what is ordered before it
 (fake_cuda/runtime.cc).  Work that a program queued on the plan's stream, or
 an asynchronous batch on a stream of its own, comes before what a later call
-does to the same buffers."""
+does to the same buffers; a transform never runs with a buffer missing."""
 import ctypes
 import os
 import subprocess
@@ -168,3 +168,22 @@ def test_calls_come_after_the_part_of_a_failed_batch(fake, plan):
     at = fake.fake_ops()
     _dense(plan)
     assert fake.fake_before(batch[0], plan.ops(at, "setup")[0])
+
+
+@pytest.mark.parametrize("call", [_dense, _dense_host, _sparse, _many_sparse])
+@pytest.mark.parametrize("limit", [1 << 14, 1 << 18, 1 << 20, 1 << 22])
+def test_buffers_are_whole_after_a_batch_that_did_not_fit(fake, plan, call, limit):
+    """Growing the workspace for a large batch fails at one of its buffers; the
+    calls after that have all of them again (or say that they have not)."""
+    fake.fake_limit(ctypes.c_size_t(limit))
+    at = fake.fake_ops()
+    ins, room = plan.signals(1)[0] if limit >= 16 * plan.n else None, vp(64)
+    big = (vp * 4)(ins, ins, ins, ins)
+    fake.sfft_exec_batch_ex(plan.p, 4, big, 0, None, room, room, room, ctypes.c_long(plan.cap), None)
+    failed = not plan.ops(at, "transform")
+    fake.fake_limit(ctypes.c_size_t(-1))
+    at = fake.fake_ops()
+    call(plan)
+    done = plan.ops(at, "transform")
+    assert done and all(fake.fake_whole(i) for i in done)
+    assert failed or limit > 1 << 18
