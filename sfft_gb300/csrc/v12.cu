@@ -1538,9 +1538,14 @@ __device__ __forceinline__ double2 ec_exact64(const V12Dev &d, const EcVal &t, i
 // element is proven when no other interval meets its own, |key - med| > e +
 // e_med for all others: then exactly as many exact values lie below it as
 // keys do.  With w = (e + e_med) - |key - med|, sum(w + |w|) over all loops
-// equals the median's own term exactly iff no other w is positive (adding
-// zeros is exact); an infinity or a NaN anywhere makes the sum NaN and the
-// test fail.  This runs on the FMA pipe; the median networks have the ALU.
+// equals the median's own term if no other w is positive (adding zeros is
+// exact).  A positive w of at most 2^-24 of the median's own term may vanish in
+// the sum's rounding; an overlap of the intervals that small is far within the
+// part of e (0.45 of it) that the bound above leaves unused.  An infinite or
+// NaN key, or an infinite e of another loop, makes the sum differ or NaN; where
+// the median's own e is infinite (values near FLT_MAX, whose scale overflows
+// before they do) every term is, so the own term must be finite.
+// This runs on the FMA pipe; the median networks have the ALU.
 constexpr float EC_ERR = 0x1p-17f;
 __device__ __forceinline__ float ec_key(float v, int j) { return __int_as_float((__float_as_int(v) & ~31) | j); }
 __device__ __forceinline__ float ec_scale(float2 x, const EcVal &t) {
@@ -1567,7 +1572,7 @@ __device__ __forceinline__ int ec_proven(const float (&key)[LN], int Lr, const E
     }
   }
   const float own = __fmaf_rn(ec_scale(ec_at<NTH>(base, tv[idx], i, mask, idx), tv[idx]), EC_ERR, em);
-  proven = sum == __fadd_rn(own, own);
+  proven = sum == __fadd_rn(own, own) && own < INFINITY;
   return idx;
 }
 
