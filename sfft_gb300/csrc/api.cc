@@ -580,8 +580,8 @@ sfft::V3Dev v3_view(PlanImpl &P) {
   d.pi2_over_n = PI2 / P.n;
   d.w_dbl = p.W_Man;
   d.inv_w2 = (1. / p.W_Man) * (1. / p.W_Man);
-  d.tol_man = P.n * 1e-10;
-  d.tol_gauss = P.n * 1e-12;  // (c1 / c0 - 1)^2 / n < 1e-12
+  d.tol_man = std::sqrt(P.n * 1e-10);    // (c1 / c0 - 1)^2 < n 1e-10
+  d.tol_gauss = std::sqrt(P.n * 1e-12);  // (c1 / c0 - 1)^2 / n < 1e-12
   d.g1 = P.g1.p;
   d.g2 = P.g2.p;
   d.est_f = P.est_f.as<int>();

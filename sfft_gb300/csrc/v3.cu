@@ -454,13 +454,13 @@ __device__ __noinline__ void estimate(const PeelCtx &c, int stage, EstScratch &x
     if (bk0 < B && (reaches(s[2 * bk0], lw - 15) || reaches(s[2 * bk0 + 1], lw - 15)))
       x.raw[atomicAdd(&x.nraw, 1)] = bk0;
     __syncthreads();
-    // c0 + c1 > 1e-8, c0 > 0.01 and (c1 / c0 - 1)^2 < tol
+    // c0 + c1 > 1e-8, c0 > 0.01 and |c1 / c0 - 1| < tol (without the square,
+    // which overflows where c0 does not)
     if (t < x.nraw) {
       const int bk = x.raw[t];
       const double2 s0 = s[2 * bk], s1 = s[2 * bk + 1];
       const double c0 = fma(s0.x, s0.x, s0.y * s0.y) * norm2, c1 = fma(s1.x, s1.x, s1.y * s1.y) * norm2;
-      const double b = c1 - c0;
-      if (c0 + c1 > 1e-8 && c0 > 0.01 && b * b < tol * (c0 * c0)) {
+      if (c0 + c1 > 1e-8 && c0 > 0.01 && fabs(c1 - c0) < tol * c0) {
         const int i = atomicAdd(&x.cnt, 1);
         x.list[i] = bk;
         x.c0[i] = c0;

@@ -32,3 +32,34 @@ def test_fp64_medians_where_the_fp32_scale_overflows(env, scale):
     o = np.argsort(rf)
     np.testing.assert_array_equal(gi, rf[o])
     np.testing.assert_array_equal(gv, rv[o])
+
+
+@pytest.mark.parametrize("exponent", [0, 200, 300, 400, 500])
+@pytest.mark.parametrize("n,k", [(1 << 16, 50), (1 << 18, 100)])
+def test_v3_tones_of_any_size(env, oracle_lib, n, k, exponent):
+    """|value|^2 fits up to 2^511: the oracle's values of the signal, scaled,
+    within the 1e-10 of the parity tests, and nothing else that size.  (What is
+    left of large tones passes v3's absolute thresholds and is listed too.)"""
+    torch, _lib, L = env
+    from sfft_gb300 import signals
+    x, _, _ = signals.make_signal(n, k, 60)
+    oi, ov = oracle_lib.OraclePlan(n, k, 2).exec(x, seed=3)
+    scale = 2.0 ** exponent
+    plan = L.sfft_make_plan_ex(n, k, 2, 0, ctypes.byref(_lib.Options(0, -1, 1)))
+    assert plan, _lib.last_error()
+    cap = L.sfft_output_capacity(plan)
+    idx = torch.empty(cap, dtype=torch.int32, device="cuda")
+    val = torch.empty(cap, dtype=torch.complex128, device="cuda")
+    cnt = torch.zeros(1, dtype=torch.int32, device="cuda")
+    xd = torch.from_numpy(x * scale).cuda()
+    torch.cuda.synchronize()
+    assert L.sfft_exec_batch_ex(plan, 1, (ctypes.c_void_p * 1)(xd.data_ptr()), 0, (ctypes.c_uint * 1)(3), idx.data_ptr(),
+                                val.data_ptr(), cnt.data_ptr(), cap, None) == 0, _lib.last_error()
+    torch.cuda.synchronize()
+    c = int(cnt[0])
+    got = np.zeros(n, dtype=np.complex128)
+    got[idx[:c].cpu().numpy()] = val[:c].cpu().numpy() / scale
+    L.sfft_free_plan(plan)
+    want = np.zeros(n, dtype=np.complex128)
+    want[oi] = ov
+    assert np.max(np.abs(got - want)) <= 1e-10
