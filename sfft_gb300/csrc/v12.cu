@@ -1368,9 +1368,10 @@ __device__ __forceinline__ long ec_place(long hb, int i, int lr, int lg) {  // h
 // waits.  Every thread of a block of NTH threads calls it.  The mbarrier in
 // sh is initialised here; a caller that stages another item with the same
 // sh invalidates it first, after a block barrier.  srcmw (optional)
-// receives each (group, loop)'s run start and window index.  Returns the
-// live groups, or -1 if the wait timed out.
-template <int NTH>
+// receives each (group, loop)'s run start and window index.  SAME_LAUNCH: the
+// bucket values were stored by this launch (the caller acquired them), not by
+// an earlier one.  Returns the live groups, or -1 if the wait timed out.
+template <int NTH, bool SAME_LAUNCH>
 __device__ __forceinline__ int ec_stage(const V12Dev &d, int slot, long h0, long total, float2 *seg,
                                         EcShared<NTH> &sh, const float2 *xsrc, const float2 *wl, const float2 *we,
                                         int2 *srcmw) {
@@ -1428,8 +1429,12 @@ __device__ __forceinline__ int ec_stage(const V12Dev &d, int slot, long h0, long
   if (tab) {
     // the copy is issued before the window value is used, so the two loads
     // overlap (the buffer's previous contents were read through the generic
-    // proxy)
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // proxy; the bucket values of the same launch were stored through it, and
+    // a copy does not follow the acquire of those without a fence of its own)
+    if constexpr (SAME_LAUNCH)
+      asm volatile("fence.proxy.async;" ::: "memory");
+    else
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     bulk_load(seg + j * NTH + (u << lg), xsrc + (long)slot * d.xs_size + src, (unsigned)(G * sizeof(float2)),
               &sh.bar);
     sh.v[u * L + j] = EcVal{8u * (unsigned)rot, 8u * ai, g.x, g.y};
@@ -1512,11 +1517,11 @@ __device__ __forceinline__ void ec32_compute(const V12Dev &d, int slot, long h0,
 }
 
 // One item staged, waited for and estimated in FP32.
-template <int LN, bool EXACT, int NTH>
+template <int LN, bool EXACT, int NTH, bool SAME_LAUNCH = false>
 __device__ __forceinline__ void ec32_block(const V12Dev &d, int slot, long h0, long total, float2 *seg,
                                            EcShared<NTH> &sh) {
-  const int live = ec_stage<NTH>(d, slot, h0, total, seg, sh, (const float2 *)d.xs, (const float2 *)d.win_loc,
-                                 (const float2 *)d.win_est, nullptr);
+  const int live = ec_stage<NTH, SAME_LAUNCH>(d, slot, h0, total, seg, sh, (const float2 *)d.xs,
+                                              (const float2 *)d.win_loc, (const float2 *)d.win_est, nullptr);
   ec32_compute<LN, EXACT, NTH>(d, slot, h0, live, seg, sh);
 }
 
@@ -1587,8 +1592,8 @@ __device__ __forceinline__ int ec_proven(const float (&key)[LN], int Lr, const E
 template <int LN, bool EXACT, int NTH>
 __device__ __forceinline__ void ec64_block(const V12Dev &d, int slot, long h0, long total, float2 *seg,
                                            EcShared<NTH> &sh, int2 *srcmw) {
-  const int live = ec_stage<NTH>(d, slot, h0, total, seg, sh, (const float2 *)d.xs32,
-                                 (const float2 *)d.win32_loc, (const float2 *)d.win32_est, srcmw);
+  const int live = ec_stage<NTH, false>(d, slot, h0, total, seg, sh, (const float2 *)d.xs32,
+                                        (const float2 *)d.win32_loc, (const float2 *)d.win32_est, srcmw);
   const int L = d.L, lg = d.xs_perm, G = 1 << lg;
   const int u = threadIdx.x >> lg, i = threadIdx.x & (G - 1);
   if (u >= live) return;
@@ -1983,7 +1988,7 @@ __device__ __forceinline__ void persist_est(const V12Dev &d, const PersistGroup 
                                             EcShared<PT> &ecsh) {
   if (g.est_comb) {
     const long total = ec_total(d, slot), h0 = (long)idx * PT;
-    if (h0 < total) ec32_block<LN, EX, PT>(d, slot, h0, total, seg, ecsh);
+    if (h0 < total) ec32_block<LN, EX, PT, true>(d, slot, h0, total, seg, ecsh);
     __syncthreads();  // the item's mbarrier is no longer read
     if (threadIdx.x == 0 && h0 < total) mbar_inval(&ecsh.bar);
   } else {
