@@ -396,7 +396,7 @@ bool ensure_slots(PlanImpl &P, int want) {
   } else {
     const auto &p = P.p3;
     P.rp_stride = 5;
-    P.est_cap = std::max(p.W_Man, std::max(p.B_g1, p.B_g2)) + 16 * 1024;  // the peel kernel's CTAs share it out
+    P.est_cap = std::max(p.W_Man, std::max(p.B_g1, p.B_g2));  // the peel kernel's CTAs share it out
     P.map_cap = 4 * (p.W_Man + p.B_g1 + p.B_g2) + 8 * P.k;
     P.table_cap = 1;
     while (P.table_cap < 2 * P.map_cap) P.table_cap <<= 1;

@@ -274,8 +274,15 @@ long estimate_bytes(const PlanKey &key, int slots, int tune) {
     return cst + per * slots;
   }
   const long W = f[0], B1 = f[1], B2 = f[3];
-  const long per = 32 * (W + B1 + B2) + 16 * 2 * (f[4] + 2) + 64 * (W + B1 + B2 + 8L * key.k) * 4;
-  return (f[2] + f[4]) * 16 + 16L * 3 * key.n / B1 + 16L * 3 * key.n / B2 + per * slots;
+  const long map = 4 * (W + B1 + B2) + 8L * key.k;
+  long table = 1;
+  while (table < 2 * map) table <<= 1;
+  // combs twice, Gaussian buckets, estimates, result table, result lists
+  const long per = 64 * W + 32 * (B1 + B2) + 20 * std::max(W, std::max(B1, B2)) + 20 * table + 24 * map + 128;
+  auto window = [&](long B) { return 16 * std::min((long)key.n, 2 * (3 * (key.n / B) / 2 + 2) + 1); };
+  // taps, windows, twiddles, phase table, diagnostics of slot 0
+  const long cst = (f[2] + f[4]) * 16 + window(B1) + window(B2) + 16 * (W + B1 + B2) + 16 * 1024 + 40 * map;
+  return cst + per * slots;
 }
 
 PlanEntry *get_plan(sfft_server *s, const PlanKey &key, std::string &err) {

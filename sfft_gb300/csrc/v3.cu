@@ -404,8 +404,7 @@ __device__ __forceinline__ int v3_spread(int tid) {
 }
 
 // Per-CTA shared scratch of the estimation loops, and the tones that the CTA
-// found in the current phase (beyond V3_LIST in est_f / est_v, which have
-// room for one tone per bucket that the CTA visits).
+// found in the current phase (beyond V3_LIST in est_f / est_v).
 struct EstScratch {
   int raw[V3_LIST], list[V3_LIST], key[V3_LIST];
   int nraw, cnt, tones;
@@ -601,8 +600,10 @@ __global__ void __launch_bounds__(V3_LIST) k_v3_peel(V3Dev dev) {
     c.tval = (double2 *)dev.map_vals + (long)slot * dev.table_cap;
     c.list = dev.map_table + (long)slot * dev.map_cap;
     c.tmask = dev.table_cap - 1;
-    // this CTA's share of the spill arrays: a tone per bucket it visits
-    const long share = (dev.est_cap - 16 * V3_LIST) / nb + V3_LIST;
+    // this CTA's share of the spill arrays.  Bucket counts and nb are powers of
+    // two: of B buckets it visits at most V3_LIST, all in shared memory, or
+    // B / nb, the first V3_LIST of whose tones are
+    const long share = dev.est_cap / nb;
     c.est_f = dev.est_f + (long)slot * dev.est_cap + rank * share;
     c.est_v = (double2 *)dev.est_v + (long)slot * dev.est_cap + rank * share;
     c.counters = dev.counters + slot * CNT_STRIDE;

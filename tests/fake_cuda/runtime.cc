@@ -114,6 +114,12 @@ cudaError_t cudaFree(void *p) {  // waits for the device
   free(p);
   return cudaSuccess;
 }
+cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
+cudaError_t cudaLaunchHostFunc(cudaStream_t s, cudaHostFn_t f, void *arg) {
+  const cudaError_t e = op("host", s);
+  if (e == cudaSuccess) f(arg);
+  return e;
+}
 cudaError_t cudaMallocHost(void **p, size_t n) { return (*p = allocate(n)) ? cudaSuccess : cudaErrorMemoryAllocation; }
 cudaError_t cudaFreeHost(void *p) { return free(p), cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {

@@ -20,7 +20,7 @@ SHAPES = [(0, 1 << 13, 50), (1, 1 << 14, 50), (2, 1 << 13, 16)]   # version, n, 
 def fake(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
     src = [os.path.join(HERE, "fake_cuda", "runtime.cc")]
-    src += [os.path.join(build.CSRC, f) for f in ("api.cc", "host_plan.cc", "tune.cc")]
+    src += [os.path.join(build.CSRC, f) for f in ("api.cc", "host_plan.cc", "tune.cc", "serve.cc")]
     subprocess.check_call(["g++", "-O1", "-fPIC", "-std=c++17", "-fopenmp", "-shared", "-Wl,-Bsymbolic", "-o", so] + src +
                           ["-I" + os.path.join(build._cuda_home(), "include"), "-I" + os.path.join(build.ROOT, "include"),
                            "-I" + build.CSRC])
@@ -28,16 +28,16 @@ def fake(tmp_path_factory):
     vp, cl = ctypes.c_void_p, ctypes.c_long
     for f in (L.sfft_make_plan_ex, L.sfft_plan_stream):
         f.restype = vp
-    for f in (L.sfft_output_capacity, L.sfft_exec_sparse):
+    for f in (L.sfft_output_capacity, L.sfft_exec_sparse, L.sfft_plan_footprint, L.sfft_server_plan_bytes):
         f.restype = cl
     L.sfft_last_error.restype = L.fake_name.restype = ctypes.c_char_p
     return L
 
 
 class Plan:
-    def __init__(self, L, version, n, k, max_batch=4):
+    def __init__(self, L, version, n, k, max_batch=4, prec=0):
         self.L, self.n = L, n
-        self.p = vp(L.sfft_make_plan_ex(n, k, version, 0, ctypes.byref(_lib.Options(0, -1, max_batch))))
+        self.p = vp(L.sfft_make_plan_ex(n, k, version, 0, ctypes.byref(_lib.Options(prec, -1, max_batch))))
         assert self.p, L.sfft_last_error()
         self.cap = L.sfft_output_capacity(self.p)
         self.bufs = []
@@ -187,3 +187,21 @@ def test_buffers_are_whole_after_a_batch_that_did_not_fit(fake, plan, call, limi
     done = plan.ops(at, "transform")
     assert done and all(fake.fake_whole(i) for i in done)
     assert failed or limit > 1 << 18
+
+
+@pytest.mark.parametrize("version,n,k,prec", [
+    (2, 1 << 14, 8, 0), (2, 1 << 14, 9, 0), (2, 1 << 15, 31, 0), (2, 1 << 16, 50, 0), (2, 1 << 14, 127, 0),
+    (2, 1 << 16, 1000, 0), (0, 1 << 13, 50, 0), (0, 1 << 16, 50, 1), (1, 1 << 14, 50, 0), (1, 1 << 16, 50, 0),
+    (1, 1 << 16, 50, 1)])
+@pytest.mark.parametrize("m", [1, 32])
+def test_the_servers_estimate_covers_a_plans_workspace(fake, version, n, k, prec, m):
+    """A server admits a plan by its estimate for max_batch signals: it is no
+    less than what such a batch makes the plan hold, but for a twentieth, and
+    not several times more."""
+    p = Plan(fake, version, n, k, m, prec)
+    r, done = p.batch(m)
+    assert r == 0 and done
+    held, estimate = fake.sfft_plan_footprint(p.p), fake.sfft_server_plan_bytes(n, k, version, prec, m)
+    p.free()
+    print(version, n, k, prec, m, held, estimate, estimate / held)
+    assert 0.95 * held <= estimate <= 4 * held
