@@ -186,7 +186,7 @@ def test_buffers_are_whole_after_a_batch_that_did_not_fit(fake, plan, call, limi
     call(plan)
     done = plan.ops(at, "transform")
     assert done and all(fake.fake_whole(i) for i in done)
-    assert failed or limit > 1 << 18
+    assert failed or limit > 1 << 14   # the smallest limit is below every workspace
 
 
 @pytest.mark.parametrize("version,n,k,prec", [
