@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -114,7 +115,13 @@ struct PlanImpl {
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;     // recorded after each asynchronous batch
   bool batch_elsewhere = false;   // one of them ran on a stream of its caller
-  // host-buffer pipeline of sfft_exec_many: copies in / out on their own streams
+  // The plan's stream may hold work that the host has not waited for: its
+  // handle was given out, or a batch (or a call that failed) was queued.
+  mutable std::atomic<bool> stream_given{false};
+  bool queued = false;
+  // host-buffer pipeline of sfft_exec_many: copies in / out on their own
+  // streams.  copy_in has the greatest priority: dense calls on device buffers
+  // run on it, ahead of the clearing of their outputs on copy_out.
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
   cudaEvent_t ev_in[2] = {nullptr, nullptr}, ev_comp[2] = {nullptr, nullptr}, ev_out[2] = {nullptr, nullptr};
   std::mutex mu;
@@ -812,18 +819,23 @@ bool ensure_host_counters(PlanImpl &P, int num) {
 // signals of 2^16 points: 472 us, from the end of the fold on 480).
 // One memset per output took 41 us for 2^24 points after a v3 transform of 110
 // us, and 64 calls for 64 outputs of 2^16 points.
+// The blocks of the transform go first where both have some to run: without a
+// priority of its own one signal of 2^24 points takes 183 us (v1, 157 with) and
+// 211 us (v3, 202).  The plan's own stream has none, so that batches share the
+// GPU evenly with other streams.
 // Work that is already queued on the plan's stream (a batch with a NULL stream,
-// or what a program put on sfft_plan_stream) may use the same buffers, so the
-// clearing comes after it; an idle stream, the usual case, costs one query.
+// or what a program put on sfft_plan_stream) may use the same buffers, so all of
+// this comes after it; where the stream cannot hold any, nothing is asked (a
+// query takes 1.5 us).
 bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out, const char *in_dev, const char *out_dev) {
-  cudaStream_t s = P.stream;
+  cudaStream_t s = P.copy_in;
   struct Drain {  // a failed call leaves nothing writing to the caller's buffers
     PlanImpl &P;
     bool done = false;
     ~Drain() {
       if (done) return;
       cudaStreamSynchronize(P.copy_out);
-      cudaStreamSynchronize(P.stream);
+      cudaStreamSynchronize(P.copy_in);
     }
   } drain{P};
   const size_t nb = sizeof(double) * 2 * (size_t)P.n;
@@ -837,11 +849,14 @@ bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out, con
   if (need_in_stage && !P.in_stage.ensure(nb * P.slots)) return false;
   if (need_out_stage && !P.dense_stage.ensure(nb * P.slots)) return false;
   if (!ensure_host_counters(P, num)) return false;
-  const cudaError_t idle = cudaStreamQuery(s);
-  cudaGetLastError();
-  if (idle != cudaSuccess && (!cuda_ok(cudaEventRecord(P.ev_in[0], s), "event") ||
-                              !cuda_ok(cudaStreamWaitEvent(P.copy_out, P.ev_in[0], 0), "wait")))
-    return false;
+  if (P.queued || P.stream_given) {
+    const cudaError_t idle = cudaStreamQuery(P.stream);
+    cudaGetLastError();
+    if (idle != cudaSuccess && (!cuda_ok(cudaEventRecord(P.ev_in[0], P.stream), "event") ||
+                                !cuda_ok(cudaStreamWaitEvent(s, P.ev_in[0], 0), "wait") ||
+                                !cuda_ok(cudaStreamWaitEvent(P.copy_out, P.ev_in[0], 0), "wait")))
+      return false;
+  }
   for (int i = 0; i < num; i++) {
     dev_in[i] = in_dev[i] ? (const void *)in[i] : (const void *)((char *)P.in_stage.p + nb * i);
     dense[i] = out_dev[i] ? (void *)out[i] : (void *)((char *)P.dense_stage.p + nb * i);
@@ -875,6 +890,7 @@ bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out, con
       !cuda_ok(cudaStreamSynchronize(s), "exec"))
     return false;
   drain.done = true;
+  P.queued = false;  // it came before what the host just waited for
   return check_counts(P.h_cnt, num);
 }
 
@@ -1319,12 +1335,11 @@ static sfft_plan *make_plan_impl(int n, int k, enum sfft_version version, const 
         !upload_twiddles(P->tw_c, p.W_Man, sfft::PREC_FP64) || !upload_trig(P->trig))
       return nullptr;
   }
-  // above the copy streams, on which outputs are cleared beside the transform
   int least = 0, greatest = 0;
   cudaDeviceGetStreamPriorityRange(&least, &greatest);
-  if (!cuda_ok(cudaStreamCreateWithPriority(&P->stream, cudaStreamNonBlocking, greatest), "stream")) return nullptr;
+  if (!cuda_ok(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking), "stream")) return nullptr;
   if (!cuda_ok(cudaEventCreateWithFlags(&P->done, cudaEventDisableTiming), "event")) return nullptr;
-  if (!cuda_ok(cudaStreamCreateWithFlags(&P->copy_in, cudaStreamNonBlocking), "stream") ||
+  if (!cuda_ok(cudaStreamCreateWithPriority(&P->copy_in, cudaStreamNonBlocking, greatest), "stream") ||
       !cuda_ok(cudaStreamCreateWithFlags(&P->copy_out, cudaStreamNonBlocking), "stream"))
     return nullptr;
   for (int h = 0; h < 2; h++)
@@ -1373,6 +1388,7 @@ void sfft_free_plan(sfft_plan *plan) {
 
 void *sfft_plan_stream(const sfft_plan *plan) {
   const PlanImpl *P = plan ? (const PlanImpl *)plan->data : nullptr;
+  if (P) P->stream_given = true;
   return P ? (void *)P->stream : nullptr;
 }
 
@@ -1443,7 +1459,8 @@ void sfft_exec_many(sfft_plan *plan, int num, complex_t **in, complex_t **out) {
     if (in_dev[i] || out_dev[i]) all_host = false;
   }
   if (all_host) {  // about 32 chunks: copies overlap the transforms with little fill and drain
-    exec_dense_pipelined(*P, num, in, out, std::max(1, std::min(chunk, (num + 31) / 32)));
+    P->queued = true;
+    if (exec_dense_pipelined(*P, num, in, out, std::max(1, std::min(chunk, (num + 31) / 32)))) P->queued = false;
     return;
   }
   if (!ensure_slots(*P, chunk)) return;
@@ -1463,6 +1480,7 @@ long sfft_exec_sparse(sfft_plan *plan, const complex_t *in, int *out_idx, comple
   cudaSetDevice(P->device);
   g_err.clear();
   if (!after_batches(*P) || !ensure_slots(*P, 1)) return -1;
+  P->queued = true;
   cudaStream_t s = P->stream;
   const size_t nb = sizeof(double) * 2 * (size_t)P->n;
   const void *dev_in = in;
@@ -1503,6 +1521,7 @@ long sfft_exec_sparse(sfft_plan *plan, const complex_t *in, int *out_idx, comple
                  "value copy"))
       return -1;
   }
+  P->queued = false;
   return c;
 }
 
@@ -1519,7 +1538,10 @@ int sfft_exec_many_sparse(sfft_plan *plan, int num, const complex_t *const *in, 
   g_err.clear();
   if (!after_batches(*P)) return -1;
   const int chunk = std::max(1, std::min(P->max_batch, (num + 31) / 32));  // about 32 pipelined chunks
-  return exec_sparse_pipelined(*P, num, in, out_idx, out_val, out_count, out_stride, chunk) ? 0 : -1;
+  P->queued = true;
+  if (!exec_sparse_pipelined(*P, num, in, out_idx, out_val, out_count, out_stride, chunk)) return -1;
+  P->queued = false;
+  return 0;
 }
 
 int sfft_exec_batch(sfft_plan *plan, int num, const void *const *in, int in_type, int *out_idx, void *out_val,
@@ -1546,6 +1568,7 @@ int sfft_exec_batch_ex(sfft_plan *plan, int num, const void *const *in, int in_t
   if (!cuda_ok(cudaStreamWaitEvent(s, P->done, 0), "event wait")) return -1;
   const size_t cs = (P->version < 2 && P->prec == sfft::PREC_FP32) ? 8 : 16;
   bool good = true;
+  P->queued = true;
   for (int i0 = 0; good && i0 < num; i0 += P->slots) {
     const int m = std::min(P->slots, num - i0);
     // results go straight into the caller's strided buffers

@@ -33,6 +33,7 @@ std::recursive_mutex mu;
 std::vector<Op> ops;
 std::map<long, Set> streams;  // what the stream's next operation comes after
 std::map<long, Set> events;
+std::map<long, int> priority; // streams with one
 Set host;                     // what the host has waited for
 std::map<char *, size_t> mem;
 size_t limit_bytes = (size_t)-1;
@@ -79,6 +80,8 @@ int fake_before(int a, int b) { return a < (int)ops[b].before.size() && ops[b].b
 // Whether the host knows operation a to be complete.
 int fake_waited(int a) { return a < (int)host.size() && host[a]; }
 void fake_work(void *stream) { op("work", stream); }
+int fake_priority(void *stream) { return priority.count((long)stream) ? priority[(long)stream] : 0; }
+int fake_op_priority(int i) { return fake_priority((void *)ops[i].stream); }
 void fake_limit(size_t bytes) { limit_bytes = bytes; }
 void fake_fail_after(const char *name, int count) { failing = name, passes = count; }
 void fake_fail(const char *name) { fake_fail_after(name, 0); }
@@ -143,7 +146,11 @@ cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t st) {
 }
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return *s = (cudaStream_t)next_handle++, cudaSuccess; }
-cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned, int) { return *s = (cudaStream_t)next_handle++, cudaSuccess; }
+cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned, int p) {
+  *s = (cudaStream_t)next_handle++;
+  priority[(long)*s] = p;
+  return cudaSuccess;
+}
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
   std::lock_guard<std::recursive_mutex> g(mu);

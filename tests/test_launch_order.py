@@ -90,10 +90,24 @@ def test_outputs_are_cleared_after_work_on_the_plans_stream(fake, plan, m):
     ins, outs = plan.signals(m), plan.signals(m)
     fake.sfft_exec_many(plan.p, m, ins, outs)
     assert fake.sfft_last_error() == b""
-    clears = plan.ops(at, "clear")
-    assert clears
-    for c in clears:
+    assert plan.ops(at, "clear")
+    for c in plan.ops(at, "clear", "setup", "transform", "scatter"):
         assert all(fake.fake_before(b, c) for b in before)
+
+
+def test_only_the_transforms_of_dense_calls_go_first(fake, plan):
+    """The plan's stream, on which batches run, has no priority over the
+    streams of the program; a dense call's transform has one over the clearing
+    of its outputs."""
+    assert fake.fake_priority(vp(fake.sfft_plan_stream(plan.p))) == 0
+    at = fake.fake_ops()
+    plan.batch(2)
+    assert all(fake.fake_op_priority(i) == 0 for i in range(at, fake.fake_ops()))
+    fake.cudaDeviceSynchronize()
+    at = fake.fake_ops()
+    fake.sfft_exec_many(plan.p, 1, plan.signals(1), plan.signals(1))
+    assert all(fake.fake_op_priority(i) < 0 for i in plan.ops(at, "transform"))
+    assert all(fake.fake_op_priority(i) == 0 for i in plan.ops(at, "clear"))
 
 
 def test_clearing_does_not_wait_for_the_calls_own_input_copies(fake, plan):
