@@ -25,7 +25,7 @@ CU_SOURCES = ["v12.cu", "v3.cu", "noalloc.cu"]
 # last-ulp rounding matters: no multiply-add contraction in that file.
 CU_EXTRA = {"v3.cu": ["--fmad=false"]}
 CC_SOURCES = ["api.cc", "host_plan.cc", "serve.cc", "mixed.cc", "tune.cc"]
-HEADERS = ["common.cuh", "fft.cuh", "engine.h", "host_plan.h", "tuned_table.inc"]
+HEADERS = ["common.cuh", "fft.cuh", "phase.cuh", "engine.h", "host_plan.h", "tuned_table.inc"]
 
 
 def _cuda_home():
