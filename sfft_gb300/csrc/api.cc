@@ -777,6 +777,19 @@ bool after_batches(PlanImpl &P) {
   return true;
 }
 
+// Work that is already queued on the plan's stream (a batch with a NULL stream,
+// or what a program put on sfft_plan_stream) may use a call's buffers: what the
+// call puts on the copy streams comes after it.  Where the plan's stream cannot
+// hold any, nothing is asked (a query takes 1.5 us).
+bool after_plan_stream(PlanImpl &P) {
+  if (!P.queued && !P.stream_given) return true;
+  const cudaError_t idle = cudaStreamQuery(P.stream);
+  cudaGetLastError();
+  return idle == cudaSuccess || (cuda_ok(cudaEventRecord(P.ev_in[0], P.stream), "event") &&
+                                 cuda_ok(cudaStreamWaitEvent(P.copy_in, P.ev_in[0], 0), "wait") &&
+                                 cuda_ok(cudaStreamWaitEvent(P.copy_out, P.ev_in[0], 0), "wait"));
+}
+
 // Whether the input and output arrays (nb bytes each) of device pointers
 // overlap anywhere, an in-place transform among them.
 bool in_out_overlap(const std::vector<const void *> &in, const std::vector<void *> &out, size_t nb) {
@@ -823,10 +836,6 @@ bool ensure_host_counters(PlanImpl &P, int num) {
 // priority of its own one signal of 2^24 points takes 183 us (v1, 157 with) and
 // 211 us (v3, 202).  The plan's own stream has none, so that batches share the
 // GPU evenly with other streams.
-// Work that is already queued on the plan's stream (a batch with a NULL stream,
-// or what a program put on sfft_plan_stream) may use the same buffers, so all of
-// this comes after it; where the stream cannot hold any, nothing is asked (a
-// query takes 1.5 us).
 bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out, const char *in_dev, const char *out_dev) {
   cudaStream_t s = P.copy_in;
   struct Drain {  // a failed call leaves nothing writing to the caller's buffers
@@ -849,14 +858,7 @@ bool exec_dense_chunk(PlanImpl &P, int num, complex_t **in, complex_t **out, con
   if (need_in_stage && !P.in_stage.ensure(nb * P.slots)) return false;
   if (need_out_stage && !P.dense_stage.ensure(nb * P.slots)) return false;
   if (!ensure_host_counters(P, num)) return false;
-  if (P.queued || P.stream_given) {
-    const cudaError_t idle = cudaStreamQuery(P.stream);
-    cudaGetLastError();
-    if (idle != cudaSuccess && (!cuda_ok(cudaEventRecord(P.ev_in[0], P.stream), "event") ||
-                                !cuda_ok(cudaStreamWaitEvent(s, P.ev_in[0], 0), "wait") ||
-                                !cuda_ok(cudaStreamWaitEvent(P.copy_out, P.ev_in[0], 0), "wait")))
-      return false;
-  }
+  if (!after_plan_stream(P)) return false;
   for (int i = 0; i < num; i++) {
     dev_in[i] = in_dev[i] ? (const void *)in[i] : (const void *)((char *)P.in_stage.p + nb * i);
     dense[i] = out_dev[i] ? (void *)out[i] : (void *)((char *)P.dense_stage.p + nb * i);
@@ -1459,6 +1461,7 @@ void sfft_exec_many(sfft_plan *plan, int num, complex_t **in, complex_t **out) {
     if (in_dev[i] || out_dev[i]) all_host = false;
   }
   if (all_host) {  // about 32 chunks: copies overlap the transforms with little fill and drain
+    if (!after_plan_stream(*P)) return;
     P->queued = true;
     if (exec_dense_pipelined(*P, num, in, out, std::max(1, std::min(chunk, (num + 31) / 32)))) P->queued = false;
     return;
@@ -1538,6 +1541,7 @@ int sfft_exec_many_sparse(sfft_plan *plan, int num, const complex_t *const *in, 
   g_err.clear();
   if (!after_batches(*P)) return -1;
   const int chunk = std::max(1, std::min(P->max_batch, (num + 31) / 32));  // about 32 pipelined chunks
+  if (!after_plan_stream(*P)) return -1;
   P->queued = true;
   if (!exec_sparse_pipelined(*P, num, in, out_idx, out_val, out_count, out_stride, chunk)) return -1;
   P->queued = false;

@@ -219,3 +219,16 @@ def test_the_servers_estimate_covers_a_plans_workspace(fake, version, n, k, prec
     p.free()
     print(version, n, k, prec, m, held, estimate, estimate / held)
     assert 0.95 * held <= estimate <= 4 * held
+
+
+@pytest.mark.parametrize("call", [_dense, _dense_host, _sparse, _many_sparse])
+def test_every_copy_comes_after_work_on_the_plans_stream(fake, plan, call):
+    """That work may still write a call's inputs or read its outputs."""
+    call(plan)                                      # the staging has its size
+    fake.cudaDeviceSynchronize()
+    work = fake.fake_ops()
+    fake.fake_work(vp(fake.sfft_plan_stream(plan.p)))
+    call(plan)
+    assert fake.sfft_last_error() == b""
+    for i in range(work + 1, fake.fake_ops()):
+        assert fake.fake_before(work, i), fake.fake_name(i)
