@@ -937,8 +937,8 @@ def roofline(p32, st32, B):
                       "algorithmic_bytes_per_launch": B * bytes_sig, "launch_ms": ms,
                       "peak_source": f"{peak_src} hbm_gbs (copy bandwidth)"}
     out["fold"]["note"] = ("random 16-byte gathers touch most DRAM bursts of the 64 MB signal: DRAM moves "
-                           "3.4x the algorithmic bytes (58.8 MB per signal at 73% of peak DRAM throughput in "
-                           "ncu); one read of the signal (9.4 us) is the floor, the kernel takes ~10 us")
+                           "3.4x the algorithmic bytes (58.8 MB per signal, 8.7 us at the measured copy rate: "
+                           "the floor; the kernel takes ~10 us)")
     out["estimate"]["note"] = ("bound by the ALU pipe, not HBM: the two lower-median selection networks "
                                "(FMNMX, 2 x 125 per candidate) keep it at 65% of peak in ncu "
                                "(profiles/k_estimate_comb32_*); every staged bucket byte is read once (58 MB of L2 "

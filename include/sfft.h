@@ -128,8 +128,10 @@ typedef struct sfft_params sfft_params;
 sfft_plan *sfft_make_plan_params(int n, int k, enum sfft_version version, const sfft_params *params,
                                  const sfft_options *opt);
 
-/* The plan's own CUDA stream (a cudaStream_t): work submitted with a NULL
- * stream runs there. */
+/* The plan's own CUDA stream (a cudaStream_t, of default priority): work
+ * submitted with a NULL stream runs there.  Calls of one plan are ordered:
+ * each comes after earlier batches, on whatever stream they run, and the
+ * synchronous calls also after what a program has queued on this stream. */
 void *sfft_plan_stream(const sfft_plan *plan);
 
 /* Device memory a plan holds (constants and workspace), in bytes. */

@@ -2,16 +2,20 @@
 //
 //   k_comb      (v2) strided W-point gather + shared-memory FFT + |.|^2 +
 //               top-num residues (computefourier-1.0-2.0.cc:48-82) -> sorted,
-//               de-duplicated residue list of the samplings  (:491-503)
+//               de-duplicated residue list of the samplings  (:491-503);
+//               from 1024 points k_comb_a / _b / _select over many CTAs
 //   k_fold      permuted-filter fold, one thread per (loop, bucket),
-//               taps summed in increasing order                      (:222-261)
+//               taps summed in increasing order                      (:222-261);
+//               FP32: k_fold_split
 //   k_bucket    per loop: B-point FFT in shared memory, |.|^2, top-num
-//               bucket selection, then (location loops) integer voting
-//               of the n/B frequencies of each selected bucket      (:270-324, :91-184)
-//   k_estimate  per candidate: value in each loop, lower median of the
+//               bucket selection                                    (:270-324);
+//               FP64 from 1024 points k_bucket_a / _b / _select
+//   k_vote_*    integer voting of the n/B frequencies of each selected
+//               bucket                                               (:91-184)
+//   k_estimate* per candidate: value in each loop, lower median of the
 //               real and imaginary parts separately                 (:340-419)
 //
-// All kernels take a slot index (blockIdx.y) so that one launch serves a
+// All kernels take a slot index (blockIdx.y or .z) so that one launch serves a
 // batch of signals sharing a plan.  FP64 instantiations reproduce the CPU
 // definition bit for bit; FP32 ones accumulate in float.
 #include <algorithm>
@@ -669,7 +673,7 @@ __global__ void __launch_bounds__(1024) k_comb_select(V12Dev d) {
 }
 
 // One Stockham stage over `narr` arrays of N points per slot (plan-time
-// transforms of up to 2^30 points and v3's long combs).
+// transforms of up to 2^30 points).
 template <typename R>
 __global__ void __launch_bounds__(256) k_fft_stage(const c2_t<R> *src, c2_t<R> *dst, int N, int Ns, int radix,
                                                    long arr_stride, int narr, long slot_stride,
@@ -1132,7 +1136,8 @@ __device__ __forceinline__ int proven_median(const float (&v)[LN], const float (
 }
 
 // Resident 128-thread blocks per SM the estimation kernels are compiled
-// for (registers per thread = 65536 / (128 * blocks), without spills).
+// for (registers per thread = 65536 / (128 * blocks); some loop counts spill
+// up to 32 bytes, ptxas: FP32 19, 20 and 22, FP64 from 18 on).
 constexpr int est32_blocks(int LN) { return LN <= 18 ? 8 : LN <= 24 ? 6 : 5; }
 constexpr int est64_blocks(int LN) { return LN <= 14 ? 6 : LN <= 20 ? 5 : 4; }
 
@@ -1287,7 +1292,10 @@ __global__ void __launch_bounds__(128, est64_blocks(LN)) k_estimate64(V12Dev d, 
 // 128 x 8 348, 128 x 9 (56 registers) 330, 128 x 10 (48) 356, 64 x 16 384,
 // 64 x 18 370; 8 FP64 signals: 256 x 4 180, 128 x 7 167, 128 x 8 166,
 // 128 x 9 179, 64 x 16 171 (before ec_place interleaved their stores, which
-// costs 2 and 6 us of that).  Groups are at most this long (xs_perm_of).
+// costs 2 and 6 us of that).  All of these are at L = 20 loops; other loop
+// counts take the same shape unmeasured, and in FP64 its 64 registers spill 16
+// to 190 bytes at L = 10 .. 13 and from 20 on (none at the four 256-thread
+// CTAs of before).  Groups are at most this long (xs_perm_of).
 constexpr int EC_THREADS = EC_GROUP_MAX;
 constexpr int EC_MAXL = 32;
 constexpr long EC_WAIT_POLLS = 1L << 22;

@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(1024) k_v3_second(V3Dev d, V3Shape sh) {
 // is latency: chains of FP64 instructions (about 100 from a bucket's values
 // to the subtraction of its tone), L2 round trips and cluster barriers.  What
 // was taken out of the chains, with the kernel's time for one signal of n =
-// 2^24, k = 1000 (6 rounds) and for 16 of n = 2^18, k = 100: library atan2 /
+// 2^24, k = 1000 (6 or 9 rounds, by the signal) and for 16 of n = 2^18, k = 100: library atan2 /
 // sincos and 8 CTAs 202 / 208 us; table phases and 16 CTAs 148 / 168; no
 // divisions for constants in every warp (8 warps a sub-partition, 64 cycles
 // an instruction) and lists by exponent 104 / 114; tones peeled by the CTA
