@@ -1339,9 +1339,12 @@ static sfft_plan *make_plan_impl(int n, int k, enum sfft_version version, const 
   }
   int least = 0, greatest = 0;
   cudaDeviceGetStreamPriorityRange(&least, &greatest);
-  if (!cuda_ok(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking), "stream")) return nullptr;
-  if (!cuda_ok(cudaEventCreateWithFlags(&P->done, cudaEventDisableTiming), "event")) return nullptr;
+  // copy_in first: with the plan's stream in front of it, clearing and transform
+  // of the first plan of a process did not overlap (stage times as without the
+  // clearing; 9 v2 signals of 2^19 points 150 us, in this order 137)
   if (!cuda_ok(cudaStreamCreateWithPriority(&P->copy_in, cudaStreamNonBlocking, greatest), "stream") ||
+      !cuda_ok(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking), "stream") ||
+      !cuda_ok(cudaEventCreateWithFlags(&P->done, cudaEventDisableTiming), "event") ||
       !cuda_ok(cudaStreamCreateWithFlags(&P->copy_out, cudaStreamNonBlocking), "stream"))
     return nullptr;
   for (int h = 0; h < 2; h++)
